@@ -264,10 +264,10 @@ long long lbm_adjoint_forward_steps(long long nsteps, int slots);
  *   nodes of that region; 7 sum phi; 8 sum rho; 9..11 sum rho u;
  *   12 number of nodes with phi >= 0; 13 max |u|^2; 14 number of nodes with a
  *   non-finite value (full domain for 7..14); 15 zero.
- * The per-block partial sums use a 1 MiB array in the library's static device
+ * The per-block partial sums use a 57 KiB array in the library's static device
  * memory, which every GPU that loads the library keeps until the process
- * exits.  That array bounds the box: more than LBM_NOALLOC_MAX_NODES nodes is
- * rejected with LBM_EINVAL, and so are parameters whose constants cannot be
+ * exits.  More than LBM_NOALLOC_MAX_NODES nodes is rejected with LBM_EINVAL,
+ * and so are parameters whose constants cannot be
  * derived (tauRho, tauPhi or width not positive, rhoH == rhoL).  The first
  * call on a device looks up the array's device address
  * (cudaGetSymbolAddress); under CUDA's lazy module loading (the default) that

@@ -130,7 +130,7 @@ namespace {
 // Stats reduction of the mom arrays into c->result_host (synchronises).
 int reduce_stats(lbm_ctx *c)
 {
-    cudaError_t e = lbm::launch_stats(c->box, c->d, c->st.mom, c->partials, c->partial_count, c->result, nullptr,
+    cudaError_t e = lbm::launch_stats(c->box, c->d, c->st.mom, c->partials, c->partial_count, c->result,
                                       c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "stats kernel launch");
     LBM_CUDA(cudaMemcpyAsync(c->result_host, c->result, sizeof(double) * lbm::kStatsValues, cudaMemcpyDeviceToHost,
@@ -503,7 +503,7 @@ extern "C" int lbm_stats(lbm_ctx *c, lbm_stats_out *s, float *phi, float *rho, f
     const size_t n = (size_t)c->box.n, bytes = sizeof(float) * n;
     if (s) {
         cudaError_t e = lbm::launch_stats(c->box, c->d, c->st.mom, c->partials, c->partial_count, c->result,
-                                          nullptr, c->stream);
+                                          c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "stats kernel launch");
         LBM_CUDA(cudaMemcpyAsync(c->result_host, c->result, sizeof(double) * lbm::kStatsValues,
                                  cudaMemcpyDeviceToHost, c->stream),
@@ -535,7 +535,7 @@ extern "C" int lbm_stats_fields(lbm_ctx *c, lbm_stats_out *s, const float *phi, 
     for (int a = 0; a < 5 && e == cudaSuccess; a++)
         e = cudaMemcpyAsync(tmp + a * n, src[a], bytes, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
-        e = lbm::launch_stats(c->box, c->d, tmp, c->partials, c->partial_count, c->result, nullptr, c->stream);
+        e = lbm::launch_stats(c->box, c->d, tmp, c->partials, c->partial_count, c->result, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(c->result_host, c->result, sizeof(double) * lbm::kStatsValues, cudaMemcpyDeviceToHost,
                             c->stream);

@@ -148,7 +148,7 @@ cudaError_t launch_field_maxabs(const Box &b, const float *f, const float *g, co
 cudaError_t launch_moments(const Box &b, const float *f, const float *g, float *mom, cudaStream_t s);
 // phi_lo / phi_hi: the phi planes below and above a z-slab (NULL: periodic z).
 cudaError_t launch_stats(const Box &b, const lbm_derived &d, const float *mom, double *partials,
-                         size_t partial_count, double *result, unsigned long long *counters, cudaStream_t s,
+                         size_t partial_count, double *result, cudaStream_t s,
                          const float *phi_lo = nullptr, const float *phi_hi = nullptr);
 size_t stats_partial_count(const Box &b);
 // Pressure field (n floats) of the mom arrays (src/vtksave.c:63-127).

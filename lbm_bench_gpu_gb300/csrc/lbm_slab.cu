@@ -487,7 +487,7 @@ extern "C" int lbm_stats_raw(lbm_ctx *c, double *raw)
     LBM_ON_DEVICE(c->p.device);
     const float *lo = c->box.zghost ? c->phi_ghost : nullptr;
     const float *hi = c->box.zghost ? c->phi_ghost + c->box.nxy : nullptr;
-    cudaError_t e = lbm::launch_stats(c->box, c->d, c->st.mom, c->partials, c->partial_count, c->result, nullptr,
+    cudaError_t e = lbm::launch_stats(c->box, c->d, c->st.mom, c->partials, c->partial_count, c->result,
                                       c->stream, lo, hi);
     if (e != cudaSuccess) return cuda_fail(e, "stats kernel launch");
     LBM_CUDA(cudaMemcpyAsync(c->result_host, c->result, sizeof(double) * lbm::kStatsValues, cudaMemcpyDeviceToHost,

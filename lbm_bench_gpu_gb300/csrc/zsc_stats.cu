@@ -5,8 +5,8 @@
 // compensated float sums (a float pair hi + lo updated with Knuth's two-sum,
 // products split exactly with an FMA), which hold ~48 bits like an FP64 sum
 // at FP32 throughput (GB300's FP64 rate is a small fraction of its FP32 rate);
-// FP64 warp-shuffle reductions per block into a partials array, then one block
-// folds the partials in a fixed order (deterministic for a given box).
+// the same pairs through the warp reduction, FP64 across warps and blocks in
+// a fixed order (deterministic for a given box).
 //
 // Partial / result layout (doubles):
 //   0 max |u|^2 (compat)    1 #phi>=0 (compat)   2..4 sum u over phi>=0 (compat)
@@ -14,13 +14,17 @@
 //   7 sum phi   8 sum rho   9..11 sum rho u   12 #phi>=0   13 max |u|^2
 //   14 #non-finite nodes    15 unused
 // "compat" skips the planes x = 0, nx-1 and y = 0, ny-1 like the reference.
+#include <algorithm>
+
 #include "lbm_internal.h"
 
 namespace lbm {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMaxBlocks = 152 * 8;
+constexpr int SX = 32, SY = kThreads / 32;   // columns of a block's tile
+constexpr int kBlocksPerSm = 3;              // resident blocks the launch bounds ask for (80 registers)
+constexpr int kMaxBlocks = 152 * kBlocksPerSm;
 constexpr float kInv6 = 0.16666666666666666667f;
 constexpr float kInv12 = 0.08333333333333333333f;
 
@@ -30,42 +34,10 @@ struct StatsConst {
     float alpha, kappa, phiStarSq;
 };
 
+__device__ __forceinline__ bool is_max(int v) { return v == 0 || v == 13; }
+
 // row index of (y, z)
 __device__ __forceinline__ int kk_row(int y, int z, int ny) { return y + ny * z; }
-
-__device__ __forceinline__ double warp_sum(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ __forceinline__ double warp_max(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// Block-wide reduction of acc[0..kStatsValues) (entries 0 and 13 by max, the
-// rest by sum); thread 0 writes the result to out.
-__device__ void block_reduce(double (&acc)[kStatsValues], double *out)
-{
-    __shared__ double red[kThreads / 32][kStatsValues];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int v = 0; v < kStatsValues; v++) {
-        const double r = (v == 0 || v == 13) ? warp_max(acc[v]) : warp_sum(acc[v]);
-        if (lane == 0) red[warp][v] = r;
-    }
-    __syncthreads();
-    if (threadIdx.x < kStatsValues) {
-        const int v = threadIdx.x;
-        double r = red[0][v];
-        for (int w = 1; w < kThreads / 32; w++) r = (v == 0 || v == 13) ? fmax(r, red[w][v]) : r + red[w][v];
-        out[v] = r;
-    }
-}
 
 // Compensated float accumulator: the sum is hi + lo.  The _rn intrinsics keep
 // the compiler from contracting the two-sum's operations into FMAs, which
@@ -86,109 +58,241 @@ struct Sum2 {
         add(p);
         lo = __fadd_rn(lo, fmaf(a, b, -p));
     }
-    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
 
-// One block works on whole x-rows (row r = y + ny z, grid-stride over rows);
-// |u|^2 and the pressure are evaluated in float as the reference does
-// (src/stats.c:45, src/logsave.c:94-137); sums are compensated, counts exact.
-// phi_lo / phi_hi: the phi planes just below and above a z-slab (NULL for a
-// periodic box, whose z neighbours wrap).
-__global__ void __launch_bounds__(kThreads) stats_kernel(Box b, StatsConst c, const float *__restrict__ phi,
-                                                         const float *__restrict__ rho, const float *__restrict__ ux,
-                                                         const float *__restrict__ uy, const float *__restrict__ uz,
-                                                         double *__restrict__ partials,
-                                                         const float *__restrict__ phi_lo = nullptr,
-                                                         const float *__restrict__ phi_hi = nullptr)
+// (h, l) += (h2, l2) of float pairs
+__device__ __forceinline__ void pair_add(float &h, float &l, float h2, float l2)
 {
-    Sum2 sum[kStatsValues];
+    const float s = __fadd_rn(h, h2);
+    const float bp = __fsub_rn(s, h);
+    l = __fadd_rn(__fadd_rn(l, l2), __fadd_rn(__fsub_rn(h, __fsub_rn(s, bp)), __fsub_rn(h2, bp)));
+    h = s;
+}
+
+// What a node needs of one plane of phi for the 19-point Laplacian, the
+// gradient and its own value: with f4 = e + w + n + s and e4 the four diagonal
+// neighbours of the plane, the Laplacian sums to
+//   (e4 + 2 f4 - 24 c) of its own plane + (f4 + 2 c) of the planes above and below,
+// and the gradient components likewise (src/logsave.c:94-127 regrouped by
+// plane): marching in z reads 9 values per node instead of 19.
+struct Plane {
+    float c, a, fx, fy;       // centre; f4 + 2 c; e - w; n - s
+    float mid, gx, gy;        // e4 + 2 f4 - 24 c; own-plane parts of the x and y gradient
+};
+
+// One block: eight warps, a 32 x 8 tile of columns; item `it` is one tile and
+// a run of kz planes, which every thread marches at its column.  Plane z + 2
+// of phi and plane z + 1 of the other fields are loaded while plane z is
+// computed.  |u|^2 and the pressure are evaluated in float as the reference
+// does (src/stats.c:45, src/logsave.c:94-137); sums are compensated, counts
+// exact.  phi_lo / phi_hi: the phi planes just below and above a z-slab (NULL
+// for a periodic box, whose z neighbours wrap).  The pressure is summed over
+// the reference's region only, so x and y need no wrap.
+//
+// Bound by instruction issue: the 20 bytes a node must be read take 49 us at
+// 256^3 at the copy bandwidth, the kernel's 223 instructions per node (100 of
+// them FP32, 51 in the compensated sums of a node outside the bubbles) 97 us
+// at one per cycle and scheduler; 72% of the cycles issue.  Measured, 256^3:
+// 351 -> 136 us, 32^3 with the fold 78 -> 12 us, against one thread per node reading 19
+// points, with 15 FP64 values per thread reduced over the block (FP64 runs at
+// a 60th of the FP32 rate: that reduction was most of a small box's time).
+// Two nodes a thread in f32x2 was slower (143 us: the packed operations issue
+// at half rate and their constants take register pairs); four resident blocks
+// (64 registers, spills) 175 us.
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm)
+stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__restrict__ rho,
+             const float *__restrict__ ux, const float *__restrict__ uy, const float *__restrict__ uz,
+             double *__restrict__ partials, const float *__restrict__ phi_lo, const float *__restrict__ phi_hi, int kz,
+             int items)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ntx = (b.nx + SX - 1) / SX, nty = (b.ny + SY - 1) / SY;
+    const unsigned nx = (unsigned)b.nx, nxy = (unsigned)b.nxy;
+    Sum2 s_phi, s_rho, s_mx, s_my, s_mz, s_ux, s_uy, s_uz, s_in, s_out;
     unsigned cnt_in = 0, cnt_all = 0, cnt_bad = 0;
     float umax_c = 0.f, umax_all = 0.f;
 
-    const int nx = b.nx, ny = b.ny, nz = b.nz;
-    const int rows = ny * nz;
-    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-        const int k = r / ny, j = r - k * ny;
-        const bool row_in = j >= 1 && j <= ny - 2;   // reference region in y
-        const int jn = j == ny - 1 ? 0 : j + 1, js = j == 0 ? ny - 1 : j - 1;
-        const int kt = k == nz - 1 ? 0 : k + 1, kb = k == 0 ? nz - 1 : k - 1;
-        const size_t row_c = (size_t)r * nx;
-        const size_t row_n = ((size_t)kk_row(jn, k, ny)) * nx, row_s = ((size_t)kk_row(js, k, ny)) * nx;
-        // the planes above and below: the neighbouring slab's at a slab's edge
-        const float *pt = (k == nz - 1 && phi_hi) ? phi_hi : phi + (size_t)kt * b.nxy;
-        const float *pb = (k == 0 && phi_lo) ? phi_lo : phi + (size_t)kb * b.nxy;
-        const float *rt = pt + (size_t)j * nx, *rb = pb + (size_t)j * nx;
-        const float *rnt = pt + (size_t)jn * nx, *rsb = pb + (size_t)js * nx;
-        const float *rnb = pb + (size_t)jn * nx, *rst = pt + (size_t)js * nx;
-        for (int i = threadIdx.x; i < nx; i += blockDim.x) {
-            const size_t t = row_c + i;
-            const float ph = phi[t], rh = rho[t], vx = ux[t], vy = uy[t], vz = uz[t];
-            if (!(isfinite(ph) && isfinite(rh) && isfinite(vx) && isfinite(vy) && isfinite(vz))) {
-                cnt_bad++;
-                continue;
-            }
-            const float u2 = vx * vx + vy * vy + vz * vz;
-            sum[7].add(ph);
-            sum[8].add(rh);
-            sum[9].add_product(rh, vx);
-            sum[10].add_product(rh, vy);
-            sum[11].add_product(rh, vz);
-            if (ph >= 0.f) cnt_all++;
-            umax_all = fmaxf(umax_all, u2);
-            if (!row_in || i < 1 || i > nx - 2) continue;
-            umax_c = fmaxf(umax_c, u2);
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+        const int tile = it % (ntx * nty), z0 = (it / (ntx * nty)) * kz;
+        const int x = (tile % ntx) * SX + lane, y = (tile / ntx) * SY + warp;
+        if (x >= b.nx || y >= b.ny) continue;   // (no barrier in this loop)
+        const bool region = x >= 1 && x <= b.nx - 2 && y >= 1 && y <= b.ny - 2;
+        const unsigned xy = (unsigned)y * nx + (unsigned)x;
+        const int n_z = min(kz, b.nz - z0);
 
-            const int ie = i == nx - 1 ? 0 : i + 1, iw = i == 0 ? nx - 1 : i - 1;
-            const float p01 = phi[row_c + ie], p02 = phi[row_c + iw], p03 = phi[row_n + i], p04 = phi[row_s + i];
-            const float p05 = rt[i], p06 = rb[i], p07 = phi[row_n + ie], p08 = phi[row_s + iw];
-            const float p09 = phi[row_s + ie], p10 = phi[row_n + iw], p11 = rt[ie], p12 = rb[iw];
-            const float p13 = rb[ie], p14 = rt[iw], p15 = rnt[i], p16 = rsb[i];
-            const float p17 = rnb[i], p18 = rst[i];
-            const float lap = (p07 + p08 + p09 + p10 + p11 + p12 + p13 + p14 + p15 + p16 + p17 + p18
-                               + 2.f * (p01 + p02 + p03 + p04 + p05 + p06 - 12.f * ph)) * kInv6;
-            const float gx = (2.f * (p01 - p02) + p07 - p08 + p09 - p10 + p11 - p12 + p13 - p14) * kInv12;
-            const float gy = (2.f * (p03 - p04) + p07 - p08 + p10 - p09 + p15 - p16 + p17 - p18) * kInv12;
-            const float gz = (2.f * (p05 - p06) + p11 - p12 + p14 - p13 + p15 - p16 + p18 - p17) * kInv12;
-            const float ph2 = ph * ph;
-            const float pres = c.alpha * (ph2 * (3.f * ph2 - 2.f * c.phiStarSq) - c.phiStarSq * c.phiStarSq)
-                               - c.kappa * (ph * lap - 0.5f * (gx * gx + gy * gy + gz * gz)) + kCsSq * rh;
-            if (ph >= 0.f) {
-                cnt_in++;
-                sum[2].add(vx);
-                sum[3].add(vy);
-                sum[4].add(vz);
-                sum[5].add(pres);
-            } else {
-                sum[6].add(pres);
+        // phi around (x, y) on plane z (one past the box: its periodic or ghost neighbour)
+        float r[9];
+        auto load_phi = [&](int z) {
+            const float *p = phi;
+            unsigned t = xy;
+            if (z < 0 && phi_lo) p = phi_lo;
+            else if (z >= b.nz && phi_hi) p = phi_hi;
+            else t += (unsigned)(z < 0 ? b.nz - 1 : (z >= b.nz ? 0 : z)) * nxy;
+            const float *m = p + t;
+            r[0] = __ldg(m);
+            if (region) {
+                const float *n = p + (t + nx), *s = p + (t - nx);
+                r[1] = __ldg(m + 1);
+                r[2] = __ldg(m - 1);
+                r[3] = __ldg(n);
+                r[4] = __ldg(s);
+                r[5] = __ldg(n + 1);
+                r[6] = __ldg(s - 1);
+                r[7] = __ldg(s + 1);
+                r[8] = __ldg(n - 1);
             }
+        };
+        auto derive = [&]() -> Plane {
+            Plane p;
+            p.c = r[0];
+            const float f4 = (r[1] + r[2]) + (r[3] + r[4]);
+            const float d1 = r[5] - r[6], d2 = r[7] - r[8];
+            p.fx = r[1] - r[2];
+            p.fy = r[3] - r[4];
+            p.a = fmaf(2.f, r[0], f4);
+            p.mid = fmaf(2.f, fmaf(-12.f, r[0], f4), (r[5] + r[6]) + (r[7] + r[8]));
+            p.gx = fmaf(2.f, p.fx, d1 + d2);
+            p.gy = fmaf(2.f, p.fy, d1 - d2);
+            return p;
+        };
+        float f_rho, f_ux, f_uy, f_uz;
+        auto load_fields = [&](int z) {
+            const unsigned t = (unsigned)z * nxy + xy;
+            f_rho = __ldg(rho + t);
+            f_ux = __ldg(ux + t);
+            f_uy = __ldg(uy + t);
+            f_uz = __ldg(uz + t);
+        };
+
+#pragma unroll
+        for (int k = 1; k < 9; k++) r[k] = 0.f;   // (outside the region: not used)
+        load_phi(z0 - 1);
+        const Plane below = derive();
+        float a_b = below.a, fx_b = below.fx, fy_b = below.fy;
+        load_phi(z0);
+        Plane cur = derive();
+        load_phi(z0 + 1);
+        load_fields(z0);
+        for (int k = 0; k < n_z; k++) {
+            const Plane top = derive();
+            const float ph = cur.c, rh = f_rho, vx = f_ux, vy = f_uy, vz = f_uz;
+            if (k + 1 < n_z) {
+                load_phi(z0 + k + 2);
+                load_fields(z0 + k + 1);
+            }
+            // 0 * x summed over the fields is 0 if all are finite, else NaN
+            const float t =
+                fmaf(0.f, vz, fmaf(0.f, vy, fmaf(0.f, vx, fmaf(0.f, rh, __fmul_rn(0.f, ph)))));
+            if (t == 0.f) {
+                const float u2 = fmaf(vz, vz, fmaf(vy, vy, vx * vx));
+                s_phi.add(ph);
+                s_rho.add(rh);
+                s_mx.add_product(rh, vx);
+                s_my.add_product(rh, vy);
+                s_mz.add_product(rh, vz);
+                const bool heavy = ph >= 0.f;
+                cnt_all += heavy;
+                umax_all = fmaxf(umax_all, u2);
+                if (region) {
+                    umax_c = fmaxf(umax_c, u2);
+                    const float lap = ((cur.mid + top.a) + a_b) * kInv6;
+                    // 12 grad; z: 2 (ct - cb) + f4t - f4b, with a = f4 + 2 c
+                    const float gx = cur.gx + (top.fx + fx_b), gy = cur.gy + (top.fy + fy_b), gz = top.a - a_b;
+                    const float ph2 = ph * ph;
+                    const float bulk = fmaf(ph2, fmaf(3.f, ph2, -2.f * c.phiStarSq), -c.phiStarSq * c.phiStarSq);
+                    const float g2 = fmaf(gz, gz, fmaf(gy, gy, gx * gx));
+                    const float surf = fmaf(-0.5f * kInv12 * kInv12, g2, ph * lap);
+                    const float pres = fmaf(kCsSq, rh, fmaf(c.alpha, bulk, -c.kappa * surf));
+                    cnt_in += heavy;
+                    if (heavy) {
+                        s_ux.add(vx);
+                        s_uy.add(vy);
+                        s_uz.add(vz);
+                        s_in.add(pres);
+                    } else {
+                        s_out.add(pres);
+                    }
+                }
+            } else {
+                cnt_bad++;
+            }
+            a_b = cur.a;
+            fx_b = cur.fx;
+            fy_b = cur.fy;
+            cur = top;
         }
     }
-    double acc[kStatsValues];
+
+    // The block's sums.  Ten float pairs per thread through a recursive halving
+    // over the warp (16 value slots: after offsets 16, 8, 4, 2 a lane holds one
+    // value of 16 lanes, then offset 1), 16 pair additions per thread instead of
+    // 50, and no FP64 until one value per warp is left.
+    float h[16], l[16];
+    const Sum2 *const all[10] = {&s_ux, &s_uy, &s_uz, &s_in, &s_out, &s_phi, &s_rho, &s_mx, &s_my, &s_mz};
 #pragma unroll
-    for (int v = 0; v < kStatsValues; v++) acc[v] = sum[v].value();
-    acc[0] = umax_c;
-    acc[1] = cnt_in;
-    acc[12] = cnt_all;
-    acc[13] = umax_all;
-    acc[14] = cnt_bad;
-    acc[15] = 0.0;
-    block_reduce(acc, partials + (size_t)blockIdx.x * kStatsValues);
+    for (int v = 0; v < 16; v++) {
+        h[v] = v < 10 ? all[v < 10 ? v : 0]->hi : 0.f;
+        l[v] = v < 10 ? all[v < 10 ? v : 0]->lo : 0.f;
+    }
+#pragma unroll
+    for (int half = 8; half >= 1; half >>= 1) {
+        const bool up = lane & (2 * half);
+#pragma unroll
+        for (int v = 0; v < half; v++) {
+            const float gh = __shfl_xor_sync(0xffffffffu, up ? h[v] : h[v + half], 2 * half);
+            const float gl = __shfl_xor_sync(0xffffffffu, up ? l[v] : l[v + half], 2 * half);
+            h[v] = up ? h[v + half] : h[v];
+            l[v] = up ? l[v + half] : l[v];
+            pair_add(h[v], l[v], gh, gl);
+        }
+    }
+    pair_add(h[0], l[0], __shfl_xor_sync(0xffffffffu, h[0], 1), __shfl_xor_sync(0xffffffffu, l[0], 1));
+    cnt_in = __reduce_add_sync(0xffffffffu, cnt_in);
+    cnt_all = __reduce_add_sync(0xffffffffu, cnt_all);
+    cnt_bad = __reduce_add_sync(0xffffffffu, cnt_bad);
+    // |u|^2 >= 0: floats order like their bits
+    const unsigned mx_c = __reduce_max_sync(0xffffffffu, __float_as_uint(umax_c));
+    const unsigned mx_a = __reduce_max_sync(0xffffffffu, __float_as_uint(umax_all));
+    __shared__ double red[kThreads / 32][kStatsValues];
+    // lane 2 v (of each pair of lanes) holds sum v: result entries 2..6 and 7..11
+    if ((lane & 1) == 0 && lane < 20) red[warp][2 + (lane >> 1)] = (double)h[0] + (double)l[0];
+    if (lane == 31) {
+        red[warp][0] = __uint_as_float(mx_c);
+        red[warp][1] = cnt_in;
+        red[warp][12] = cnt_all;
+        red[warp][13] = __uint_as_float(mx_a);
+        red[warp][14] = cnt_bad;
+        red[warp][15] = 0.0;
+    }
+    __syncthreads();
+    if (threadIdx.x < kStatsValues) {
+        const int v = threadIdx.x;
+        double s = red[0][v];
+        for (int w = 1; w < kThreads / 32; w++) s = is_max(v) ? fmax(s, red[w][v]) : s + red[w][v];
+        partials[(size_t)blockIdx.x * kStatsValues + v] = s;
+    }
 }
 
+// The blocks' partials in a fixed order: thread (row group, value) sums every
+// 16th row, then the 16 groups in order.
 __global__ void __launch_bounds__(kThreads) fold_kernel(const double *__restrict__ partials, int nparts,
                                                         double *__restrict__ out)
 {
-    double acc[kStatsValues];
-#pragma unroll
-    for (int v = 0; v < kStatsValues; v++) acc[v] = 0.0;
-    for (int p = threadIdx.x; p < nparts; p += blockDim.x) {
-#pragma unroll
-        for (int v = 0; v < kStatsValues; v++) {
-            const double x = partials[(size_t)p * kStatsValues + v];
-            acc[v] = (v == 0 || v == 13) ? fmax(acc[v], x) : acc[v] + x;
-        }
+    constexpr int kGroups = kThreads / kStatsValues;
+    __shared__ double red[kGroups][kStatsValues];
+    const int v = threadIdx.x % kStatsValues, grp = threadIdx.x / kStatsValues;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int p = grp; p < nparts; p += kGroups) {
+        const double x = partials[(size_t)p * kStatsValues + v];
+        acc = is_max(v) ? fmax(acc, x) : acc + x;
     }
-    block_reduce(acc, out);
+    red[grp][v] = acc;
+    __syncthreads();
+    if (grp == 0) {
+        for (int g = 1; g < kGroups; g++) acc = is_max(v) ? fmax(acc, red[g][v]) : acc + red[g][v];
+        out[v] = acc;
+    }
 }
 
 // Pressure of every node (src/vtksave.c:63-127): the same float expression as
@@ -228,30 +332,46 @@ __global__ void __launch_bounds__(kThreads) pressure_kernel(Box b, StatsConst c,
     }
 }
 
-unsigned stats_blocks(const Box &b)
+// How a box is cut: items of one tile and kz planes, the deepest (up to 16)
+// that still give every resident block four of them, so that uneven items
+// even out; a small box takes single planes.
+struct Cut {
+    int kz, items, blocks;
+};
+Cut stats_cut(const Box &b)
 {
-    long long blocks = (long long)b.ny * b.nz;   // one x-row per block and pass
-    if (blocks > kMaxBlocks) blocks = kMaxBlocks;
-    return (unsigned)(blocks < 1 ? 1 : blocks);
+    const long long tiles = (long long)((b.nx + SX - 1) / SX) * ((b.ny + SY - 1) / SY);
+    auto items_of = [&](int kz) { return tiles * ((b.nz + kz - 1) / kz); };
+    int kz = 16;
+    while (kz > 1 && items_of(kz) < 4 * kMaxBlocks) kz /= 2;
+    const long long items = items_of(kz);
+    return Cut{kz, (int)items, (int)std::min<long long>(items, kMaxBlocks)};
+}
+
+cudaError_t launch_stats_kernels(const Box &b, const StatsConst &c, const float *const f[5], const float *phi_lo,
+                                 const float *phi_hi, double *partials, double *result, cudaStream_t s)
+{
+    const Cut k = stats_cut(b);
+    stats_kernel<<<(unsigned)k.blocks, kThreads, 0, s>>>(b, c, f[0], f[1], f[2], f[3], f[4], partials, phi_lo,
+                                                         phi_hi, k.kz, k.items);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    fold_kernel<<<1, kThreads, 0, s>>>(partials, k.blocks, result);
+    return cudaGetLastError();
 }
 
 }  // namespace
 
-size_t stats_partial_count(const Box &b) { return stats_blocks(b); }
+size_t stats_partial_count(const Box &b) { return (size_t)stats_cut(b).blocks; }
 
 cudaError_t launch_stats(const Box &b, const lbm_derived &d, const float *mom, double *partials,
-                         size_t partial_count, double *result, unsigned long long *, cudaStream_t s,
-                         const float *phi_lo, const float *phi_hi)
+                         size_t partial_count, double *result, cudaStream_t s, const float *phi_lo,
+                         const float *phi_hi)
 {
-    const unsigned blocks = stats_blocks(b);
-    if (partial_count < blocks) return cudaErrorInvalidValue;
-    StatsConst c{d.alpha, d.kappa, d.phiStarSq};
-    stats_kernel<<<blocks, kThreads, 0, s>>>(b, c, mom, mom + b.n, mom + 2 * b.n, mom + 3 * b.n, mom + 4 * b.n,
-                                             partials, phi_lo, phi_hi);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    fold_kernel<<<1, kThreads, 0, s>>>(partials, (int)blocks, result);
-    return cudaGetLastError();
+    if (partial_count < stats_partial_count(b)) return cudaErrorInvalidValue;
+    const float *f[5];
+    for (int a = 0; a < 5; a++) f[a] = mom + (size_t)a * b.n;
+    return launch_stats_kernels(b, StatsConst{d.alpha, d.kappa, d.phiStarSq}, f, phi_lo, phi_hi, partials, result, s);
 }
 
 cudaError_t launch_pressure(const Box &b, const lbm_derived &d, const float *mom, float *out, cudaStream_t s)
@@ -279,11 +399,11 @@ cudaError_t launch_pressure(const Box &b, const lbm_derived &d, const float *mom
 // already owns; this entry point adds nothing to them.
 //
 // The per-block partial sums live in a fixed array in the library's static
-// device memory (1 MiB, reserved on every GPU that loads the library until the
-// process exits).  One block reduces 16384 nodes, so the array holds the
-// partials of at most 512^3 nodes; larger boxes are rejected.  Every row the
-// final fold reads is written earlier in the same call, so no part of the
-// array has to be cleared between calls.  All calls share the array: two calls
+// device memory (57 KiB, one row per resident block, reserved on every GPU that
+// loads the library until the process exits).  Boxes of more than 512^3 nodes
+// are rejected (LBM_NOALLOC_MAX_NODES).  Every row the final fold reads is
+// written earlier in the same call, so no part of the array has to be cleared
+// between calls.  All calls share the array: two calls
 // whose kernels overlap on the GPU (different streams, or different host
 // threads on one device) race on it and must be ordered by the caller.
 // ---------------------------------------------------------------------------
@@ -292,12 +412,9 @@ cudaError_t launch_pressure(const Box &b, const lbm_derived &d, const float *mom
 namespace lbm {
 namespace {
 
-constexpr int kNoAllocNodesPerBlock = kThreads * 64;
 constexpr long long kNoAllocMaxNodes = LBM_NOALLOC_MAX_NODES;
-constexpr int kNoAllocRows = (int)(kNoAllocMaxNodes / kNoAllocNodesPerBlock);
-static_assert(kNoAllocMaxNodes % kNoAllocNodesPerBlock == 0, "whole rows");
 
-static __device__ __align__(256) double g_noalloc_partials[kNoAllocRows * kStatsValues];
+static __device__ __align__(256) double g_noalloc_partials[kMaxBlocks * kStatsValues];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mutex;
@@ -364,15 +481,9 @@ extern "C" int lbm_stats_noalloc(const lbm_params *p, const float *phi, const fl
         b.nz = p->nz;
         b.nxy = (long long)p->nx * p->ny;
         b.n = n;
-        const unsigned blocks = (unsigned)((n + lbm::kNoAllocNodesPerBlock - 1) / lbm::kNoAllocNodesPerBlock);
-        const cudaStream_t s = static_cast<cudaStream_t>(stream);
-        lbm::StatsConst c{d.alpha, d.kappa, d.phiStarSq};
-        lbm::stats_kernel<<<blocks, lbm::kThreads, 0, s>>>(b, c, phi, rho, ux, uy, uz, scratch);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) {
-            lbm::fold_kernel<<<1, lbm::kThreads, 0, s>>>(scratch, (int)blocks, raw_out);
-            e = cudaGetLastError();
-        }
+        const float *f[5] = {phi, rho, ux, uy, uz};
+        e = lbm::launch_stats_kernels(b, lbm::StatsConst{d.alpha, d.kappa, d.phiStarSq}, f, nullptr, nullptr, scratch,
+                                      raw_out, static_cast<cudaStream_t>(stream));
     }
     if (switch_device && have_prev) cudaSetDevice(prev);
     if (e != cudaSuccess) {
