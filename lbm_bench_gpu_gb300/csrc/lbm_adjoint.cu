@@ -114,8 +114,8 @@ struct Adjoint {
     // double-buffered by step parity so that the side stream can prepare
     // step n while the main stream still runs step n + 1
     float *phi = nullptr;     // 2 x n
-    float *lam[2] = {nullptr, nullptr};   // 26 x n each: f (7) then g (19)
-    float *lst[2] = {nullptr, nullptr};
+    // lambda: L, the 19 lg and, when tauPhi is not 1, the seven q (AdjointBuffers)
+    float *lam_L[2] = {nullptr, nullptr}, *lam_g[2] = {nullptr, nullptr}, *lam_q[2] = {nullptr, nullptr};
     float4 *lsrc = nullptr;
     float *phi0 = nullptr, *mom_save = nullptr;
     double *partials = nullptr, *dgrav = nullptr, *ab = nullptr, *acc = nullptr;
@@ -124,7 +124,7 @@ struct Adjoint {
     unsigned char *host = nullptr;    // pinned host checkpoints (second tier), slot layout
     std::vector<Snapshot> hsnaps;
     std::vector<int> free_slots;
-    int cur = 0;                 // lam[cur] holds lambda^{k+1}
+    int cur = 0;                 // lam_*[cur] hold lambda^{k+1}
     bool lambda_ready = false;
     long long fwd_steps = 0, adj_steps = 0;
     lbm::StepConst k;
@@ -322,11 +322,13 @@ struct Adjoint {
             e = lbm::launch_objective(c->box, o.objective, c->d.phiStar, scale, c->q, st, ph, partials, abT, acc,
                                       c->stream);
             if (e == cudaSuccess)
-                e = lbm::launch_source_init(c->box, o.objective, scale, abT, c->d.phiStar, c->q, st, ph, lam[cur],
-                                            lam[cur] + lbm::kQf * n, lst[cur], c->stream);
+                e = lbm::launch_source_init(c->box, o.objective, scale, abT, c->d.phiStar, c->q, st, ph, lam_q[cur],
+                                            lam_g[cur], lam_L[cur], c->stream);
         } else {
-            e = cudaMemsetAsync(lam[cur], 0, sizeof(float) * (lbm::kQf + lbm::kQg) * n, c->stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(lst[cur], 0, sizeof(float) * n, c->stream);
+            e = cudaMemsetAsync(lam_g[cur], 0, sizeof(float) * lbm::kQg * n, c->stream);
+            if (e == cudaSuccess) e = cudaMemsetAsync(lam_L[cur], 0, sizeof(float) * n, c->stream);
+            if (e == cudaSuccess && lam_q[cur])
+                e = cudaMemsetAsync(lam_q[cur], 0, sizeof(float) * lbm::kQf * n, c->stream);
         }
         if (e != cudaSuccess) return cuda_fail(e, "adjoint: terminal source");
         if (side) {
@@ -358,12 +360,12 @@ struct Adjoint {
         if (e != cudaSuccess) return cuda_fail(e, "adjoint: side stream");
         lbm::AdjointBuffers a;
         a.phi = ph;
-        a.lf_in = lam[cur];
-        a.lg_in = lam[cur] + lbm::kQf * n;
-        a.lst_in = lst[cur];
-        a.lf_out = lam[1 - cur];
-        a.lg_out = lam[1 - cur] + lbm::kQf * n;
-        a.lst_out = lst[1 - cur];
+        a.lq_in = lam_q[cur];
+        a.lg_in = lam_g[cur];
+        a.L_in = lam_L[cur];
+        a.lq_out = lam_q[1 - cur];
+        a.lg_out = lam_g[1 - cur];
+        a.L_out = lam_L[1 - cur];
         a.lsrc = lsrc;
         a.dgrav = dgrav;
         a.ab = abs_;
@@ -547,10 +549,11 @@ struct Adjoint {
         ab = w.take<double>(8);
         acc = w.take<double>(2);
         if (!gradient) return;
-        lam[0] = w.take<float>((size_t)(lbm::kQf + lbm::kQg) * n);
-        lam[1] = w.take<float>((size_t)(lbm::kQf + lbm::kQg) * n);
-        lst[0] = w.take<float>(n);
-        lst[1] = w.take<float>(n);
+        for (int i = 0; i < 2; i++) {
+            lam_g[i] = w.take<float>((size_t)lbm::kQg * n);
+            lam_L[i] = w.take<float>(n);
+            if (k.invTauPhiOne != 0.f) lam_q[i] = w.take<float>((size_t)lbm::kQf * n);
+        }
         lsrc = w.take<float4>(n);
         phi0 = w.take<float>(n);
         dgrav = w.take<double>(lbm::adjoint_dgrav_parts(c->box));
@@ -737,8 +740,8 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
     if (!rc) {
         e = lbm::launch_dgrav_fold(c->box, A.dgrav, A.acc, c->stream);
         if (e == cudaSuccess)
-            e = lbm::launch_init_adjoint(c->box, c->d, c->p.Gamma, A.phi0, A.lam[A.cur], A.lst[A.cur],
-                                         A.lam[A.cur] + lbm::kQf * n, lphi0, A.phi, c->stream);
+            e = lbm::launch_init_adjoint(c->box, c->d, c->p.Gamma, A.phi0, A.lam_q[A.cur], A.lam_L[A.cur],
+                                         A.lam_g[A.cur], lphi0, A.phi, c->stream);
         if (e != cudaSuccess) rc = cuda_fail(e, "lbm_step_adjoint: initial-state adjoint");
     }
     double acc[2] = {0.0, 0.0};

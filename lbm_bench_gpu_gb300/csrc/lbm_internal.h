@@ -99,16 +99,44 @@ struct NativeState {
     bool g_odd;               // g in the reversed layout (the next step is odd)
 };
 
-// Buffers of one adjoint step (FP32, n elements per field).
+// Buffers of one adjoint step (FP32, n elements per field).  lambda_f,i is
+// q_i + L with one L for the seven populations; the q_i = (1 - 1/tauPhi) lP_i
+// vanish when tauPhi is 1 and their buffers are NULL then.
 struct AdjointBuffers {
     const float *phi;                  // phi of s^n
-    const float *lf_in, *lg_in;        // lambda^{n+1} (f part without its stencil term)
-    const float *lst_in;               //   stencil term of lambda^{n+1}, common to the 7 f fields
-    float *lf_out, *lg_out, *lst_out;  // lambda^n
+    const float *lq_in, *lg_in, *L_in; // lambda^{n+1}
+    float *lq_out, *lg_out, *L_out;    // lambda^n
     float4 *lsrc;                      // scratch per node: (lambda_lap, mu lambda_F)
     double *dgrav;                     // per-warp running sums of the dJ/dgrav terms
     const double *ab;                  // objective sums of s^n
 };
+
+// Planes per block of a kernel whose blocks march `planes` planes on `tiles`
+// column tiles, per_sm of them resident on each of sms SMs.  A block's time is
+// about (tz + prologue) plane-times, and r blocks that share an SM slow each
+// other down by share[r] (less than r: a lone block is bound by its own
+// latencies).  The launch takes as many full rounds of resident blocks as there
+// are, then a last, partly filled one, which overlaps the end of the others
+// (tail).  The depth that minimises the sum is taken.
+inline int march_depth(long long tiles, int planes, int sms, int per_sm, double prologue, double tail,
+                       const double *share)
+{
+    const long long slots = (long long)sms * per_sm;
+    int best = 1;
+    double best_cost = -1.0;
+    for (int tz = 1; tz <= 64; tz++) {
+        const long long blocks = tiles * ((planes + tz - 1) / tz);
+        const long long full = blocks / slots, rest = blocks % slots;
+        double rounds = (double)full * share[per_sm];
+        if (rest > 0) rounds += (full > 0 ? tail : 1.0) * share[(rest + sms - 1) / sms];
+        const double cost = rounds * (tz + prologue);
+        if (best_cost < 0.0 || cost < best_cost) {
+            best_cost = cost;
+            best = tz;
+        }
+    }
+    return best;
+}
 
 void set_error(const std::string &msg);
 const std::string &last_error();
@@ -155,11 +183,10 @@ size_t stats_partial_count(const Box &b);
 cudaError_t launch_pressure(const Box &b, const lbm_derived &d, const float *mom, float *out, cudaStream_t s);
 
 // Adjoint (zsc_adjoint.cu).  acc[0] accumulates J, acc[1] dJ/dgrav (FP64).
-// All adjoint kernels run on one grid of 32 x 8 column tiles, each block
-// marching a few z planes; adjoint_blocks is its block count (the length of
-// the dgrav array, and half the length of the objective partials).
+// adjoint_blocks: blocks of the objective kernel's grid (half the length of
+// the objective partials).
 size_t adjoint_blocks(const Box &b);
-// Length of the dgrav array: one running sum per warp of the local kernel's grid.
+// Length of the dgrav array: one running sum per warp of the march kernel's grid.
 size_t adjoint_dgrav_parts(const Box &b);
 cudaError_t launch_adjoint_phi(const Box &b, float eta, const Quant &q, const NativeState &st, float *phi,
                                cudaStream_t s);
@@ -167,15 +194,15 @@ cudaError_t launch_objective(const Box &b, int objective, float phiStar, double 
                              const NativeState &st, const float *phi, double *partials, double *ab, double *acc,
                              cudaStream_t s);
 cudaError_t launch_source_init(const Box &b, int objective, double scale, const double *ab, float phiStar,
-                               const Quant &q, const NativeState &st, const float *phi, float *lf, float *lg,
-                               float *lst, cudaStream_t s);
+                               const Quant &q, const NativeState &st, const float *phi, float *lq, float *lg,
+                               float *L, cudaStream_t s);
 cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar, const Quant &q,
                                 const NativeState &st, const AdjointBuffers &a, bool add_source, int objective,
                                 double scale, cudaStream_t s);
 // acc[1] = sum of the per-warp dgrav sums.
 cudaError_t launch_dgrav_fold(const Box &b, const double *dgrav, double *acc, cudaStream_t s);
-cudaError_t launch_init_adjoint(const Box &b, const lbm_derived &d, float Gamma, const float *phi0, const float *lf,
-                                const float *lst, const float *lg, float *lphi0, float *llap, cudaStream_t s);
+cudaError_t launch_init_adjoint(const Box &b, const lbm_derived &d, float Gamma, const float *phi0, const float *lq,
+                                const float *L, const float *lg, float *lphi0, float *llap, cudaStream_t s);
 
 // Number of doubles produced by launch_stats in `result`.
 constexpr int kStatsValues = 16;

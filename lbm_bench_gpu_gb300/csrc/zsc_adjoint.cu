@@ -14,31 +14,26 @@
 //   stencil:  lambda_phi += L[lambda_lap] - sum_k D_k[lambda_grad_k]
 //             (the Laplacian stencil is symmetric, the gradient antisymmetric)
 //   moments:  lf_i += lambda_phi;  lg_i += lambda_rho + c_i . lambda_m
-// The stencil part is kept as a separate field lst (the same for all seven f
-// populations) and added when lambda is read.
+// All seven lf hold the same part: with a = 1 - 1/tauPhi, lf_i = q_i + L where
+// q_i = a lP_i of the step before and L = lambda_phi + the stencil part.  So
+// lambda is kept as L (one field), lg (19) and, only when tauPhi is not 1, the
+// seven q_i.
 //
 // The forward state is read where the step kernel keeps it (a checkpoint slot
 // or the context's buffers): f_0 FP32, f_1..f_6 post-collision (the eta-blend
 // is redone on read), g in the AA layout, 16-bit formats mapped back to FP32.
 // The collision's Jacobian needs g only through rho and the momentum, and f
 // only through phi, so only phi is materialised (the stencil needs it at the
-// neighbours).  Per step:
-//   adjoint_phi_kernel     s^n -> phi                          ~32 B/node (FP32)
-//   adjoint_local_kernel   lambda^{n+1}, s^n, phi -> lambda^n   ~320 B/node
-//                          and (lambda_lap, mu lambda_F) as one float4
-//   adjoint_stencil_kernel float4 -> lst                        ~20 B/node
+// neighbours).  Per step (bytes per node, FP32 / 16-bit state, tauPhi = 1):
+//   adjoint_phi_kernel     s^n -> phi                                 32 / 20
+//   adjoint_march_kernel   lambda^{n+1}, s^n, phi -> lg^n, lambda_phi
+//                          and (lambda_lap, mu lambda_F) as a float4  256 / 218
+//   adjoint_stencil_kernel float4, lambda_phi -> L^n                  24
 // All per-node arithmetic is FP32; the objective sums and dJ/dgrav are FP64.
-// Every kernel runs on one grid: 32 x 8 column tiles, each block marching
-// kPlanes (4) consecutive z planes (so the z neighbours of one plane are the
-// block's previous and next planes, mostly L1 hits), except the local kernel,
-// whose blocks take kLocalPlanes (2) planes gridDim.z apart (with consecutive
-// planes the compiler keeps more values live across iterations and spills),
-// with the next plane's rows prefetched into L2.  Measured at 128^3 (T = 2000,
-// 40 GB): 1, 2, 4 local planes -> adjoint/forward 4.06, 3.99, 4.09 (and, later,
-// 3.92, 3.81, 3.87; at 256^3 with an FP16 state, T = 400: 6.21, 6.07, 6.12);
-// 8 and 16 stencil planes are slower.  32-bit node indices (n * 19 < 2^32 is checked at
-// init).
+// The kernels work on 32 x 8 column tiles, each block marching z planes.
+// 32-bit node indices (n * 19 < 2^32 is checked at init).
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 
 #include "lattice.cuh"
@@ -50,26 +45,7 @@ constexpr int TXA = 32, TYA = 8, NTA = TXA * TYA;
 #ifndef ZSC_ADJ_PLANES
 #define ZSC_ADJ_PLANES 4
 #endif
-// Resident blocks per SM the local kernel's launch bounds ask for: 3 (80
-// registers) for an FP32 state, 4 (64 registers, ~100 bytes spilled) for a
-// 16-bit state, whose two-byte gathers leave more latency to hide.  Measured
-// (adjoint / forward wall time): 256^3 FP16 state, T = 400, 40 GB: 2, 3, 4
-// blocks -> 6.18, 6.07, 5.79; 128^3 FP32 state, T = 2000, 40 GB: 4.03, 3.81,
-// 3.92.  ZSC_ADJ_MIN_BLOCKS overrides both.
-template <typename ST>
-constexpr int adj_min_blocks()
-{
-#ifdef ZSC_ADJ_MIN_BLOCKS
-    return ZSC_ADJ_MIN_BLOCKS;
-#else
-    return sizeof(ST) == 2 ? 4 : 3;
-#endif
-}
-#ifndef ZSC_ADJ_LOCAL_PLANES
-#define ZSC_ADJ_LOCAL_PLANES 2
-#endif
 constexpr int kPlanes = ZSC_ADJ_PLANES;
-constexpr int kLocalPlanes = ZSC_ADJ_LOCAL_PLANES;   // planes per block of the local kernel
 constexpr float kInv6 = 0.16666666666666666667f;
 constexpr float kInv12 = 0.08333333333333333333f;
 constexpr float kW0 = 0.33333333333333333333f, kW1 = 0.05555555555555555556f, kW2 = 0.02777777777777777778f;
@@ -134,6 +110,30 @@ __device__ __forceinline__ void stencil19(const float *__restrict__ v, const Nb 
     gx = (2.f * (s[1] - s[2]) + s[7] - s[8] + s[9] - s[10] + s[11] - s[12] + s[13] - s[14]) * kInv12;
     gy = (2.f * (s[3] - s[4]) + s[7] - s[8] + s[10] - s[9] + s[15] - s[16] + s[17] - s[18]) * kInv12;
     gz = (2.f * (s[5] - s[6]) + s[11] - s[12] + s[14] - s[13] + s[15] - s[16] + s[18] - s[17]) * kInv12;
+}
+
+// What the 19-point stencils of a node take from one plane of phi (row pitch
+// PITCH), at the node p points to: the Laplacian sums to mid of the node's own
+// plane plus a of the planes above and below, and the gradient likewise.
+struct PlaneSums {
+    float c, a, fx, fy;    // centre; e + w + n + s + 2 c; e - w; n - s
+    float mid, gx, gy;     // corners + 2 (e + w + n + s) - 24 c; own-plane parts of the x and y gradient
+};
+template <int PITCH>
+__device__ __forceinline__ PlaneSums plane_sums(const float *p)
+{
+    const float e = p[1], w = p[-1], n = p[PITCH], s = p[-PITCH];
+    const float en = p[PITCH + 1], ws = p[-PITCH - 1], es = p[-PITCH + 1], wn = p[PITCH - 1];
+    PlaneSums r;
+    r.c = p[0];
+    const float f4 = (e + w) + (n + s), d1 = en - ws, d2 = es - wn;
+    r.fx = e - w;
+    r.fy = n - s;
+    r.a = f4 + 2.f * r.c;
+    r.mid = 2.f * (f4 - 12.f * r.c) + ((en + ws) + (es + wn));
+    r.gx = 2.f * r.fx + (d1 + d2);
+    r.gy = 2.f * r.fy + (d1 - d2);
+    return r;
 }
 
 // Per-field base pointers of a state (kernel parameters: a field's address is
@@ -310,8 +310,8 @@ template <typename ST, bool ODD>
 __global__ void __launch_bounds__(NTA) source_init_kernel(Box b, int objective, double scale,
                                                           const double *__restrict__ ab, float phiStar, Quant q,
                                                           const GFields g, const float *__restrict__ phi,
-                                                          float *__restrict__ lf, float *__restrict__ lg,
-                                                          float *__restrict__ lst)
+                                                          float *__restrict__ lq, float *__restrict__ lg,
+                                                          float *__restrict__ L)
 {
     const unsigned n = (unsigned)b.n;
     const SourceCoef k = source_coef(ab, phiStar);
@@ -322,11 +322,11 @@ __global__ void __launch_bounds__(NTA) source_init_kernel(Box b, int objective, 
         g_moments<ST, ODD>(g, q, state_neighbourhood<ST>(b, x, y, z), rho, m);
         float dphi, drho, dmz;
         objective_source(z, objective, k, phiStar, phi[t], rho, m[2], dphi, drho, dmz);
-#pragma unroll
-        for (int i = 0; i < kQf; i++) lf[i * n + t] = dphi;
+        L[t] = dphi;
+        if (lq)
+            for (int i = 0; i < kQf; i++) lq[i * n + t] = 0.f;
 #pragma unroll
         for (int i = 0; i < kQg; i++) lg[i * n + t] = drho + kCz(i) * dmz;
-        lst[t] = 0.f;
     }
 }
 
@@ -334,12 +334,13 @@ struct AdjIn {
     // per-field base pointers (kernel parameters: a field's address is one
     // multiply-add on the node index, with no i * n on the load's path)
     const void *g_f[kQg];                  // the state's g fields
-    const float *lf_f[kQf], *lg_f[kQg];    // lambda^{n+1}
-    float *lf_o[kQf], *lg_o[kQg];          // lambda^n
-    const void *g;                         // native g of s^n
+    const float *lg_f[kQg];                // lambda_g^{n+1}
+    float *lg_o[kQg];                      // lambda_g^n
+    const float *lq_f[kQf];                // q^{n+1} and q^n (tauPhi != 1 only)
+    float *lq_o[kQf];
     const float *phi;                      // phi of s^n
-    const float *lf, *lg, *lst;            // lambda^{n+1} (lf without its stencil part lst)
-    float *lf_out, *lg_out;                // lambda^n without its stencil part
+    const float *L;                        // L^{n+1}
+    float *lphi;                           // lambda_phi^n (L^n without its stencil part)
     float4 *lsrc;                          // (lambda_lap, mu lambda_F) at every node
     double *dgrav;                         // per warp of each block, accumulated over steps
     const double *ab;                      // objective sums of s^n (when add_source)
@@ -347,74 +348,237 @@ struct AdjIn {
     int objective, add_source;
 };
 
-// L2 prefetch of the block's tile rows of plane z in every field the local
-// kernel reads (lambda_g, lambda_f, lst, g, phi): one bulk prefetch per row
-// (128 B of floats, 32 storage elements of g), about 1.5 per thread.  The
-// kernel is latency-bound on its neighbour gathers; with the rows already on
-// their way to L2 they hit there.  The blocks of neighbouring tiles and planes
-// (which run at the same time) prefetch the halo rows.
-template <typename ST>
-__device__ __forceinline__ void prefetch_plane(const Box &b, const AdjIn &a, int z)
+__device__ __forceinline__ int wrap_to(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
+
+// 16-byte global -> shared copy, cached in L2 only; completes asynchronously.
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 {
-    constexpr int kFields = kQg + kQf + 1 + kQg + 1;
-    const unsigned n = (unsigned)b.n;
-    const int tid = threadIdx.y * TXA + threadIdx.x;
-    for (int r = tid; r < kFields * TYA; r += NTA) {
-        const int field = r / TYA;
-        const unsigned node =
-            (unsigned)z * (unsigned)b.nxy + (blockIdx.y * TYA + (unsigned)(r % TYA)) * (unsigned)b.nx + blockIdx.x * TXA;
-        const void *src;
-        unsigned bytes = TXA * sizeof(float);
-        if (field < kQg) {
-            src = a.lg + field * n + node;
-        } else if (field < kQg + kQf) {
-            src = a.lf + (field - kQg) * n + node;
-        } else if (field == kQg + kQf) {
-            src = a.lst + node;
-        } else if (field < 2 * kQg + kQf + 1) {
-            // the tile row's nodes in the state's layout: FP32 the node range;
-            // pair layout the 32 words holding them (and the other half's)
-            unsigned first = node, count = TXA;
-            if constexpr (sizeof(ST) == 2) {
-                const unsigned h = (unsigned)b.nx >> 1, x0 = blockIdx.x * TXA;
-                first = node - x0 + 2u * (x0 < h ? x0 : x0 - h);
-                count = 2 * TXA;
-            }
-            src = static_cast<const ST *>(a.g) + (field - kQg - kQf - 1) * n + first;
-            bytes = count * sizeof(ST);
-        } else {
-            src = a.phi + node;
-        }
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src), "r"(bytes) : "memory");
+    const unsigned sm = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sm), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+template <int I>
+struct Dir {
+    static constexpr int value = I;
+};
+// f(Dir<i>) for i = I, I + D, I + 2D, ... < 19
+template <int I, int D, typename F>
+__device__ __forceinline__ void for_dirs(F &&f)
+{
+    if constexpr (I < kQg) {
+        f(Dir<I>{});
+        for_dirs<I + D, D>(f);
+    }
+}
+// the same from the run-time first direction q < D (uniform per warp)
+template <int D, int Q = 0, typename F>
+__device__ __forceinline__ void for_dirs_of(int q, F &&f)
+{
+    if constexpr (Q < D) {
+        if (q == Q) for_dirs<Q, D>(f);
+        else for_dirs_of<D, Q + 1>(q, f);
     }
 }
 
+// Shared-memory geometry of the march kernel.  A tile is 32 nodes x 8 rows.
+// For an FP32 state the 32 nodes are consecutive; for a 16-bit state, kept in
+// the pair layout, they are the two nodes of 16 consecutive words (x = w and
+// x = w + nx/2: lanes 0..15 and 16..31), so that every staged byte of g is used.
+// The FP32 fields are then staged as two segments of 16 nodes, a segment's rows
+// kSeg floats apart with kSeg = 16 mod 32, which keeps the two half-warps in
+// different banks.
+template <typename ST>
+struct Geo {
+    static constexpr bool kPair = sizeof(ST) == 2;
+    static constexpr int SEGS = kPair ? 2 : 1;
+    static constexpr int W = TXA / SEGS;                // nodes of a segment
+    static constexpr int LP = W + 4;                    // lambda_g row: a chunk for the x-shifted nodes
+    static constexpr int LSEG = kQg * TYA * LP + (kPair ? 16 : 0);   // floats between segments
+    static constexpr int LSTAGE = SEGS * LSEG;          // floats per plane
+    static constexpr int GP = kPair ? 2 * (W + 4) : LP; // g row, elements
+    static constexpr int GSTAGE = kQg * TYA * GP;       // elements per plane
+    static constexpr int HP = W + 8;                    // phi / L row with its halo
+    static constexpr int HROWS = TYA + 2;
+    static constexpr int HSEG = HROWS * HP;             // (16-bit: 240 = 16 mod 32)
+    static constexpr int HPLANE = SEGS * HSEG;
+    static constexpr int HCHUNKS = HPLANE / 4;          // 16-byte chunks of a phi / L plane
+    static constexpr int L_OFF = 0;                     // bytes: [2][LSTAGE] floats
+    static constexpr int G_OFF = L_OFF + 2 * LSTAGE * 4;
+    static constexpr int PHI_OFF = G_OFF + 2 * GSTAGE * (int)sizeof(ST);   // [3][HPLANE] floats
+    static constexpr int LF_OFF = PHI_OFF + 3 * HPLANE * 4;                // [3][HPLANE] floats
+    static constexpr int SMEM = LF_OFF + 3 * HPLANE * 4;
+    static constexpr int GCH = kPair ? 4 : 8;           // chunks of an unshifted g row
+    static constexpr int GD = NTA / (TYA * GCH);        // directions the block stages at a time
+    static_assert(HCHUNKS <= NTA / 2, "one chunk of phi and of L per thread at most");
+    static_assert(G_OFF % 16 == 0 && PHI_OFF % 16 == 0 && LF_OFF % 16 == 0 && HPLANE % 4 == 0, "16-byte stages");
+};
+
 // The local part of one adjoint step (see the file comment).
-template <typename ST, bool ODD>
-__global__ void __launch_bounds__(NTA, adj_min_blocks<ST>()) adjoint_local_kernel(Box b, StepConst c, float phiStar, Quant q, AdjIn a)
+//
+// A block owns a 32 x 8 tile of columns and marches tz planes.  Everything a
+// node reads comes from shared memory, staged one plane ahead with 16-byte
+// cp.async copies (periodic in x and y by their addresses): the 19 lambda_g
+// rows the node's directions point to (x + c_i), the 19 g rows of the state
+// (own slots, or in the odd AA layout the reversed slots of x - c_i), and phi
+// and L on the tile plus one node; phi of the plane above is reduced to the
+// sums its stencils need (PlaneSums) once and carried down the march.
+template <typename ST, bool ODD, bool LQ>
+__global__ void __launch_bounds__(NTA, 2)
+adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_constant__ AdjIn a, int tz)
 {
+    using Gm = Geo<ST>;
+    constexpr bool PAIR = Gm::kPair;
+    constexpr int W = Gm::W;
+    extern __shared__ __align__(128) unsigned char smem[];
+    float *const SL = reinterpret_cast<float *>(smem + Gm::L_OFF);
+    ST *const SG = reinterpret_cast<ST *>(smem + Gm::G_OFF);
+    float *const SP = reinterpret_cast<float *>(smem + Gm::PHI_OFF);
+    float *const SF = reinterpret_cast<float *>(smem + Gm::LF_OFF);
+
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TXA + tx;
+    const int half = b.nx / Gm::SEGS;             // x distance of the segments
+    const int ntx = b.nx / TXA, nty = b.ny / TYA;
+    const int bx = blockIdx.x % ntx, by = (blockIdx.x / ntx) % nty, bz = blockIdx.x / (ntx * nty);
+    const int w0 = bx * W, y0 = by * TYA;         // first node of segment 0
+    const int z0 = bz * tz, nzc = min(tz, b.nz - z0);
+    const int seg = PAIR ? tx >> 4 : 0, k = tx & (W - 1);
+    const int x = w0 + seg * half + k, y = y0 + ty;
+    const unsigned nxy = (unsigned)b.nxy;
+
+    // ---- staging roles, fixed per thread ----
+    // lambda_g: row s_r, chunk s_k (of segment s_seg) of every 4th direction from s_q
+    const int s_q = tid >> 6, s_r = (tid >> 3) & 7, s_c = tid & 7;
+    const int s_seg = PAIR ? s_c >> 2 : 0, s_k = PAIR ? s_c & 3 : s_c;
+    const int s_x = w0 + s_seg * half + 4 * s_k;                       // first node of the chunk
+    const int s_xl = wrap_to(w0 + s_seg * half - 4, b.nx), s_xr = wrap_to(w0 + s_seg * half + W, b.nx);
+    const int s_row0 = b.nx * (y0 + s_r), s_rowp = b.nx * wrap_to(y0 + s_r + 1, b.ny),
+              s_rowm = b.nx * wrap_to(y0 + s_r - 1, b.ny);
+    // g: the same for FP32; 16-bit rows are 4 chunks of 8 elements, every 8th direction
+    const int g_q = PAIR ? tid >> 5 : s_q, g_r = PAIR ? (tid >> 2) & 7 : s_r, g_k = PAIR ? tid & 3 : s_k;
+    constexpr int GE = PAIR ? 8 : 4;              // elements per chunk
+    const int g_x = (PAIR ? 2 * w0 : w0) + GE * g_k;
+    const int g_xl = wrap_to((PAIR ? 2 * w0 : w0) - GE, b.nx), g_xr = wrap_to((PAIR ? 2 : 1) * (w0 + W), b.nx);
+    const int g_row0 = b.nx * (y0 + g_r), g_rowp = b.nx * wrap_to(y0 + g_r + 1, b.ny),
+              g_rowm = b.nx * wrap_to(y0 + g_r - 1, b.ny);
+    // phi (threads 0..127) and L (threads 128..255): one chunk of the tile and its halo
+    const int h_t = tid & (NTA / 2 - 1);
+    const bool h_issuer = h_t < Gm::HCHUNKS;
+    int h_xy = 0;
+    {
+        constexpr int RC = Gm::HP / 4;            // chunks per row
+        const int sg = h_t / (Gm::HROWS * RC), rr = (h_t / RC) % Gm::HROWS, kk = h_t % RC;
+        if (h_issuer)
+            h_xy = wrap_to(w0 + sg * half - 4 + 4 * kk, b.nx) + b.nx * wrap_to(y0 - 1 + rr, b.ny);
+    }
+    auto issue_h = [&](int z) {                   // plane z >= z0 - 1 into ring slot (z - z0 + 1) % 3
+        if (!h_issuer) return;
+        const int slot = (int)((unsigned)(z - z0 + 1) % 3u);
+        const unsigned t = (unsigned)wrap_to(z, b.nz) * nxy + (unsigned)h_xy;
+        cp_async16((tid < NTA / 2 ? SP : SF) + slot * Gm::HPLANE + 4 * h_t, (tid < NTA / 2 ? a.phi : a.L) + t);
+    };
+    auto issue = [&](int z, int stage) {          // lambda_g and g rows of plane z
+        const unsigned zc = (unsigned)z * nxy, zp = (unsigned)wrap_to(z + 1, b.nz) * nxy,
+                       zm = (unsigned)wrap_to(z - 1, b.nz) * nxy;
+        float *dl = SL + stage * Gm::LSTAGE + s_seg * Gm::LSEG + s_r * Gm::LP;
+        for_dirs_of<4>(s_q, [&](auto d) {
+            constexpr int i = decltype(d)::value;
+            constexpr int sx = kCx(i), sy = kCy(i), sz = kCz(i);
+            const float *src = a.lg_f[i] + ((sz > 0 ? zp : sz < 0 ? zm : zc) +
+                                            (unsigned)(sy > 0 ? s_rowp : sy < 0 ? s_rowm : s_row0));
+            float *dst = dl + i * TYA * Gm::LP;
+            cp_async16(dst + (sx < 0 ? 4 : 0) + 4 * s_k, src + s_x);
+            if (sx != 0 && s_k == 0) cp_async16(dst + (sx < 0 ? 0 : W), src + (sx < 0 ? s_xl : s_xr));
+        });
+        ST *dg = SG + stage * Gm::GSTAGE + g_r * Gm::GP;
+        for_dirs_of<Gm::GD>(g_q, [&](auto d) {
+            constexpr int i = decltype(d)::value;
+            constexpr int sx = ODD ? -kCx(i) : 0, sy = ODD ? -kCy(i) : 0, sz = ODD ? -kCz(i) : 0;
+            const ST *src = static_cast<const ST *>(a.g_f[ODD ? kOpp(i) : i]) +
+                            ((sz > 0 ? zp : sz < 0 ? zm : zc) +
+                             (unsigned)(sy > 0 ? g_rowp : sy < 0 ? g_rowm : g_row0));
+            ST *dst = dg + i * TYA * Gm::GP;
+            cp_async16(dst + (sx < 0 ? GE : 0) + GE * g_k, src + g_x);
+            if (sx != 0 && g_k == 0)
+                cp_async16(dst + (sx < 0 ? 0 : GE * Gm::GCH), src + (sx < 0 ? g_xl : g_xr));
+        });
+    };
+
+    // where the node finds its values: column of a row staged with x shift sx
+    constexpr auto col = [](int sx) { return sx > 0 ? 1 : sx < 0 ? 3 : 0; };
+    const float *const rl = SL + seg * Gm::LSEG + ty * Gm::LP + k;
+    const ST *const rg = SG + ty * Gm::GP + (PAIR ? 2 * k : k);
+    // 16-bit g: the half of the word; past the x seam (word nx/2 - 1 -> 0 and
+    // back) a word's halves are the other way round
+    const int hf = PAIR ? seg : 0;
+    const int hf_r = PAIR && k == W - 1 && w0 + W == half ? 1 - seg : hf;
+    const int hf_l = PAIR && k == 0 && w0 == 0 ? 1 - seg : hf;
+    const int hc = seg * Gm::HSEG + (ty + 1) * Gm::HP + k + 4;   // the node in a phi / L plane
+    auto hslot = [&](int z) { return (int)((unsigned)(z - z0 + 1) % 3u) * Gm::HPLANE + hc; };
+
+    issue_h(z0 - 1);
+    issue_h(z0);
+    issue_h(z0 + 1);
+    issue(z0, 0);
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();
+    const PlaneSums below = plane_sums<Gm::HP>(SP + hslot(z0 - 1));
+    float a_b = below.a, fx_b = below.fx, fy_b = below.fy;
+    PlaneSums cur = plane_sums<Gm::HP>(SP + hslot(z0));
+    float L_m = SF[hslot(z0 - 1)], L_c = SF[hslot(z0)];
     double dg = 0.0;
-    const int x = blockIdx.x * TXA + threadIdx.x, y = blockIdx.y * TYA + threadIdx.y;
-    if (blockIdx.z < (unsigned)b.nz) prefetch_plane<ST>(b, a, blockIdx.z);
-    for (int z = blockIdx.z; z < b.nz; z += gridDim.z) {
-        if (z + (int)gridDim.z < b.nz) prefetch_plane<ST>(b, a, z + gridDim.z);
-        const Nb p = neighbourhood(b, x, y, z);
-        const unsigned t = p.at(0, 0, 0);
-        float lap, gr[3];
-        stencil19(a.phi, p, lap, gr[0], gr[1], gr[2]);
-        const float ph = __ldg(a.phi + t);
-        float rh = 0.f, m[3] = {0.f, 0.f, 0.f};
-        const Nb ps = state_neighbourhood<ST>(b, x, y, z);
+
+    for (int j = 0; j < nzc; ++j) {
+        const int z = z0 + j, st = j & 1;
+        cp_async_wait_all();
+        __syncthreads();   // plane z has landed; the stages of plane z - 1 are free
+        if (j + 1 < nzc) {
+            issue(z + 1, 1 - st);
+            issue_h(z + 2);
+        }
+        cp_async_commit();
+        const unsigned t = (unsigned)z * nxy + (unsigned)y * (unsigned)b.nx + (unsigned)x;
+
+        const PlaneSums top = plane_sums<Gm::HP>(SP + hslot(z + 1));
+        const float ph = cur.c;
+        const float lap = ((cur.mid + top.a) + a_b) * kInv6;
+        const float gr[3] = {(cur.gx + (top.fx + fx_b)) * kInv12, (cur.gy + (top.fy + fy_b)) * kInv12,
+                             (top.a - a_b) * kInv12};
+        a_b = cur.a;
+        fx_b = cur.fx;
+        fy_b = cur.fy;
+        cur = top;
+
+        // moments of the streamed g (16-bit: of the stored values; the shifts
+        // cancel in the momentum's opposite pairs)
+        float rh, m[3];
+        {
+            const ST *gs = rg + st * Gm::GSTAGE;
+            auto g = [&](int i) -> float {
+                const int sx = ODD ? -kCx(i) : 0;
+                const int cc = PAIR ? 2 * (sx > 0 ? 1 : sx < 0 ? 3 : 0) + (sx > 0 ? hf_r : sx < 0 ? hf_l : hf) : col(sx);
+                return Fmt<ST>::load(gs[i * TYA * Gm::GP + cc]);
+            };
+            rh = g(0);
+            m[0] = m[1] = m[2] = 0.f;
 #pragma unroll
-        for (int i = 0; i < kQg; i++) {
-            const ST v = ODD ? static_cast<const ST *>(a.g_f[kOpp(i)])[dir_at(ps, i, -1)]
-                             : static_cast<const ST *>(a.g_f[i])[ps.at(0, 0, 0)];
-            float gi = Fmt<ST>::load(v);
-            if constexpr (Fmt<ST>::kMapped) gi = gi * q.g_inv + q.g_shift[i];
-            rh += gi;
-            if (kCx(i)) m[0] += kCx(i) * gi;
-            if (kCy(i)) m[1] += kCy(i) * gi;
-            if (kCz(i)) m[2] += kCz(i) * gi;
+            for (int p = 1; p < kQg; p += 2) {    // opposite pairs
+                const float u = g(p), v = g(p + 1), d = u - v;
+                rh += u + v;
+                if (kCx(p)) m[0] += kCx(p) * d;
+                if (kCy(p)) m[1] += kCy(p) * d;
+                if (kCz(p)) m[2] += kCz(p) * d;
+            }
+            if constexpr (Fmt<ST>::kMapped) {
+                float shift = 0.f;
+#pragma unroll
+                for (int i = 0; i < kQg; i++) shift += q.g_shift[i];
+                rh = fmaf(rh, q.g_inv, shift);
+#pragma unroll
+                for (int d = 0; d < 3; d++) m[d] *= q.g_inv;
+            }
         }
         const float inv = 1.0f / rh;
         const float u[3] = {m[0] * inv, m[1] * inv, m[2] * inv};
@@ -429,15 +593,26 @@ __global__ void __launch_bounds__(NTA, adj_min_blocks<ST>()) adjoint_local_kerne
 
         // stream adjoint
         float lP[kQf], lQ[kQg];
-        const float lst_here = __ldg(a.lst + t);
-        lP[0] = __ldg(a.lf_f[0] + t) + lst_here;
+        {
+            const float *Lp = SF + hslot(z);
+            const float L_p = SF[hslot(z + 1)];
+            const float up[kQf] = {L_c, Lp[1], Lp[-1], Lp[Gm::HP], Lp[-Gm::HP], L_p, L_m};
+            lP[0] = L_c;
 #pragma unroll
-        for (int i = 1; i < kQf; i++) {
-            const unsigned dn = dir_at(p, i, 1);
-            lP[i] = c.eta * (__ldg(a.lf_f[i] + dn) + __ldg(a.lst + dn)) + c.eta2 * (__ldg(a.lf_f[i] + t) + lst_here);
+            for (int i = 1; i < kQf; i++) lP[i] = c.eta * up[i] + c.eta2 * L_c;
+            if constexpr (LQ) {   // lf_i = q_i + L
+                const Nb p = neighbourhood(b, x, y, z);
+                lP[0] += __ldg(a.lq_f[0] + t);
+#pragma unroll
+                for (int i = 1; i < kQf; i++)
+                    lP[i] += c.eta * __ldg(a.lq_f[i] + dir_at(p, i, 1)) + c.eta2 * __ldg(a.lq_f[i] + t);
+            }
+            L_m = L_c;
+            L_c = L_p;
+            const float *ls = rl + st * Gm::LSTAGE;
+#pragma unroll
+            for (int i = 0; i < kQg; i++) lQ[i] = ls[i * TYA * Gm::LP + col(kCx(i))];
         }
-#pragma unroll
-        for (int i = 0; i < kQg; i++) lQ[i] = __ldg(a.lg_f[i] + dir_at(p, i, 1));
 
         // D3Q7 collision
         float lphi = 0.f, lmu = 0.f, lus[3] = {0.f, 0.f, 0.f}, lF[3] = {0.f, 0.f, 0.f}, lrho = 0.f;
@@ -526,8 +701,11 @@ __global__ void __launch_bounds__(NTA, adj_min_blocks<ST>()) adjoint_local_kerne
             lrho += drho;
             lm[2] += dmz;
         }
+        a.lphi[t] = lphi;
+        if constexpr (LQ) {
 #pragma unroll
-        for (int i = 0; i < kQf; i++) a.lf_o[i][t] = c.invTauPhiOne * lP[i] + lphi;
+            for (int i = 0; i < kQf; i++) a.lq_o[i][t] = c.invTauPhiOne * lP[i];
+        }
 #pragma unroll
         for (int i = 0; i < kQg; i++) {
             float o = c.invTauRhoOne * lQ[i] + lrho;
@@ -537,16 +715,14 @@ __global__ void __launch_bounds__(NTA, adj_min_blocks<ST>()) adjoint_local_kerne
             a.lg_o[i][t] = o;
         }
     }
-    // per-warp sums into the warp's own slot: no block barrier, so warps that
-    // finish early leave at once (with a block reduction here they waited for
-    // the block's slowest warp: 1.5 barrier stalls per issued instruction at
-    // 160^3 with an FP16 state), and the FP64 sums stay in a fixed order
+    // per-warp sums into the warp's own slot, in a fixed order
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dg += __shfl_down_sync(0xffffffffu, dg, o);
-    if (threadIdx.x == 0) a.dgrav[block_id() * (NTA / 32) + threadIdx.y] += dg;
+    if (tx == 0) a.dgrav[blockIdx.x * (NTA / 32) + ty] += dg;
 }
 
-// lst = L[lambda_lap] - sum_k D_k[lambda_grad_k]: the transposed stencils.
+// L = lambda_phi + Lap[lambda_lap] - sum_k D_k[lambda_grad_k]: the transposed
+// stencils, added to lambda_phi in place.
 // Laplacian weights: 2/6 on faces, 1/6 on edges, -4 at the centre; gradient
 // component k: c_ik times 2/12 on faces, 1/12 on edges.
 //
@@ -561,7 +737,7 @@ __global__ void __launch_bounds__(NTA, adj_min_blocks<ST>()) adjoint_local_kerne
 constexpr int SW = TXA + 2, SH = TYA + 2, SPLANE = SW * SH;
 
 __global__ void __launch_bounds__(NTA) adjoint_stencil_kernel(Box b, const float4 *__restrict__ lsrc,
-                                                              float *__restrict__ lst)
+                                                              float *__restrict__ lphi)
 {
     __shared__ float sm[3][4][SPLANE];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TXA + tx;
@@ -631,7 +807,7 @@ __global__ void __launch_bounds__(NTA) adjoint_stencil_kernel(Box b, const float
         const float c0 = sm[z % 3][0][cell];
         const float L = (ledge + 2.f * (lface - 12.f * c0)) * kInv6;
         const float D = (2.f * dface + dedge) * kInv12;
-        lst[(unsigned)z * (unsigned)b.nxy + (unsigned)(y0 + ty) * nx + (unsigned)(x0 + tx)] = L - D;
+        lphi[(unsigned)z * (unsigned)b.nxy + (unsigned)(y0 + ty) * nx + (unsigned)(x0 + tx)] += L - D;
         __syncthreads();          // plane z - 1's slot is free (z + 2 takes it)
         if (next) put(z + 2);
         __syncthreads();
@@ -653,8 +829,8 @@ __global__ void __launch_bounds__(NTA) dgrav_fold_kernel(const double *__restric
 // src/init_g.cu:69-91), local part; llap receives lambda of the Laplacian.
 __global__ void __launch_bounds__(NTA) init_adjoint_kernel(Box b, float alpha4, float kappa, float phiStarSq,
                                                            float Gamma, const float *__restrict__ phi0,
-                                                           const float *__restrict__ lf,
-                                                           const float *__restrict__ lst,
+                                                           const float *__restrict__ lq,
+                                                           const float *__restrict__ L,
                                                            const float *__restrict__ lg, float *__restrict__ lphi0,
                                                            float *__restrict__ llap)
 {
@@ -667,10 +843,11 @@ __global__ void __launch_bounds__(NTA) init_adjoint_kernel(Box b, float alpha4, 
         stencil19(phi0, p, lap, gx, gy, gz);
         const float ph = phi0[t];
         const float mu = alpha4 * ph * (ph * ph - phiStarSq) - kappa * lap;
-        const float add = lst[t];
-        const float l0 = lf[t] + add;
-        float lfs = 0.f, lga = 0.f, lgd = 0.f;
-        for (int i = 1; i < kQf; i++) lfs += lf[i * n + t] + add;
+        const float add = L[t];   // lf_i = q_i + L
+        const float l0 = lq ? lq[t] + add : add;
+        float lfs = 6.f * add, lga = 0.f, lgd = 0.f;
+        if (lq)
+            for (int i = 1; i < kQf; i++) lfs += lq[i * n + t];
         for (int i = 1; i < 7; i++) lga += lg[i * n + t];
         for (int i = 7; i < kQg; i++) lgd += lg[i * n + t];
         const float lg0 = lg[t];
@@ -700,10 +877,24 @@ dim3 adjoint_grid(const Box &b)
     return dim3((unsigned)(b.nx / TXA), (unsigned)(b.ny / TYA), (unsigned)((b.nz + kPlanes - 1) / kPlanes));
 }
 
-// the local kernel's grid (its blocks take planes gridDim.z apart)
-dim3 local_grid(const Box &b)
+// The march kernel's planes per block and its blocks.  Constants of the cost
+// (march_depth): a block's prologue is about one plane, two blocks on an SM
+// take 1.4 times as long as one.
+struct March {
+    int tz, blocks;
+};
+March march_of(const Box &b)
 {
-    return dim3((unsigned)(b.nx / TXA), (unsigned)(b.ny / TYA), (unsigned)((b.nz + kLocalPlanes - 1) / kLocalPlanes));
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return std::max(1, n);
+    }();
+    constexpr double share[3] = {0.0, 1.0, 1.4};
+    const int tiles = (b.nx / TXA) * (b.ny / TYA);
+    const int tz = march_depth(tiles, b.nz, sms, 2, 1.0, 0.88, share);
+    return March{tz, tiles * ((b.nz + tz - 1) / tz)};
 }
 
 size_t blocks_of(const dim3 &g) { return (size_t)g.x * g.y * g.z; }
@@ -741,12 +932,9 @@ FQFields fq_fields(const Box &b, const NativeState &st)
     return r;
 }
 
-size_t adjoint_dgrav_parts(const Box &b) { return blocks_of(local_grid(b)) * (NTA / 32); }
+size_t adjoint_dgrav_parts(const Box &b) { return (size_t)march_of(b).blocks * (NTA / 32); }
 
-size_t adjoint_blocks(const Box &b)
-{
-    return std::max(blocks_of(adjoint_grid(b)), blocks_of(local_grid(b)));
-}
+size_t adjoint_blocks(const Box &b) { return blocks_of(adjoint_grid(b)); }
 
 cudaError_t launch_adjoint_phi(const Box &b, float eta, const Quant &q, const NativeState &st, float *phi,
                                cudaStream_t s)
@@ -777,13 +965,13 @@ cudaError_t launch_objective(const Box &b, int objective, float phiStar, double 
 }
 
 cudaError_t launch_source_init(const Box &b, int objective, double scale, const double *ab, float phiStar,
-                               const Quant &q, const NativeState &st, const float *phi, float *lf, float *lg,
-                               float *lst, cudaStream_t s)
+                               const Quant &q, const NativeState &st, const float *phi, float *lq, float *lg,
+                               float *L, cudaStream_t s)
 {
     return dispatch(st, [&](auto tag, auto odd) {
         using ST = decltype(tag);
         source_init_kernel<ST, decltype(odd)::value><<<adjoint_grid(b), kBlock, 0, s>>>(
-            b, objective, scale, ab, phiStar, q, g_fields(b, st), phi, lf, lg, lst);
+            b, objective, scale, ab, phiStar, q, g_fields(b, st), phi, lq, lg, L);
         return cudaGetLastError();
     });
 }
@@ -793,22 +981,19 @@ cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar,
                                 double scale, cudaStream_t s)
 {
     AdjIn in;
-    in.g = st.g;
+    std::memset(&in, 0, sizeof(in));
     in.phi = a.phi;
-    in.lf = a.lf_in;
-    in.lg = a.lg_in;
-    in.lst = a.lst_in;
-    in.lf_out = a.lf_out;
-    in.lg_out = a.lg_out;
+    in.L = a.L_in;
+    in.lphi = a.L_out;
     const size_t n = (size_t)b.n, esz = storage_bytes(st.storage);
     for (int i = 0; i < kQg; i++) {
         in.g_f[i] = static_cast<const unsigned char *>(st.g) + (size_t)i * n * esz;
         in.lg_f[i] = a.lg_in + (size_t)i * n;
         in.lg_o[i] = a.lg_out + (size_t)i * n;
     }
-    for (int i = 0; i < kQf; i++) {
-        in.lf_f[i] = a.lf_in + (size_t)i * n;
-        in.lf_o[i] = a.lf_out + (size_t)i * n;
+    for (int i = 0; i < kQf && a.lq_in; i++) {
+        in.lq_f[i] = a.lq_in + (size_t)i * n;
+        in.lq_o[i] = a.lq_out + (size_t)i * n;
     }
     in.lsrc = a.lsrc;
     in.dgrav = a.dgrav;
@@ -816,13 +1001,21 @@ cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar,
     in.scale = scale;
     in.objective = objective;
     in.add_source = add_source ? 1 : 0;
+    const March march = march_of(b);
     cudaError_t e = dispatch(st, [&](auto tag, auto odd) {
-        adjoint_local_kernel<decltype(tag), decltype(odd)::value>
-            <<<local_grid(b), kBlock, 0, s>>>(b, c, phiStar, q, in);
-        return cudaGetLastError();
+        using ST = decltype(tag);
+        auto go = [&](auto kernel) {
+            // per launch: the attribute belongs to the device's function, and this is not a hot path of the host
+            cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<ST>::SMEM);
+            if (ea != cudaSuccess) return ea;
+            kernel<<<(unsigned)march.blocks, kBlock, Geo<ST>::SMEM, s>>>(b, c, phiStar, q, in, march.tz);
+            return cudaGetLastError();
+        };
+        return a.lq_in ? go(adjoint_march_kernel<ST, decltype(odd)::value, true>)
+                       : go(adjoint_march_kernel<ST, decltype(odd)::value, false>);
     });
     if (e != cudaSuccess) return e;
-    adjoint_stencil_kernel<<<adjoint_grid(b), kBlock, 0, s>>>(b, a.lsrc, a.lst_out);
+    adjoint_stencil_kernel<<<adjoint_grid(b), kBlock, 0, s>>>(b, a.lsrc, a.L_out);
     return cudaGetLastError();
 }
 
@@ -832,10 +1025,10 @@ cudaError_t launch_dgrav_fold(const Box &b, const double *dgrav, double *acc, cu
     return cudaGetLastError();
 }
 
-cudaError_t launch_init_adjoint(const Box &b, const lbm_derived &d, float Gamma, const float *phi0, const float *lf,
-                                const float *lst, const float *lg, float *lphi0, float *llap, cudaStream_t s)
+cudaError_t launch_init_adjoint(const Box &b, const lbm_derived &d, float Gamma, const float *phi0, const float *lq,
+                                const float *L, const float *lg, float *lphi0, float *llap, cudaStream_t s)
 {
-    init_adjoint_kernel<<<adjoint_grid(b), kBlock, 0, s>>>(b, d.alpha4, d.kappa, d.phiStarSq, Gamma, phi0, lf, lst,
+    init_adjoint_kernel<<<adjoint_grid(b), kBlock, 0, s>>>(b, d.alpha4, d.kappa, d.phiStarSq, Gamma, phi0, lq, L,
                                                            lg, lphi0, llap);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

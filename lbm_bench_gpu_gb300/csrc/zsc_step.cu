@@ -1265,12 +1265,7 @@ bool encode_f_maps(const Box &b, const float *f0, const ST *fq, CUtensorMap *f0m
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Planes per block.  A block's time is about (tz + kPrologue) plane-times (the
-// prologue stages and rebuilds the planes around its first one), and r blocks
-// that share an SM slow each other down by share[r], less than r: a lone block
-// is bound by its own latencies.  The launch takes as many full rounds of
-// resident blocks as there are, then a last, partly filled one, which overlaps
-// the end of the others (kTail).  The depth that minimises the sum is taken.
+// Planes per block (march_depth).
 // The four constants were fitted to forced depths 1 .. 64 on nine boxes from
 // 32^3 to 256^3 in FP32 and FP16: the choice is within 1.1% of the best depth
 // on average, 6.4% at most.  (Measured, depth before -> now: 32^3 FP32 4 -> 1
@@ -1301,22 +1296,8 @@ int choose_tz(const Box &b)
     static thread_local int last[4] = {0, 0, 0, 0};
     if (last[0] == b.nx && last[1] == b.ny && last[2] == b.nz) return last[3];
     const auto [sms, per_sm] = resident_slots<ST>();
-    constexpr double kPrologue = 1.25, kTail = 0.88;
     constexpr double share[5] = {0.0, 1.0, sizeof(ST) == 2 ? 1.43 : 1.40, 1.90, 2.28};
-    const long long tiles = (long long)(b.nx / TX) * (b.ny / TY), slots = (long long)sms * per_sm;
-    int best = 1;
-    double best_cost = -1.0;
-    for (int tz = 1; tz <= 64; tz++) {
-        const long long blocks = tiles * ((b.nz + tz - 1) / tz);
-        const long long full = blocks / slots, rest = blocks % slots;
-        double rounds = (double)full * share[per_sm];
-        if (rest > 0) rounds += (full > 0 ? kTail : 1.0) * share[(rest + sms - 1) / sms];
-        const double cost = rounds * (tz + kPrologue);
-        if (best_cost < 0.0 || cost < best_cost) {
-            best_cost = cost;
-            best = tz;
-        }
-    }
+    const int best = march_depth((long long)(b.nx / TX) * (b.ny / TY), b.nz, sms, per_sm, 1.25, 0.88, share);
     last[0] = b.nx;
     last[1] = b.ny;
     last[2] = b.nz;
