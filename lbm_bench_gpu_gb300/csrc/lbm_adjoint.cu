@@ -116,7 +116,7 @@ struct Adjoint {
     float *phi = nullptr;     // 2 x n
     // lambda: L, the 19 lg and, when tauPhi is not 1, the seven q (AdjointBuffers)
     float *lam_L[2] = {nullptr, nullptr}, *lam_g[2] = {nullptr, nullptr}, *lam_q[2] = {nullptr, nullptr};
-    float4 *lsrc = nullptr;
+    float *lsrc = nullptr;        // 4 x n
     float *phi0 = nullptr, *mom_save = nullptr;
     double *partials = nullptr, *dgrav = nullptr, *ab = nullptr, *acc = nullptr;
     unsigned char *slots = nullptr;   // the context's checkpoint pool
@@ -554,7 +554,7 @@ struct Adjoint {
             lam_L[i] = w.take<float>(n);
             if (k.invTauPhiOne != 0.f) lam_q[i] = w.take<float>((size_t)lbm::kQf * n);
         }
-        lsrc = w.take<float4>(n);
+        lsrc = w.take<float>(4 * n);
         phi0 = w.take<float>(n);
         dgrav = w.take<double>(lbm::adjoint_dgrav_parts(c->box));
     }
@@ -736,7 +736,7 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
     if (!rc) rc = hslots >= 1 ? A.two_level(hslots, nslots) : A.revolve(0, o->nsteps, 0, (int)(nslots - 1));
     // lambda^0 -> dJ/dphi0 through the initial equilibrium (output in the
     // lsrc buffer, phi as the scratch for the Laplacian's adjoint)
-    float *lphi0 = reinterpret_cast<float *>(A.lsrc);
+    float *lphi0 = A.lsrc;
     if (!rc) {
         e = lbm::launch_dgrav_fold(c->box, A.dgrav, A.acc, c->stream);
         if (e == cudaSuccess)

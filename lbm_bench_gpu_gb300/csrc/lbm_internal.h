@@ -106,7 +106,7 @@ struct AdjointBuffers {
     const float *phi;                  // phi of s^n
     const float *lq_in, *lg_in, *L_in; // lambda^{n+1}
     float *lq_out, *lg_out, *L_out;    // lambda^n
-    float4 *lsrc;                      // scratch per node: (lambda_lap, mu lambda_F)
+    float *lsrc;                       // scratch: lambda_lap and mu lambda_F, four fields
     double *dgrav;                     // per-warp running sums of the dJ/dgrav terms
     const double *ab;                  // objective sums of s^n
 };

@@ -27,8 +27,8 @@
 // neighbours).  Per step (bytes per node, FP32 / 16-bit state, tauPhi = 1):
 //   adjoint_phi_kernel     s^n -> phi                                 32 / 20
 //   adjoint_march_kernel   lambda^{n+1}, s^n, phi -> lg^n, lambda_phi
-//                          and (lambda_lap, mu lambda_F) as a float4  256 / 218
-//   adjoint_stencil_kernel float4, lambda_phi -> L^n                  24
+//                          and (lambda_lap, mu lambda_F)              256 / 218
+//   adjoint_stencil_kernel these four, lambda_phi -> L^n              24
 // All per-node arithmetic is FP32; the objective sums and dJ/dgrav are FP64.
 // The kernels work on 32 x 8 column tiles, each block marching z planes.
 // 32-bit node indices (n * 19 < 2^32 is checked at init).
@@ -46,6 +46,7 @@ constexpr int TXA = 32, TYA = 8, NTA = TXA * TYA;
 #define ZSC_ADJ_PLANES 4
 #endif
 constexpr int kPlanes = ZSC_ADJ_PLANES;
+constexpr int kStencilBlocks = 5;   // resident blocks of the stencil kernel per SM
 constexpr float kInv6 = 0.16666666666666666667f;
 constexpr float kInv12 = 0.08333333333333333333f;
 constexpr float kW0 = 0.33333333333333333333f, kW1 = 0.05555555555555555556f, kW2 = 0.02777777777777777778f;
@@ -341,7 +342,7 @@ struct AdjIn {
     const float *phi;                      // phi of s^n
     const float *L;                        // L^{n+1}
     float *lphi;                           // lambda_phi^n (L^n without its stencil part)
-    float4 *lsrc;                          // (lambda_lap, mu lambda_F) at every node
+    float *lsrc[4];                        // lambda_lap, mu lambda_F at every node
     double *dgrav;                         // per warp of each block, accumulated over steps
     const double *ab;                      // objective sums of s^n (when add_source)
     double scale;
@@ -358,6 +359,11 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_prior()   // all but this thread's last N groups
+{
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
 template <int I>
 struct Dir {
@@ -693,7 +699,9 @@ adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_co
         for (int k = 0; k < 3; k++) lmu += gr[k] * lF[k];
         if (heavy) dg += lF[2];
         lphi += c.alpha4 * (3.f * ph * ph - c.phiStarSq) * lmu;
-        a.lsrc[t] = make_float4(-c.kappa * lmu, mu * lF[0], mu * lF[1], mu * lF[2]);
+        a.lsrc[0][t] = -c.kappa * lmu;
+#pragma unroll
+        for (int k = 0; k < 3; k++) a.lsrc[1 + k][t] = mu * lF[k];
         if (a.add_source) {
             float dphi, drho, dmz;
             objective_source(z, a.objective, source_coef(a.ab, phiStar), phiStar, ph, rh, m[2], dphi, drho, dmz);
@@ -722,95 +730,99 @@ adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_co
 }
 
 // L = lambda_phi + Lap[lambda_lap] - sum_k D_k[lambda_grad_k]: the transposed
-// stencils, added to lambda_phi in place.
-// Laplacian weights: 2/6 on faces, 1/6 on edges, -4 at the centre; gradient
-// component k: c_ik times 2/12 on faces, 1/12 on edges.
+// stencils, added to lambda_phi in place.  Laplacian weights: 2/6 on faces, 1/6
+// on edges, -4 at the centre; gradient component k: c_ik times 2/12 on faces,
+// 1/12 on edges.
 //
-// The block marches its kPlanes planes with a ring of three planes of the
-// float4 source in shared memory, each on the tile plus a one-node ring
-// (34 x 10), split into its four components so that a node reads the 49
-// scalars it needs (lambda_lap at 19 points, each gradient component at the
-// 10 points with c_k != 0) without bank conflicts.  Plane z + 2 is read into
-// registers before plane z is computed (its loads overlap the computation) and
-// stored into the slot plane z - 1 frees; each thread's staging coordinates
-// are computed once.
-constexpr int SW = TXA + 2, SH = TYA + 2, SPLANE = SW * SH;
+// A block marches tz planes of a 32 x 8 tile.  The four source fields of a
+// plane (the tile plus one node) are staged one plane ahead with 16-byte
+// cp.async copies.  Regrouped by plane, a node takes three numbers from each:
+// what it adds to the node in it, to the node above and to the node below,
+// which two registers carry down the march; a plane is read at 26 scalars per
+// node, not 49 in three planes.  Bound by DRAM at 24 bytes a node (59 us at
+// 256^3 at the copy bandwidth).
+struct StencilGeo {
+    static constexpr int P = TXA + 8, ROWS = TYA + 2;      // staged row and rows (floats)
+    static constexpr int FIELD = P * ROWS, PLANE = 4 * FIELD;
+    static constexpr int CHUNKS = PLANE / 4;               // 16-byte chunks of a plane
+    static constexpr int PER = (CHUNKS + NTA - 1) / NTA;   // per thread
+};
 
-__global__ void __launch_bounds__(NTA) adjoint_stencil_kernel(Box b, const float4 *__restrict__ lsrc,
-                                                              float *__restrict__ lphi)
+__global__ void __launch_bounds__(NTA, kStencilBlocks)
+adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict__ lphi, int tz)
 {
-    __shared__ float sm[3][4][SPLANE];
+    using G = StencilGeo;
+    __shared__ __align__(16) float sm[2][G::PLANE];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TXA + tx;
-    const int x0 = blockIdx.x * TXA, y0 = blockIdx.y * TYA;
-    const int z_begin = blockIdx.z * kPlanes, z_end = min(b.nz, z_begin + kPlanes);
-    const unsigned nx = (unsigned)b.nx;
-    // the (up to two) ring-tile nodes this thread stages, as in-plane offsets
-    // (periodic in x and y), fixed for the block
-    auto xy_of = [&](int e) {
-        const int r = e / SW, c = e - r * SW;
-        int gx = x0 - 1 + c, gy = y0 - 1 + r;
-        gx = gx < 0 ? gx + b.nx : (gx >= b.nx ? gx - b.nx : gx);
-        gy = gy < 0 ? gy + b.ny : (gy >= b.ny ? gy - b.ny : gy);
-        return (unsigned)gy * nx + (unsigned)gx;
-    };
-    const int e0 = tid, e1 = tid + NTA;
-    const bool two = e1 < SPLANE;
-    const unsigned xy0 = xy_of(e0), xy1 = two ? xy_of(e1) : 0u;
-    float4 v0, v1;
-    auto fetch = [&](int z) {   // plane z into registers (its loads stay in flight)
-        const int zw = z < 0 ? z + b.nz : (z >= b.nz ? z - b.nz : z);
-        const unsigned zo = (unsigned)zw * (unsigned)b.nxy;
-        v0 = __ldg(lsrc + zo + xy0);
-        if (two) v1 = __ldg(lsrc + zo + xy1);
-    };
-    auto put = [&](int z) {     // ... and into its ring slot, components apart
-        const int slot = (z + 3) % 3;
-        sm[slot][0][e0] = v0.x;
-        sm[slot][1][e0] = v0.y;
-        sm[slot][2][e0] = v0.z;
-        sm[slot][3][e0] = v0.w;
-        if (two) {
-            sm[slot][0][e1] = v1.x;
-            sm[slot][1][e1] = v1.y;
-            sm[slot][2][e1] = v1.z;
-            sm[slot][3][e1] = v1.w;
-        }
-    };
-    for (int z = z_begin - 1; z <= min(z_begin + 1, z_end); z++) {
-        fetch(z);
-        put(z);
-    }
-    __syncthreads();
-    const int cell = (ty + 1) * SW + tx + 1;
-    for (int z = z_begin; z < z_end; z++) {
-        // plane z + 2 is read from memory while plane z is computed
-        const bool next = z + 2 <= z_end;
-        if (next) fetch(z + 2);
-        float lface = 0.f, ledge = 0.f, dface = 0.f, dedge = 0.f;
+    const int ntx = b.nx / TXA, nty = b.ny / TYA;
+    const int bx = blockIdx.x % ntx, by = (blockIdx.x / ntx) % nty, bz = blockIdx.x / (ntx * nty);
+    const int x0 = bx * TXA, y0 = by * TYA, z0 = bz * tz, nzc = min(tz, b.nz - z0);
+    const unsigned nxy = (unsigned)b.nxy;
+    const unsigned n = (unsigned)b.n;
+    // the chunks this thread stages: in-plane offset (periodic) and field
+    unsigned off[G::PER];
 #pragma unroll
-        for (int i = 1; i < kQg; i++) {
-            const int slot = (z + kCz(i) + 3) % 3;
-            const int at = cell + kCy(i) * SW + kCx(i);
-            const float lx = sm[slot][0][at];
-            float d = 0.f;
-            if (kCx(i)) d += kCx(i) * sm[slot][1][at];
-            if (kCy(i)) d += kCy(i) * sm[slot][2][at];
-            if (kCz(i)) d += kCz(i) * sm[slot][3][at];
-            if (i < 7) {
-                lface += lx;
-                dface += d;
-            } else {
-                ledge += lx;
-                dedge += d;
-            }
+    for (int q = 0; q < G::PER; q++) {
+        const int e = tid + q * NTA, f = e / (G::FIELD / 4), r = e % (G::FIELD / 4);
+        const int row = r / (G::P / 4), kk = r % (G::P / 4);
+        off[q] = (unsigned)f * n + (unsigned)(b.nx * wrap_to(y0 - 1 + row, b.ny) + wrap_to(x0 - 4 + 4 * kk, b.nx));
+    }
+    auto issue = [&](int z, int stage) {
+        const unsigned zo = (unsigned)wrap_to(z, b.nz) * nxy;
+#pragma unroll
+        for (int q = 0; q < G::PER; q++) {
+            const int e = tid + q * NTA;
+            if (e < G::CHUNKS) cp_async16(&sm[stage][4 * e], lsrc + zo + off[q]);
         }
-        const float c0 = sm[z % 3][0][cell];
-        const float L = (ledge + 2.f * (lface - 12.f * c0)) * kInv6;
-        const float D = (2.f * dface + dedge) * kInv12;
-        lphi[(unsigned)z * (unsigned)b.nxy + (unsigned)(y0 + ty) * nx + (unsigned)(x0 + tx)] += L - D;
-        __syncthreads();          // plane z - 1's slot is free (z + 2 takes it)
-        if (next) put(z + 2);
-        __syncthreads();
+    };
+    // contributions of plane values at this node: to its own plane, to the
+    // plane below it (it is the plane above that one) and to the plane above
+    const int cell = (ty + 1) * G::P + tx + 4;
+    struct Part {
+        float own, below, above;
+    };
+    auto part = [&](int stage) -> Part {
+        const float *l = sm[stage] + cell, *gx = l + G::FIELD, *gy = gx + G::FIELD, *gz = gy + G::FIELD;
+        constexpr int N = G::P;
+        const float lc = l[0], lf = (l[1] + l[-1]) + (l[N] + l[-N]);
+        const float le = (l[N + 1] + l[-N - 1]) + (l[-N + 1] + l[N - 1]);
+        const float sx = gx[1] - gx[-1], sy = gy[N] - gy[-N];
+        const float dx = (gx[N + 1] - gx[-N - 1]) + (gx[-N + 1] - gx[N - 1]);
+        const float dy = (gy[N + 1] - gy[-N - 1]) - (gy[-N + 1] - gy[N - 1]);
+        const float sz = ((gz[1] + gz[-1]) + (gz[N] + gz[-N])) + 2.f * gz[0];
+        Part p;
+        p.own = (le + 2.f * (lf - 12.f * lc)) * kInv6 - (2.f * (sx + sy) + (dx + dy)) * kInv12;
+        const float side = (lf + 2.f * lc) * kInv6 - (sx + sy) * kInv12;
+        p.below = side - sz * kInv12;   // c_z = +1 of the node below
+        p.above = side + sz * kInv12;
+        return p;
+    };
+    // plane p is staged in stage (p - z0 + 1) & 1
+    issue(z0 - 1, 0);
+    cp_async_commit();
+    issue(z0, 1);
+    cp_async_commit();
+    cp_async_wait_prior<1>();
+    __syncthreads();
+    float from_below = part(0).above;   // what plane z0 - 1 adds to plane z0
+    __syncthreads();
+    issue(z0 + 1, 0);
+    cp_async_commit();
+    cp_async_wait_prior<1>();
+    __syncthreads();
+    Part cur = part(1);
+    unsigned t = (unsigned)z0 * nxy + (unsigned)((y0 + ty) * b.nx + x0 + tx);
+    for (int j = 0; j < nzc; ++j, t += nxy) {
+        const float base = lphi[t];
+        __syncthreads();   // plane z is read: its stage takes plane z + 2
+        if (j + 1 < nzc) issue(z0 + j + 2, (j + 3) & 1);
+        cp_async_commit();
+        cp_async_wait_prior<1>();
+        __syncthreads();   // plane z + 1 has landed
+        const Part top = part((j + 2) & 1);
+        lphi[t] = base + ((cur.own + top.below) + from_below);
+        from_below = cur.above;
+        cur = top;
     }
 }
 
@@ -883,7 +895,7 @@ dim3 adjoint_grid(const Box &b)
 struct March {
     int tz, blocks;
 };
-March march_of(const Box &b)
+int sm_count()
 {
     static const int sms = [] {
         int dev = 0, n = 0;
@@ -891,9 +903,21 @@ March march_of(const Box &b)
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         return std::max(1, n);
     }();
+    return sms;
+}
+March march_of(const Box &b)
+{
     constexpr double share[3] = {0.0, 1.0, 1.4};
     const int tiles = (b.nx / TXA) * (b.ny / TYA);
-    const int tz = march_depth(tiles, b.nz, sms, 2, 1.0, 0.88, share);
+    const int tz = march_depth(tiles, b.nz, sm_count(), 2, 1.0, 0.88, share);
+    return March{tz, tiles * ((b.nz + tz - 1) / tz)};
+}
+// The stencil kernel's: a prologue of two planes, kStencilBlocks blocks on an SM.
+March stencil_march(const Box &b)
+{
+    constexpr double share[kStencilBlocks + 1] = {0.0, 1.0, 1.2, 1.5, 1.8, 2.2};
+    const int tiles = (b.nx / TXA) * (b.ny / TYA);
+    const int tz = march_depth(tiles, b.nz, sm_count(), kStencilBlocks, 2.0, 0.88, share);
     return March{tz, tiles * ((b.nz + tz - 1) / tz)};
 }
 
@@ -995,7 +1019,7 @@ cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar,
         in.lq_f[i] = a.lq_in + (size_t)i * n;
         in.lq_o[i] = a.lq_out + (size_t)i * n;
     }
-    in.lsrc = a.lsrc;
+    for (int k = 0; k < 4; k++) in.lsrc[k] = a.lsrc + (size_t)k * n;
     in.dgrav = a.dgrav;
     in.ab = a.ab;
     in.scale = scale;
@@ -1015,7 +1039,8 @@ cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar,
                        : go(adjoint_march_kernel<ST, decltype(odd)::value, false>);
     });
     if (e != cudaSuccess) return e;
-    adjoint_stencil_kernel<<<adjoint_grid(b), kBlock, 0, s>>>(b, a.lsrc, a.L_out);
+    const March sten = stencil_march(b);
+    adjoint_stencil_kernel<<<(unsigned)sten.blocks, kBlock, 0, s>>>(b, a.lsrc, a.L_out, sten.tz);
     return cudaGetLastError();
 }
 
