@@ -140,72 +140,67 @@ int reduce_stats(lbm_ctx *c)
     return LBM_OK;
 }
 
+// The shifts of the 16-bit storage map: w_i times the mean density.
+void g_shifts(double rho_mean, float (&shift)[lbm::kQg])
+{
+    for (int i = 0; i < lbm::kQg; i++) shift[i] = (float)(kW[i] * rho_mean);
+}
+
+// The 16-bit storage map from the 26 maxima |f_k|, |g_i - shift_i|.
+// Scales: powers of two that put a generous bound on each field at
+// 2^12, leaving 16x headroom below the FP16 maximum (65504).  The bound
+// covers the flow developing later: |u| up to 0.1 moves g_i by about
+// 3 w_i rho |u| and f_i by about phiStar |u| / (tauPhi (1 - eta)).
+// BF16 has the FP32 exponent range and keeps scale 1.
+// One scale per set, the smallest of its fields' (scaling by a power
+// of two changes no rounding of normal FP16 numbers).
+void choose_map(lbm_ctx *c, const float *maxabs, double rho_mean, const float *shift)
+{
+    const bool fp16 = c->p.storage == LBM_STORAGE_FP16;
+    auto pick = [&](float m_abs, double bound) -> float {
+        double m = std::max((double)m_abs, bound);
+        if (!fp16 || !(m > 0.0) || !std::isfinite(m)) return 1.f;
+        int ex = (int)std::floor(std::log2(4096.0 / m));
+        ex = std::max(-60, std::min(60, ex));
+        return std::ldexp(1.f, ex);
+    };
+    const double fbound = 0.1 * std::fabs((double)c->d.phiStar) * c->d.invTauPhi * c->d.invEta2;
+    float fs = INFINITY, gs = INFINITY;
+    for (int a = 0; a < lbm::kQf - 1; a++) fs = std::min(fs, pick(maxabs[a + 1], fbound));
+    for (int i = 0; i < lbm::kQg; i++) {
+        c->q.g_shift[i] = shift[i];
+        gs = std::min(gs, pick(maxabs[lbm::kQf + i], 0.3 * kW[i] * std::fabs(rho_mean)));
+    }
+    c->q.f_scale = fs;
+    c->q.f_inv = 1.f / fs;
+    c->q.g_scale = gs;
+    c->q.g_inv = 1.f / gs;
+}
+
 // Load streamed FP32 distributions tf (7 x n) and tg (19 x n) into the state
 // (half 0, natural g layout), choosing the 16-bit storage map from the data.
-// c->st.mom must already hold the fields (for the mean density).  maxabs_in
-// (26 floats: |f_k| and |g_i - shift_i| maxima) replaces the maxima of this
-// context's data (a z-slab takes the maxima of the whole box, reduced over
-// its slabs); maxabs_out receives this context's maxima (zeros for FP32).
-int load_state(lbm_ctx *c, const float *tf, const float *tg, const float *maxabs_in = nullptr,
-               float *maxabs_out = nullptr)
+// c->st.mom must already hold the fields (for the mean density).
+int load_state(lbm_ctx *c, const float *tf, const float *tg)
 {
-    if (maxabs_out)
-        for (int k = 0; k < lbm::kQf + lbm::kQg; k++) maxabs_out[k] = 0.f;
     identity_quant(c->q);
     if (c->p.storage != LBM_STORAGE_FP32) {
         int rc = reduce_stats(c);
         if (rc) return rc;
         const double rho_mean = c->result_host[8] / (double)c->box.n;
-        float shift[lbm::kQg];
-        for (int i = 0; i < lbm::kQg; i++) shift[i] = (float)(kW[i] * rho_mean);
+        float shift[lbm::kQg], maxabs[lbm::kQf + lbm::kQg];
+        g_shifts(rho_mean, shift);
         float *shift_dev = nullptr;
         unsigned *bits_dev = nullptr;
-        unsigned bits[lbm::kQf + lbm::kQg];
         cudaError_t e = cudaMalloc(&shift_dev, sizeof(shift));
-        if (e == cudaSuccess) e = cudaMalloc(&bits_dev, sizeof(bits));
+        if (e == cudaSuccess) e = cudaMalloc(&bits_dev, sizeof(maxabs));
         if (e == cudaSuccess) e = cudaMemcpyAsync(shift_dev, shift, sizeof(shift), cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) e = lbm::launch_field_maxabs(c->box, tf, tg, shift_dev, bits_dev, c->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(bits, bits_dev, sizeof(bits), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(maxabs, bits_dev, sizeof(maxabs), cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         cudaFree(shift_dev);
         cudaFree(bits_dev);
         if (e != cudaSuccess) return cuda_fail(e, "storage map");
-        for (int k = 0; k < lbm::kQf + lbm::kQg; k++) {
-            if (maxabs_out) std::memcpy(&maxabs_out[k], &bits[k], sizeof(float));
-            if (maxabs_in) std::memcpy(&bits[k], &maxabs_in[k], sizeof(float));
-        }
-        // Scales: powers of two that put a generous bound on each field at
-        // 2^12, leaving 16x headroom below the FP16 maximum (65504).  The bound
-        // covers the flow developing later: |u| up to 0.1 moves g_i by about
-        // 3 w_i rho |u| and f_i by about phiStar |u| / (tauPhi (1 - eta)).
-        // BF16 has the FP32 exponent range and keeps scale 1.
-        // One scale per set, the smallest of its fields' (scaling by a power
-        // of two changes no rounding of normal FP16 numbers).
-        const bool fp16 = c->p.storage == LBM_STORAGE_FP16;
-        auto pick = [&](float maxabs, double bound) -> float {
-            double m = std::max((double)maxabs, bound);
-            if (!fp16 || !(m > 0.0) || !std::isfinite(m)) return 1.f;
-            int ex = (int)std::floor(std::log2(4096.0 / m));
-            ex = std::max(-60, std::min(60, ex));
-            return std::ldexp(1.f, ex);
-        };
-        const double fbound = 0.1 * std::fabs((double)c->d.phiStar) * c->d.invTauPhi * c->d.invEta2;
-        float fs = INFINITY, gs = INFINITY;
-        for (int a = 0; a < lbm::kQf - 1; a++) {
-            float m;
-            std::memcpy(&m, &bits[a + 1], sizeof(float));
-            fs = std::min(fs, pick(m, fbound));
-        }
-        for (int i = 0; i < lbm::kQg; i++) {
-            float m;
-            std::memcpy(&m, &bits[lbm::kQf + i], sizeof(float));
-            c->q.g_shift[i] = shift[i];
-            gs = std::min(gs, pick(m, 0.3 * kW[i] * std::fabs(rho_mean)));
-        }
-        c->q.f_scale = fs;
-        c->q.f_inv = 1.f / fs;
-        c->q.g_scale = gs;
-        c->q.g_inv = 1.f / gs;
+        choose_map(c, maxabs, rho_mean, shift);
     }
     lbm::StepView v = view(c, 0);
     LBM_CUDA(lbm::launch_quantize(c->box, c->q, c->p.storage, tf, tg, c->st.f0, const_cast<void *>(v.fq_in),
@@ -218,40 +213,51 @@ int load_state(lbm_ctx *c, const float *tf, const float *tg, const float *maxabs
     return LBM_OK;
 }
 
-// Equilibrium from the fields in c->st.mom into the state.  FP32 storage
-// holds the streamed FP32 distributions as they are, so the equilibrium is
-// written straight into half 0; the 16-bit formats go through FP32 scratch,
-// from which the storage map is chosen.
-int init_from_mom(lbm_ctx *c, const float *ghost_lo, const float *ghost_hi, const float *maxabs_in = nullptr,
-                  float *maxabs_out = nullptr)
+// Equilibrium from the fields in c->st.mom straight into the state's half 0.
+// The 16-bit storage map comes from the equilibrium's maxima, found by one
+// pass over phi and rho before the pass that stores.  rho_mean: the mean
+// density if the caller knows it (not positive: it is reduced here).
+// maxabs_in (26 floats: |f_k| and |g_i - shift_i| maxima) replaces the maxima
+// of this context's data (a z-slab takes the maxima of the whole box, reduced
+// over its slabs); maxabs_out receives this context's maxima (zeros for FP32).
+int init_from_mom(lbm_ctx *c, const float *ghost_lo, const float *ghost_hi, double rho_mean = 0.0,
+                  const float *maxabs_in = nullptr, float *maxabs_out = nullptr)
 {
     if (maxabs_out)
         for (int k = 0; k < lbm::kQf + lbm::kQg; k++) maxabs_out[k] = 0.f;
     const size_t n = (size_t)c->box.n;
-    if (c->p.storage == LBM_STORAGE_FP32) {
-        identity_quant(c->q);
-        const lbm::StepView v = view(c, 0);
-        LBM_CUDA(lbm::launch_equilibrium(c->box, c->d, c->p.Gamma, c->st.mom, c->st.mom + n, ghost_lo, ghost_hi,
-                                         c->st.f0, static_cast<float *>(const_cast<void *>(v.fq_in)),
-                                         static_cast<float *>(c->st.g), c->stream),
-                 "equilibrium kernel");
-        LBM_CUDA(cudaStreamSynchronize(c->stream), "init");
-        c->st.f_cur = 0;
-        c->st.f_streamed = true;
-        c->st.g_odd_next = false;
-        c->st.steps = 0;
-        return LBM_OK;
+    const float *phi = c->st.mom, *rho = c->st.mom + n;
+    identity_quant(c->q);
+    if (c->p.storage != LBM_STORAGE_FP32) {
+        if (!(rho_mean > 0.0)) {
+            if (int rc = reduce_stats(c)) return rc;
+            rho_mean = c->result_host[8] / (double)n;
+        }
+        float shift[lbm::kQg], maxabs[lbm::kQf + lbm::kQg], five[5];
+        g_shifts(rho_mean, shift);
+        unsigned *bits = reinterpret_cast<unsigned *>(c->result);   // free between statistics
+        LBM_CUDA(lbm::launch_equilibrium_maxabs(c->box, c->d, c->p.Gamma, shift, phi, rho, ghost_lo, ghost_hi, bits,
+                                                c->stream),
+                 "equilibrium maxima kernel");
+        LBM_CUDA(cudaMemcpyAsync(c->result_host, bits, sizeof(five), cudaMemcpyDeviceToHost, c->stream),
+                 "storage map");
+        LBM_CUDA(cudaStreamSynchronize(c->stream), "storage map");
+        std::memcpy(five, c->result_host, sizeof(five));
+        for (int k = 0; k < lbm::kQf; k++) maxabs[k] = five[k ? 1 : 0];
+        for (int i = 0; i < lbm::kQg; i++) maxabs[lbm::kQf + i] = five[i ? (i < 7 ? 3 : 4) : 2];
+        if (maxabs_out) std::memcpy(maxabs_out, maxabs, sizeof(maxabs));
+        choose_map(c, maxabs_in ? maxabs_in : maxabs, rho_mean, shift);
     }
-    float *tmp = nullptr;
-    LBM_CUDA(cudaMalloc(&tmp, sizeof(float) * (lbm::kQf + lbm::kQg) * n), "init scratch");
-    cudaError_t e = lbm::launch_equilibrium(c->box, c->d, c->p.Gamma, c->st.mom, c->st.mom + n, ghost_lo, ghost_hi,
-                                            tmp, tmp + n, tmp + lbm::kQf * n, c->stream);
-    int rc = e == cudaSuccess ? load_state(c, tmp, tmp + lbm::kQf * n, maxabs_in, maxabs_out)
-                              : cuda_fail(e, "equilibrium kernel");
-    cudaStreamSynchronize(c->stream);
-    cudaFree(tmp);
+    const lbm::StepView v = view(c, 0);
+    LBM_CUDA(lbm::launch_equilibrium(c->box, c->d, c->p.Gamma, c->q, c->p.storage, phi, rho, ghost_lo, ghost_hi,
+                                     c->st.f0, const_cast<void *>(v.fq_in), c->st.g, c->stream),
+             "equilibrium kernel");
+    LBM_CUDA(cudaStreamSynchronize(c->stream), "init");
+    c->st.f_cur = 0;
+    c->st.f_streamed = true;
+    c->st.g_odd_next = false;
     c->st.steps = 0;
-    return rc;
+    return LBM_OK;
 }
 
 }  // namespace
@@ -327,9 +333,8 @@ extern "C" int lbm_init(lbm_ctx **out, const lbm_params *p, const float *phi0, c
     if (e == cudaSuccess) e = cudaEventRecord(u_done, side);
     if (e == cudaSuccess && c->p.storage != LBM_STORAGE_FP32) e = cudaStreamWaitEvent(c->stream, u_done, 0);
     if (e == cudaSuccess && phi_ghost) {
-        e = cudaMalloc(&ghost, sizeof(float) * 2 * c->box.nxy);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(ghost, phi_ghost, sizeof(float) * 2 * c->box.nxy, cudaMemcpyHostToDevice, c->stream);
+        ghost = static_cast<float *>(view(c, 0).fq_out);   // f's other half is free until the first step
+        e = cudaMemcpyAsync(ghost, phi_ghost, sizeof(float) * 2 * c->box.nxy, cudaMemcpyHostToDevice, c->stream);
     }
     auto release_side = [&]() {
         if (side) cudaStreamSynchronize(side);
@@ -339,7 +344,6 @@ extern "C" int lbm_init(lbm_ctx **out, const lbm_params *p, const float *phi0, c
     if (e != cudaSuccess) {
         cudaStreamSynchronize(c->stream);
         release_side();
-        if (ghost) cudaFree(ghost);
         lbm_destroy(c);
         return cuda_fail(e, "lbm_init");
     }
@@ -348,7 +352,6 @@ extern "C" int lbm_init(lbm_ctx **out, const lbm_params *p, const float *phi0, c
     const cudaError_t ew = cudaStreamWaitEvent(c->stream, u_done, 0);
     if (ew != cudaSuccess && !rc) rc = cuda_fail(ew, "lbm_init");
     release_side();
-    if (ghost) cudaFree(ghost);
     if (rc) {
         lbm_destroy(c);
         return rc;
@@ -368,24 +371,31 @@ int init_bubbles_into(lbm_ctx *c, const float *bubbles, int nbubbles, int z0, co
                       float *maxabs_out)
 {
     const size_t n = (size_t)c->box.n, nxy = (size_t)c->box.nxy;
-    float *phig = nullptr, *bub = nullptr;
     float *mom = c->st.mom;
-    cudaError_t e = cudaMalloc(&phig, sizeof(float) * nxy * (c->box.nz + 2));
-    if (e == cudaSuccess && nbubbles > 0) e = cudaMalloc(&bub, sizeof(float) * 4 * nbubbles);
-    if (e == cudaSuccess && nbubbles > 0)
-        e = cudaMemcpyAsync(bub, bubbles, sizeof(float) * 4 * nbubbles, cudaMemcpyHostToDevice, c->stream);
+    // scratch inside the state: phi with its ghost planes in f's other half
+    // (at least 12 n bytes against 4 n + 8 nx ny), the bubble list in g, which
+    // is written only after the bubble kernel has read it
+    float *phig = static_cast<float *>(view(c, 0).fq_out);
+    float *bub = nullptr, *own = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (nbubbles > 0) {
+        const size_t bytes = sizeof(float) * 4 * (size_t)nbubbles;
+        if (bytes <= c->esz * lbm::kQg * n) bub = static_cast<float *>(c->st.g);
+        else if ((e = cudaMalloc(&own, bytes)) == cudaSuccess) bub = own;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(bub, bubbles, bytes, cudaMemcpyHostToDevice, c->stream);
+    }
     if (e == cudaSuccess)
         e = lbm::launch_bubble_phi(c->box, bub, nbubbles, c->d.phiStar, c->p.width, z0, phig, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(mom, phig + nxy, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream);
-    if (e == cudaSuccess) e = lbm::launch_fill(mom + n, (long long)n, 0.5f * (c->p.rhoH + c->p.rhoL), c->stream);
+    const float rho0 = 0.5f * (c->p.rhoH + c->p.rhoL);
+    if (e == cudaSuccess) e = lbm::launch_fill(mom + n, (long long)n, rho0, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(mom + 2 * n, 0, sizeof(float) * 3 * n, c->stream);
     const int rc = e == cudaSuccess
-                       ? init_from_mom(c, phig, phig + nxy * (c->box.nz + 1), maxabs_in, maxabs_out)
+                       ? init_from_mom(c, phig, phig + nxy * (c->box.nz + 1), rho0, maxabs_in, maxabs_out)
                        : cuda_fail(e, "bubble initial state");
     cudaStreamSynchronize(c->stream);
-    if (phig) cudaFree(phig);
-    if (bub) cudaFree(bub);
+    if (own) cudaFree(own);
     return rc;
 }
 

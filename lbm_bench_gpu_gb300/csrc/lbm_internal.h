@@ -152,11 +152,16 @@ StepConst step_const(const lbm_derived &d, const lbm_params &p, float grav);
 // being plane z0 of the bubbles' frame (0 for a whole box).
 cudaError_t launch_bubble_phi(const Box &b, const float *bubbles_dev, int nbubbles, float phiStar, float width,
                               int z0, float *phi_ghosted, cudaStream_t s);
-// At-rest equilibrium into FP32 arrays f_0 (n), f_1..f_6 (6 x n) and g (19 x n),
-// streamed natural layout.
-cudaError_t launch_equilibrium(const Box &b, const lbm_derived &d, float Gamma, const float *phi, const float *rho,
-                               const float *ghost_lo, const float *ghost_hi, float *f0, float *fq, float *g,
-                               cudaStream_t s);
+// At-rest equilibrium into f_0 (n floats), f_1..f_6 (6 x n) and g (19 x n) of a
+// state in its storage format and layout, streamed, mapped by q.
+cudaError_t launch_equilibrium(const Box &b, const lbm_derived &d, float Gamma, const Quant &q, int storage,
+                               const float *phi, const float *rho, const float *ghost_lo, const float *ghost_hi,
+                               float *f0, void *fq, void *g, cudaStream_t s);
+// Bits of the maxima of |f_0|, |f_1..6|, |g_0 - shift|, |g_1..6 - shift| and
+// |g_7..18 - shift| of that equilibrium (5 words at out, device; g_shift: 19, host).
+cudaError_t launch_equilibrium_maxabs(const Box &b, const lbm_derived &d, float Gamma, const float *g_shift,
+                                      const float *phi, const float *rho, const float *ghost_lo,
+                                      const float *ghost_hi, unsigned *out_bits, cudaStream_t s);
 cudaError_t launch_fill(float *p, long long n, float v, cudaStream_t s);
 // One step of the state in v; a z-slab (Box::zghost) may step planes
 // [zlo, zhi) of it only (zhi < 0: all), a periodic box steps whole.

@@ -1,8 +1,8 @@
 // zsc_init.cu -- initial condition kernels.
 //
 // bubble_phi_kernel   : src/init.c:39-59 (phi from the bubble list, on the GPU)
-// equilibrium_kernel  : src/init_f.cu:42-79 and src/init_g.cu:46-93
-#include "lbm_internal.h"
+// equilibrium_*kernel : src/init_f.cu:42-79 and src/init_g.cu:46-93
+#include "lattice.cuh"
 
 namespace lbm {
 namespace {
@@ -119,41 +119,134 @@ __global__ void __launch_bounds__(BTX * BTY) bubble_phi_tiled_kernel(Box b, cons
     }
 }
 
-// At-rest equilibrium from phi and rho.  z neighbours outside [0, nz) come
-// from ghost_lo / ghost_hi (nx*ny each) when given, else by periodic wrap.
-__global__ void equilibrium_kernel(Box b, float alpha4, float kappa, float phiStarSq, float Gamma,
-                                   const float *__restrict__ phi, const float *__restrict__ rho,
-                                   const float *__restrict__ ghost_lo, const float *__restrict__ ghost_hi,
-                                   float *__restrict__ f0, float *__restrict__ fq, float *__restrict__ g)
+// At-rest equilibrium of a node from phi and rho: f_0, the common value of
+// f_1..f_6, and g_0, of g_1..g_6 and of g_7..g_18.  z neighbours outside
+// [0, nz) come from ghost_lo / ghost_hi (nx*ny each) when given, else by
+// periodic wrap.  The last product of each g is kept from contracting with
+// what its reader subtracts, so every kernel below sees the same FP32 values.
+struct EqConst {
+    float alpha4, kappa, phiStarSq, Gamma;
+};
+struct Eq {
+    float f0, f1, g0, g1, g2;
+};
+__device__ __forceinline__ Eq equilibrium_at(const Box &b, const EqConst &c, const float *__restrict__ phi,
+                                             const float *__restrict__ rho, const float *__restrict__ ghost_lo,
+                                             const float *__restrict__ ghost_hi, int i, int j, int k)
 {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < b.n;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % b.nx);
-        const int j = (int)((t / b.nx) % b.ny);
-        const int k = (int)(t / b.nxy);
-        const int ie = i == b.nx - 1 ? 0 : i + 1, iw = i == 0 ? b.nx - 1 : i - 1;
-        const int jn = j == b.ny - 1 ? 0 : j + 1, js = j == 0 ? b.ny - 1 : j - 1;
-        auto P = [&](int x, int y, int z) -> float {
-            if (z < 0) return ghost_lo ? ghost_lo[x + b.nx * y] : phi[x + b.nx * (y + (long long)b.ny * (b.nz - 1))];
-            if (z >= b.nz) return ghost_hi ? ghost_hi[x + b.nx * y] : phi[x + b.nx * y];
-            return phi[x + b.nx * (y + (long long)b.ny * z)];
+    const int ie = i == b.nx - 1 ? 0 : i + 1, iw = i == 0 ? b.nx - 1 : i - 1;
+    const int rn = (j == b.ny - 1 ? 0 : j + 1) * b.nx, rs = (j == 0 ? b.ny - 1 : j - 1) * b.nx, rc = j * b.nx;
+    const float *const pc = phi + (size_t)k * b.nxy;
+    const float *const pt = k == b.nz - 1 ? (ghost_hi ? ghost_hi : phi) : pc + b.nxy;
+    const float *const pb = k == 0 ? (ghost_lo ? ghost_lo : phi + (size_t)(b.nz - 1) * b.nxy) : pc - b.nxy;
+    const float phin = pc[rc + i];
+    const float lap = (pc[rn + ie] + pc[rs + iw] + pc[rs + ie] + pc[rn + iw] + pt[rc + ie] + pb[rc + iw] + pb[rc + ie]
+                       + pt[rc + iw] + pt[rn + i] + pb[rs + i] + pb[rn + i] + pt[rs + i]
+                       + 2.f * (pc[rc + ie] + pc[rc + iw] + pc[rn + i] + pc[rs + i] + pt[rc + i] + pb[rc + i]
+                                - 12.f * phin)) * kInv6;
+    const float mu = c.alpha4 * phin * (phin * phin - c.phiStarSq) - c.kappa * lap;
+    const float rhon = rho[(size_t)k * b.nxy + rc + i];
+    Eq e;
+    e.f0 = phin - 3.f * c.Gamma * mu;
+    e.f1 = 0.5f * c.Gamma * mu;
+    e.g0 = __fmul_rn(kW0, rhon - 6.f * phin * mu);
+    e.g1 = __fmul_rn(kW1, 3.f * phin * mu + rhon);
+    e.g2 = __fmul_rn(kW2, 3.f * phin * mu + rhon);
+    return e;
+}
+
+// A block: a 32 x 8 tile (16-bit: 16 words of the pair layout, i.e. 32 nodes, x
+// 8 rows) of EQZ planes.  The stores bound these kernels (104 or 54 bytes a
+// node against 8 read).
+constexpr int EQZ = 4;
+
+// FP32 storage: the streamed natural layout is the equilibrium itself.
+__global__ void __launch_bounds__(256) equilibrium_kernel(Box b, EqConst c, const float *__restrict__ phi,
+                                                          const float *__restrict__ rho,
+                                                          const float *__restrict__ ghost_lo,
+                                                          const float *__restrict__ ghost_hi, float *__restrict__ f0,
+                                                          float *__restrict__ fq, float *__restrict__ g)
+{
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+#pragma unroll 1
+    for (int k = blockIdx.z * EQZ, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
+        const Eq e = equilibrium_at(b, c, phi, rho, ghost_lo, ghost_hi, i, j, k);
+        const size_t t = (size_t)k * b.nxy + j * b.nx + i;
+        f0[t] = e.f0;
+#pragma unroll
+        for (int q = 0; q < kQf - 1; q++) fq[q * b.n + t] = e.f1;
+        g[t] = e.g0;
+#pragma unroll
+        for (int q = 1; q < kQg; q++) g[q * b.n + t] = q < 7 ? e.g1 : e.g2;
+    }
+}
+
+// 16-bit storage: the two nodes of one pair-layout word, mapped and stored as
+// one word per field (the values a quantize_kernel of the FP32 equilibrium
+// would store, without that scratch copy).
+template <typename ST>
+__global__ void __launch_bounds__(128) equilibrium_store_kernel(Box b, EqConst c, Quant q,
+                                                                const float *__restrict__ phi,
+                                                                const float *__restrict__ rho,
+                                                                const float *__restrict__ ghost_lo,
+                                                                const float *__restrict__ ghost_hi,
+                                                                float *__restrict__ f0, ST *__restrict__ fq,
+                                                                ST *__restrict__ g)
+{
+    using T2 = typename Fmt<ST>::T2;
+    const int w = blockIdx.x * 16 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+#pragma unroll 1
+    for (int k = blockIdx.z * EQZ, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
+        const Eq a = equilibrium_at(b, c, phi, rho, ghost_lo, ghost_hi, w, j, k);
+        const Eq d = equilibrium_at(b, c, phi, rho, ghost_lo, ghost_hi, w + b.nx / 2, j, k);
+        const size_t t = (size_t)k * b.nxy + j * b.nx + 2 * w;   // the word's first element
+        *reinterpret_cast<float2 *>(f0 + t) = make_float2(a.f0, d.f0);
+        const T2 f1 = Fmt<ST>::store2(make_float2(__fmul_rn(a.f1, q.f_scale), __fmul_rn(d.f1, q.f_scale)));
+#pragma unroll
+        for (int m = 0; m < kQf - 1; m++) *reinterpret_cast<T2 *>(fq + m * b.n + t) = f1;
+        auto map = [&](float va, float vb, int m) {
+            return Fmt<ST>::store2(make_float2((va - q.g_shift[m]) * q.g_scale, (vb - q.g_shift[m]) * q.g_scale));
         };
-        const int kt = k + 1, kb = k - 1;
-        const float phin = phi[t];
-        const float lap = (P(ie, jn, k) + P(iw, js, k) + P(ie, js, k) + P(iw, jn, k) + P(ie, j, kt) + P(iw, j, kb)
-                           + P(ie, j, kb) + P(iw, j, kt) + P(i, jn, kt) + P(i, js, kb) + P(i, jn, kb) + P(i, js, kt)
-                           + 2.f * (P(ie, j, k) + P(iw, j, k) + P(i, jn, k) + P(i, js, k) + P(i, j, kt) + P(i, j, kb)
-                                    - 12.f * phin)) * kInv6;
-        const float mu = alpha4 * phin * (phin * phin - phiStarSq) - kappa * lap;
-        const float Af = 0.5f * Gamma * mu;
-        f0[t] = phin - 3.f * Gamma * mu;
-        for (int q = 1; q < kQf; q++) fq[(q - 1) * b.n + t] = Af;
-        const float rhon = rho[t];
-        const float Ag1 = kW1 * (3.f * phin * mu + rhon);
-        const float Ag2 = kW2 * (3.f * phin * mu + rhon);
-        g[t] = kW0 * (rhon - 6.f * phin * mu);
-        for (int q = 1; q < 7; q++) g[q * b.n + t] = Ag1;
-        for (int q = 7; q < kQg; q++) g[q * b.n + t] = Ag2;
+        const T2 g0 = map(a.g0, d.g0, 0), g1 = map(a.g1, d.g1, 1), g2 = map(a.g2, d.g2, 7);
+        *reinterpret_cast<T2 *>(g + t) = g0;
+#pragma unroll
+        for (int m = 1; m < kQg; m++) *reinterpret_cast<T2 *>(g + m * b.n + t) = m < 7 ? g1 : g2;
+    }
+}
+
+// out_bits[0..4] = bits of max |f_0|, |f_1..6|, |g_0 - s_0|, |g_1..6 - s_1|,
+// |g_7..18 - s_2| over the equilibrium (non-negative floats order like their
+// bits), from which the 16-bit storage map is chosen.
+__global__ void __launch_bounds__(256) equilibrium_maxabs_kernel(Box b, EqConst c, float s0, float s1, float s2,
+                                                                 const float *__restrict__ phi,
+                                                                 const float *__restrict__ rho,
+                                                                 const float *__restrict__ ghost_lo,
+                                                                 const float *__restrict__ ghost_hi,
+                                                                 unsigned *__restrict__ out_bits)
+{
+    __shared__ unsigned red[8][5];
+    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    float m[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int k = blockIdx.z * EQZ, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
+        const Eq e = equilibrium_at(b, c, phi, rho, ghost_lo, ghost_hi, i, j, k);
+        m[0] = fmaxf(m[0], fabsf(e.f0));
+        m[1] = fmaxf(m[1], fabsf(e.f1));
+        m[2] = fmaxf(m[2], fabsf(e.g0 - s0));
+        m[3] = fmaxf(m[3], fabsf(e.g1 - s1));
+        m[4] = fmaxf(m[4], fabsf(e.g2 - s2));
+    }
+#pragma unroll
+    for (int v = 0; v < 5; v++) {
+        const unsigned r = __reduce_max_sync(0xffffffffu, __float_as_uint(m[v]));
+        if (threadIdx.x == 0) red[threadIdx.y][v] = r;
+    }
+    __syncthreads();
+    if (threadIdx.y == 0 && threadIdx.x < 5) {
+        unsigned r = red[0][threadIdx.x];
+        for (int w = 1; w < 8; w++) r = max(r, red[w][threadIdx.x]);
+        // most blocks do not raise the maximum: look before the atomic
+        if (r > *reinterpret_cast<volatile unsigned *>(out_bits + threadIdx.x)) atomicMax(out_bits + threadIdx.x, r);
     }
 }
 
@@ -186,12 +279,50 @@ cudaError_t launch_bubble_phi(const Box &b, const float *bubbles_dev, int nbubbl
     return cudaGetLastError();
 }
 
-cudaError_t launch_equilibrium(const Box &b, const lbm_derived &d, float Gamma, const float *phi, const float *rho,
-                               const float *ghost_lo, const float *ghost_hi, float *f0, float *fq, float *g,
-                               cudaStream_t s)
+namespace {
+EqConst eq_const(const lbm_derived &d, float Gamma) { return EqConst{d.alpha4, d.kappa, d.phiStarSq, Gamma}; }
+dim3 eq_grid(const Box &b)
 {
-    equilibrium_kernel<<<grid_for(b.n), 256, 0, s>>>(b, d.alpha4, d.kappa, d.phiStarSq, Gamma, phi, rho, ghost_lo,
-                                                      ghost_hi, f0, fq, g);
+    return dim3((unsigned)(b.nx / 32), (unsigned)(b.ny / 8), (unsigned)((b.nz + EQZ - 1) / EQZ));
+}
+}  // namespace
+
+cudaError_t launch_equilibrium(const Box &b, const lbm_derived &d, float Gamma, const Quant &q, int storage,
+                               const float *phi, const float *rho, const float *ghost_lo, const float *ghost_hi,
+                               float *f0, void *fq, void *g, cudaStream_t s)
+{
+    if (b.nx % 32 != 0 || b.ny % 8 != 0) return cudaErrorInvalidValue;
+    const EqConst c = eq_const(d, Gamma);
+    const dim3 pair(16, 8);
+    switch (storage) {
+    case LBM_STORAGE_FP32:
+        equilibrium_kernel<<<eq_grid(b), dim3(32, 8), 0, s>>>(b, c, phi, rho, ghost_lo, ghost_hi, f0,
+                                                             static_cast<float *>(fq), static_cast<float *>(g));
+        break;
+    case LBM_STORAGE_FP16:
+        equilibrium_store_kernel<__half><<<eq_grid(b), pair, 0, s>>>(b, c, q, phi, rho, ghost_lo, ghost_hi, f0,
+                                                                     static_cast<__half *>(fq),
+                                                                     static_cast<__half *>(g));
+        break;
+    case LBM_STORAGE_BF16:
+        equilibrium_store_kernel<__nv_bfloat16><<<eq_grid(b), pair, 0, s>>>(
+            b, c, q, phi, rho, ghost_lo, ghost_hi, f0, static_cast<__nv_bfloat16 *>(fq),
+            static_cast<__nv_bfloat16 *>(g));
+        break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_equilibrium_maxabs(const Box &b, const lbm_derived &d, float Gamma, const float *g_shift,
+                                      const float *phi, const float *rho, const float *ghost_lo,
+                                      const float *ghost_hi, unsigned *out_bits, cudaStream_t s)
+{
+    if (b.nx % 32 != 0 || b.ny % 8 != 0) return cudaErrorInvalidValue;
+    cudaError_t e = cudaMemsetAsync(out_bits, 0, 5 * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    equilibrium_maxabs_kernel<<<eq_grid(b), dim3(32, 8), 0, s>>>(b, eq_const(d, Gamma), g_shift[0], g_shift[1],
+                                                                 g_shift[7], phi, rho, ghost_lo, ghost_hi, out_bits);
     return cudaGetLastError();
 }
 
