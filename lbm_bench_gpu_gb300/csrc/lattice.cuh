@@ -28,16 +28,11 @@ __host__ __device__ constexpr int kCz(int i)
 }
 __host__ __device__ constexpr int kOpp(int i) { return i == 0 ? 0 : ((i & 1) ? i + 1 : i - 1); }
 
-// Storage formats: element conversions, and the resident blocks per SM the
-// step kernel's launch bounds ask for.  FP32 stages 108 KB of shared memory
-// per block (2 blocks of 256 threads per SM, 128 registers); the 16-bit
-// formats stage 54 KB per block of 128 threads, 4 blocks per SM (128
-// registers).
+// Storage formats: element conversions.
 template <typename ST>
 struct Fmt;
 template <>
 struct Fmt<float> {
-    static constexpr int kMinBlocks = 2;
     static constexpr bool kMapped = false;
     using T2 = float2;   // (unused: FP32 keeps one node per thread)
     __device__ static float load(float v) { return v; }
@@ -49,7 +44,6 @@ struct Fmt<float> {
 };
 template <>
 struct Fmt<__half> {
-    static constexpr int kMinBlocks = 4;
     static constexpr bool kMapped = true;
     using T2 = __half2;   // two adjacent nodes, one 32-bit word
     __device__ static float load(__half v) { return __half2float(v); }
@@ -66,7 +60,6 @@ struct Fmt<__half> {
 };
 template <>
 struct Fmt<__nv_bfloat16> {
-    static constexpr int kMinBlocks = 4;
     static constexpr bool kMapped = true;
     using T2 = __nv_bfloat162;
     __device__ static float load(__nv_bfloat16 v) { return __bfloat162float(v); }

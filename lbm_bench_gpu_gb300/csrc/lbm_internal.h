@@ -113,13 +113,17 @@ struct AdjointBuffers {
 
 // Planes per block of a kernel whose blocks march `planes` planes on `tiles`
 // column tiles, per_sm of them resident on each of sms SMs.  A block's time is
-// about (tz + prologue) plane-times, and r blocks that share an SM slow each
-// other down by share[r] (less than r: a lone block is bound by its own
-// latencies).  The launch takes as many full rounds of resident blocks as there
-// are, then a last, partly filled one, which overlaps the end of the others
-// (tail).  The depth that minimises the sum is taken.
-inline int march_depth(long long tiles, int planes, int sms, int per_sm, double prologue, double tail,
-                       const double *share)
+// about (tz + prologue) plane-times (of `plane`, to compare kernels), and r
+// blocks that share an SM slow each other down by share[r] (less than r: a lone
+// block is bound by its own latencies).  The launch takes as many full rounds
+// of resident blocks as there are, then a last, partly filled one, which
+// overlaps the end of the others (tail).  The depth that minimises the sum is
+// taken.
+struct MarchCost {
+    double prologue, tail;
+    double share[8];
+};
+inline int march_depth(long long tiles, int planes, int sms, int per_sm, const MarchCost &m)
 {
     const long long slots = (long long)sms * per_sm;
     int best = 1;
@@ -127,9 +131,9 @@ inline int march_depth(long long tiles, int planes, int sms, int per_sm, double 
     for (int tz = 1; tz <= 64; tz++) {
         const long long blocks = tiles * ((planes + tz - 1) / tz);
         const long long full = blocks / slots, rest = blocks % slots;
-        double rounds = (double)full * share[per_sm];
-        if (rest > 0) rounds += (full > 0 ? tail : 1.0) * share[(rest + sms - 1) / sms];
-        const double cost = rounds * (tz + prologue);
+        double rounds = (double)full * m.share[per_sm];
+        if (rest > 0) rounds += (full > 0 ? m.tail : 1.0) * m.share[(rest + sms - 1) / sms];
+        const double cost = rounds * (tz + m.prologue);
         if (best_cost < 0.0 || cost < best_cost) {
             best_cost = cost;
             best = tz;
@@ -137,6 +141,7 @@ inline int march_depth(long long tiles, int planes, int sms, int per_sm, double 
     }
     return best;
 }
+int sm_count();   // SMs of the current device (read once per process)
 
 void set_error(const std::string &msg);
 const std::string &last_error();

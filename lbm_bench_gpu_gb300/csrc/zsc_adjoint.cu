@@ -895,29 +895,19 @@ dim3 adjoint_grid(const Box &b)
 struct March {
     int tz, blocks;
 };
-int sm_count()
-{
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return std::max(1, n);
-    }();
-    return sms;
-}
 March march_of(const Box &b)
 {
-    constexpr double share[3] = {0.0, 1.0, 1.4};
+    constexpr MarchCost cost = {1.0, 0.88, {0.0, 1.0, 1.4}};
     const int tiles = (b.nx / TXA) * (b.ny / TYA);
-    const int tz = march_depth(tiles, b.nz, sm_count(), 2, 1.0, 0.88, share);
+    const int tz = march_depth(tiles, b.nz, sm_count(), 2, cost);
     return March{tz, tiles * ((b.nz + tz - 1) / tz)};
 }
 // The stencil kernel's: a prologue of two planes, kStencilBlocks blocks on an SM.
 March stencil_march(const Box &b)
 {
-    constexpr double share[kStencilBlocks + 1] = {0.0, 1.0, 1.2, 1.5, 1.8, 2.2};
+    constexpr MarchCost cost = {2.0, 0.88, {0.0, 1.0, 1.2, 1.5, 1.8, 2.2}};
     const int tiles = (b.nx / TXA) * (b.ny / TYA);
-    const int tz = march_depth(tiles, b.nz, sm_count(), kStencilBlocks, 2.0, 0.88, share);
+    const int tz = march_depth(tiles, b.nz, sm_count(), kStencilBlocks, cost);
     return March{tz, tiles * ((b.nz + tz - 1) / tz)};
 }
 

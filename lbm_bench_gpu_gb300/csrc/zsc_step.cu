@@ -76,7 +76,6 @@ constexpr int RING = 2 * RW + 2 * TY;
 constexpr int TXW = TX / 2;
 constexpr int RWP = TXW + 2;
 constexpr int RINGP = 2 * RWP + 2 * TY;
-constexpr int NG = 2;               // g stages
 static_assert(RING <= NT, "one ring node per thread at most");
 static_assert(TX == 32 && TY == 8, "issuer roles assume a 32 x 8 tile");
 
@@ -127,19 +126,32 @@ struct Dir {
     static constexpr int value = I;
 };
 
-// Staging geometry implied by the element size.  FP32 (two blocks per SM)
-// stages 4 P_f planes and 4 phi planes; the 16-bit formats fit four blocks per
-// SM into the shared memory with 3 + 3 and g rows one chunk narrower (the odd
-// step's shifted rows need one extra chunk on one side only).
-template <typename ST>
+// Staging geometry.  16-bit storage: 2 g stages, 3 P_f planes (54 KB a block of
+// 128 threads, four blocks per SM).  FP32 has two:
+//   deep  2 g stages, 4 P_f planes (103 KB a block of 256 threads, two per SM):
+//         the next plane's g and the P_f plane three ahead are in flight for a
+//         whole plane, which a lone block on an SM needs;
+//   dense 1 g stage, 3 P_f planes (66 KB, 80 registers, three per SM): the next
+//         g rows follow once the current ones are in registers, and the third
+//         block covers the shorter flight.
+// FP32, deep -> dense: 256^3 610 -> 605 us a step, 128^3 84.3 -> 81.0, 160 x 104
+// x 93 65.5 -> 60.7; but 64^3 13.8 -> 14.7, 32^3 4.1 -> 4.5: choose_plan takes
+// one by the box.  (16-bit storage with one
+// g stage and five blocks of 96 registers spills and is slower: 256^3 346 ->
+// 400 us.)
+// g rows carry one extra chunk (an odd step's shifted rows need it on one side
+// only).
+template <typename ST, bool DEEP>
 struct Geo {
     static constexpr bool kSmall = sizeof(ST) == 2;
     static constexpr int E = 16 / (int)sizeof(ST);   // elements per 16-byte chunk
     static constexpr int W = TX + 2 * E;             // staged P_f row: x in [x0 - E, x0 + TX + E)
-    static constexpr int GW = kSmall ? TX + E : TX + 2 * E;   // staged g row
-    static constexpr int GX0 = kSmall ? 0 : E;       // g row column of x0 (even step: E)
-    static constexpr int NF = kSmall ? 3 : 4;        // P_f stages
-    static constexpr int NPHI = kSmall ? 3 : 4;      // phi planes
+    static constexpr int GW = TX + E;                // staged g row
+    static constexpr int GX0 = 0;                    // g row column of x0 (even step: E)
+    static constexpr int NG = kSmall || DEEP ? 2 : 1;     // g stages
+    static constexpr int NF = !kSmall && DEEP ? 4 : 3;    // P_f stages
+    static constexpr int NPHI = NF;                  // phi planes
+    static constexpr int kMinBlocks = kSmall ? 4 : DEEP ? 2 : 3;   // resident blocks per SM
     static constexpr int CR = W / E;                 // chunks per staged row
     static constexpr int CM = TX / E;                // chunks covering [x0, x0 + TX)
     static constexpr int G_STAGE = kQg * TY * GW * (int)sizeof(ST);           // bytes
@@ -203,6 +215,11 @@ __device__ __forceinline__ bool in_field(long long idx, int count, long long n, 
     return true;
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_prior()   // all but this thread's last N groups
+{
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
 // ---- mbarrier + TMA (bulk tensor copy) ----
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -368,16 +385,16 @@ __device__ __forceinline__ unsigned node_index(const StepBox &b, int x, int y, i
 
 // ZG: the box is a z-slab whose fields carry ghost planes (Box::zghost): a
 // separate instance, so the periodic kernels keep their registers.
-template <typename ST, bool STREAMED, bool ODD, bool TMA, bool ZG>
-__global__ void __launch_bounds__(threads_of<ST>(), Fmt<ST>::kMinBlocks)
+template <typename ST, bool DEEP, bool STREAMED, bool ODD, bool TMA, bool ZG>
+__global__ void __launch_bounds__(threads_of<ST>(), (Geo<ST, DEEP>::kMinBlocks))
 zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const StepMap m, const int tz,
                 const int write_moments, const int zlo, const int zhi, const __grid_constant__ CUtensorMap gmap,
                 const __grid_constant__ CUtensorMap f0map, const __grid_constant__ CUtensorMap fqmap)
 {
-    using Gm = Geo<ST>;
+    using Gm = Geo<ST, DEEP>;
     using Fm = Fmt<ST>;
     constexpr int E = Gm::E, W = Gm::W, GW = Gm::GW, GX0 = Gm::GX0, CR = Gm::CR, CM = Gm::CM;
-    constexpr int NF = Gm::NF, NPHI = Gm::NPHI;
+    constexpr int NG = Gm::NG, NF = Gm::NF, NPHI = Gm::NPHI;
     extern __shared__ __align__(128) unsigned char smem[];
     ST *const G = reinterpret_cast<ST *>(smem + Gm::G_OFF);            // [NG][19][TY][GW]
     unsigned char *const F = smem + Gm::F_OFF;                          // [NF]{f0 [FR][W0]; fq [6][FR][W]}
@@ -708,17 +725,16 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
 
     // prologue: P_f planes z0-2 .. z0+1 (with 3 stages: z0+1 after the first
     // build), g of plane z0; phi of z0-1 and z0
-    constexpr int kAhead = NF - 1;   // P_f planes past z0 - 2 staged before the first build
     issue_f(z0 - 2);
     issue_f(z0 - 1);
     issue_f(z0);
-    if (kAhead >= 3) issue_f(z0 + 1);
+    if constexpr (NF == 4) issue_f(z0 + 1);
     issue_g(z0, 0);
     cp_async_commit();
     cp_async_wait_all();
     bool late = false;
     if (tile_tma_f) {
-        for (int p = z0 - 2; p <= z0 - 2 + kAhead; p++) late |= !mbar_wait(fbar(p), fphase(p));
+        for (int p = z0 - 2; p <= z0 - 3 + NF; p++) late |= !mbar_wait(fbar(p), fphase(p));
     }
     __syncthreads();
     if constexpr (PAIR) {
@@ -728,7 +744,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
         float tmp[XPT][kQf];
         build_plane(z0 - 1, pslot(z0 - 1), tmp);
     }
-    if (kAhead < 3) {
+    if constexpr (NF == 3) {
         // the stage of plane z0 - 2 is free once every thread has built z0 - 1
         __syncthreads();
         issue_f(z0 + 1);
@@ -742,41 +758,55 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
     __syncthreads();
     issue_f(z0 + 2);
     cp_async_commit();
+    if constexpr (NG == 1) cp_async_commit();   // (g of plane z0 has landed: its group is empty)
 
     for (int j = 0; j < nzc; ++j) {
         const int z = z0 + j;
-        cp_async_wait_all();
+        if constexpr (NG == 1) cp_async_wait_prior<1>();   // P_f of plane z + 2; g of plane z may be on its way
+        else cp_async_wait_all();
         __syncthreads();
-        if (j + 1 < nzc) {
-            issue_g(z + 1, (j + 1) & 1);
-            if (kAhead >= 3) issue_f(z + 3);
+        if constexpr (NG == 2) {
+            if (j + 1 < nzc) {
+                issue_g(z + 1, (j + 1) & 1);
+                if constexpr (NF == 4) issue_f(z + 3);
+            }
+            cp_async_commit();
         }
-        cp_async_commit();
         // P_f plane z + 2 is first read here (a late copy only spoils values:
         // the uniform exit below comes before anything is stored)
         if (tile_tma_f) late |= !mbar_wait(fbar(z + 2), fphase(z + 2));
         if constexpr (PAIR) build_pair(z + 1, pslot(z + 1), fnext2);
         else build_plane(z + 1, pslot(z + 1), fnext);
+        if constexpr (NG == 1) cp_async_wait_all();   // g of plane z (cp.async tiles)
         if constexpr (TMA) {
-            // g of plane z: stage j & 1, its (j >> 1)-th use (cp.async tiles
-            // were complete at the barrier above)
-            if (g_tma) late |= !mbar_wait(&mbar[j & 1], (unsigned)(j >> 1) & 1u);
+            // g of plane z: stage j % NG, its (j / NG)-th use (cp.async tiles
+            // are complete at this barrier)
+            if (g_tma) late |= !mbar_wait(&mbar[j % NG], (unsigned)(j / NG) & 1u);
             if (__syncthreads_or(late)) {
                 if (tid == 0) atomicOr(P.err, 1);
                 // copies still in flight: wait for them (bounded) before leaving
-                if (g_tma && j + 1 < nzc) mbar_wait(&mbar[(j + 1) & 1], (unsigned)((j + 1) >> 1) & 1u);
-                if (kAhead >= 3 && tile_tma_f && j + 1 < nzc) mbar_wait(fbar(z + 3), fphase(z + 3));
+                if (NG == 2 && g_tma && j + 1 < nzc) mbar_wait(&mbar[(j + 1) & 1], (unsigned)((j + 1) >> 1) & 1u);
+                if (NF == 4 && tile_tma_f && j + 1 < nzc) mbar_wait(fbar(z + 3), fphase(z + 3));
                 return;
             }
         } else {
             __syncthreads();
         }
-        // with 3 P_f stages plane z + 3 goes into plane z's stage, free now
-        // that every thread has built phi of z + 1
-        if (kAhead < 3) {
+        // with 3 P_f stages plane z + 3 goes into plane z's, free now that
+        // every thread has built phi of z + 1
+        if constexpr (NF == 3) {
             if (j + 1 < nzc) issue_f(z + 3);
             cp_async_commit();
         }
+        // with one g stage plane z + 1's rows follow once every thread holds
+        // its g values of plane z in registers
+        auto g_is_read = [&]() {
+            if constexpr (NG == 1) {
+                __syncthreads();
+                if (j + 1 < nzc) issue_g(z + 1, 0);
+                cp_async_commit();
+            }
+        };
 
         const float *S0 = PHI + pslot(z - 1) * (RH * RW);   // plane z - 1
         const float *S1 = PHI + pslot(z) * (RH * RW);       // plane z
@@ -812,12 +842,13 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
 
         // D3Q19 values of this node from the staged rows (AA pattern), in
         // stored units
-        const ST *Gs = G + (j & 1) * G_ELEMS;
+        const ST *Gs = G + (j % NG) * G_ELEMS;
         float g[kQg];
 #pragma unroll
         for (int i = 0; i < kQg; i++)
             g[i] = Fm::load((TMA && !ODD) ? Gs[(i * TY + ty) * TX + tx]
                             : Gs[(i * TY + ty) * GW + (!ODD || kCx(i) > 0 ? E : GX0) + tx - (ODD ? kCx(i) : 0)]);
+        g_is_read();
 
         // moments: src/update_rho.cu:46-50, src/update_velocity.cu:47-59
         float rho = g[0];
@@ -1028,7 +1059,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
             // odd step's x-shifted direction reads the neighbouring word, which
             // came round the x seam (swapped) for the first / last word of a
             // seam tile
-            const ST *Gs = G + (j & 1) * G_ELEMS;
+            const ST *Gs = G + (j % NG) * G_ELEMS;
             const bool wrap_l = seam_l && tx == 0, wrap_r = seam_r && tx == TXW - 1;
             const unsigned sel_l = wrap_l ? kSwap : kKeep, sel_r = wrap_r ? kSwap : kKeep;
             float2 g[kQg];
@@ -1046,6 +1077,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
                     g[i] = Fm::load2(Fm::perm2(v, kCx(i) > 0 ? sel_l : sel_r));
                 }
             }
+            g_is_read();
 
             // moments (stored units: rho = g_inv sum + sum of shifts)
             float2 rho = g[0];
@@ -1176,17 +1208,17 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
     }
 }
 
-template <typename ST, bool S, bool O, bool T, bool Z>
+template <typename ST, bool DEEP, bool S, bool O, bool T, bool Z>
 cudaError_t configure()
 {
     static bool done = false;   // per template instance, per process
     if (done) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(zsc_step_kernel<ST, S, O, T, Z>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Geo<ST>::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(zsc_step_kernel<ST, DEEP, S, O, T, Z>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         Geo<ST, DEEP>::SMEM);
     // all of the unified L1 / shared storage as shared memory: the resident
     // blocks per SM the launch bounds ask for need it
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(zsc_step_kernel<ST, S, O, T, Z>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        e = cudaFuncSetAttribute(zsc_step_kernel<ST, DEEP, S, O, T, Z>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  (int)cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess) done = true;
     return e;
@@ -1259,50 +1291,66 @@ bool encode_f_maps(const Box &b, const float *f0, const ST *fq, CUtensorMap *f0m
     const cuuint64_t es = sizeof(ST);
     const cuuint64_t dims[4] = {(cuuint64_t)b.nx, (cuuint64_t)b.ny, (cuuint64_t)(b.nf / b.nxy), (cuuint64_t)(kQf - 1)};
     const cuuint64_t strides[3] = {(cuuint64_t)b.nx * es, (cuuint64_t)b.nxy * es, (cuuint64_t)b.nf * es};
-    const cuuint32_t box[4] = {(cuuint32_t)Geo<ST>::W, (cuuint32_t)FR, 1u, (cuuint32_t)(kQf - 1)};
+    const cuuint32_t box[4] = {(cuuint32_t)Geo<ST, false>::W, (cuuint32_t)FR, 1u, (cuuint32_t)(kQf - 1)};
     return encode(fqmap, tensor_type<ST>(), 4, const_cast<ST *>(fq), dims, strides, box, elem,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Planes per block (march_depth).
-// The four constants were fitted to forced depths 1 .. 64 on nine boxes from
-// 32^3 to 256^3 in FP32 and FP16: the choice is within 1.1% of the best depth
-// on average, 6.4% at most.  (Measured, depth before -> now: 32^3 FP32 4 -> 1
-// plane, 8.2 -> 4.1 us; 32 x 64 x 48 FP32 12.1 -> 6.8, FP16 16.0 -> 7.1 us;
-// 64^3 FP16 4 -> 2 planes, 16.9 -> 11.0 us; 192^3 FP16 48 -> 24 planes, 171 ->
-// 159 us; 256^3 unchanged.)
-struct Slots {
-    int sms, per_sm;   // SMs, and the kernel's resident blocks on each
+// Staging geometry and planes per block of a launch.
+//
+// FP32 takes the deep geometry below 16 tile-planes (32 x 8 nodes) per SM, the
+// dense one from there: below, blocks are alone or two on an SM and bound by
+// their own latencies.  Best of each over forced depths, deep / dense: 6.7
+// tile-planes per SM (64^3) 13.9 / 14.7 us, 12.6 (96 x 64 x 80) 21.0 / 21.1,
+// 22.7 (96^3) 35.0 / 34.5, 39.8 (160 x 104 x 93) 64.4 / 60.7.
+//
+// The depth comes from march_depth, its constants fitted to forced depths
+// 1 .. 64 on nine boxes from 32^3 to 256^3: the choice is within 1.1% of the
+// best depth on average for the deep and the 16-bit kernels (6.4% at most) and
+// 0.3% for the dense one.  (Depth of at least 4 planes and a cost without the
+// share of an SM, before -> now: 32^3 FP32 8.2 -> 4.1 us, 32 x 64 x 48 FP32
+// 12.1 -> 6.8, FP16 16.0 -> 7.1; 64^3 FP16 16.9 -> 11.0; 192^3 FP16 171 -> 159.)
+struct Plan {
+    bool deep;
+    int tz;
 };
-template <typename ST>
-Slots resident_slots()
+
+template <typename ST, bool DEEP>
+int resident_blocks()   // per SM; per instance, per process
 {
-    static const Slots slots = [] {   // per storage type, per process
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, zsc_step_kernel<ST, false, false, false, false>,
-                                                      threads_of<ST>(), Geo<ST>::SMEM);
-        return Slots{std::max(1, sms), std::max(1, std::min(per_sm, Fmt<ST>::kMinBlocks))};
+    static const int blocks = [] {
+        int n = 0;
+        configure<ST, DEEP, false, false, false, false>();   // its shared memory above the default limit
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, zsc_step_kernel<ST, DEEP, false, false, false, false>,
+                                                      threads_of<ST>(), Geo<ST, DEEP>::SMEM);
+        return std::max(1, std::min(n, Geo<ST, DEEP>::kMinBlocks));
     }();
-    return slots;
+    return blocks;
 }
 
 template <typename ST>
-int choose_tz(const Box &b)
+Plan choose_plan(const Box &b)
 {
     // a thread's steps are mostly on one box: its last answer is kept
-    static thread_local int last[4] = {0, 0, 0, 0};
-    if (last[0] == b.nx && last[1] == b.ny && last[2] == b.nz) return last[3];
-    const auto [sms, per_sm] = resident_slots<ST>();
-    constexpr double share[5] = {0.0, 1.0, sizeof(ST) == 2 ? 1.43 : 1.40, 1.90, 2.28};
-    const int best = march_depth((long long)(b.nx / TX) * (b.ny / TY), b.nz, sms, per_sm, 1.25, 0.88, share);
+    static thread_local int last[3] = {0, 0, 0};
+    static thread_local Plan plan = {false, 1};
+    if (last[0] == b.nx && last[1] == b.ny && last[2] == b.nz) return plan;
+    const long long tiles = (long long)(b.nx / TX) * (b.ny / TY);
+    const int sms = sm_count();
+    if constexpr (sizeof(ST) == 2) {
+        constexpr MarchCost cost = {1.25, 0.88, {0.0, 1.0, 1.43, 1.90, 2.28}};
+        plan.tz = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), cost);
+    } else {
+        constexpr MarchCost deep = {1.25, 0.88, {0.0, 1.0, 1.40}}, dense = {3.0, 0.84, {0.0, 1.0, 1.60, 1.71}};
+        plan.deep = tiles * b.nz < 16LL * sms;
+        plan.tz = plan.deep ? march_depth(tiles, b.nz, sms, resident_blocks<ST, true>(), deep)
+                            : march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), dense);
+    }
     last[0] = b.nx;
     last[1] = b.ny;
     last[2] = b.nz;
-    last[3] = best;
-    return best;
+    return plan;
 }
 
 // A step launch with programmatic stream serialization (the kernel orders
@@ -1346,13 +1394,6 @@ cudaError_t launch_typed(const Box &b, const StepConst &c, const Quant &q, const
     }
     for (int i = 0; i < 5; i++) P.mom[i] = v.mom + (size_t)i * b.n;
     P.err = v.err;
-    cudaError_t e = configure<ST, true, false, false, ZG>();
-    if (e == cudaSuccess) e = configure<ST, false, true, false, ZG>();
-    if (e == cudaSuccess) e = configure<ST, false, false, false, ZG>();
-    if (e == cudaSuccess) e = configure<ST, true, false, true, ZG>();
-    if (e == cudaSuccess) e = configure<ST, false, false, true, ZG>();
-    if (e == cudaSuccess) e = configure<ST, false, true, true, ZG>();
-    if (e != cudaSuccess) return e;
     // staging by TMA when the driver encodes every map the step needs: the g
     // tile (even steps) and the P_f planes (if enabled)
     CUtensorMap gmap, f0map, fqmap;
@@ -1365,24 +1406,33 @@ cudaError_t launch_typed(const Box &b, const StepConst &c, const Quant &q, const
     if (tma && use_tma_f<ST>()) tma = encode_f_maps<ST>(b, P.f0in, fin, &f0map, &fqmap);
     Box range = b;   // the chunk depth for the planes this launch covers
     range.nz = zhi - zlo;
-    const int tz = choose_tz<ST>(range);
+    const Plan plan = choose_plan<ST>(range);
+    const int tz = plan.tz;
     const int nchunks = (range.nz + tz - 1) / tz;
     const unsigned nblocks = (unsigned)((b.nx / TX) * (b.ny / TY) * nchunks);
     const dim3 block(TX / (use_pair<ST>() ? 2 : 1), TY, 1);
     const int wm = write_moments ? 1 : 0;
-    constexpr int smem = Geo<ST>::SMEM;
     const StepBox kb{b.nx, b.ny, b.nz, b.nxy, b.n};
-    auto go = [&](auto kernel) {
-        return launch_step_kernel(kernel, nblocks, block, smem, s, P, kb, c, m, tz, wm, zlo, zhi, gmap, f0map,
-                                  fqmap);
+    auto launch = [&](auto deep, auto streamed, auto is_odd, auto with_tma) -> cudaError_t {
+        constexpr bool D = decltype(deep)::value, S = decltype(streamed)::value, O = decltype(is_odd)::value,
+                       T = decltype(with_tma)::value;
+        const cudaError_t e = configure<ST, D, S, O, T, ZG>();
+        if (e != cudaSuccess) return e;
+        return launch_step_kernel(zsc_step_kernel<ST, D, S, O, T, ZG>, nblocks, block, Geo<ST, D>::SMEM, s, P, kb, c,
+                                  m, tz, wm, zlo, zhi, gmap, f0map, fqmap);
     };
-    if (f_streamed) {
-        if (odd) return cudaErrorInvalidValue;  // the streamed initial state is always read by an even step
-        return tma ? go(zsc_step_kernel<ST, true, false, true, ZG>) : go(zsc_step_kernel<ST, true, false, false, ZG>);
-    }
-    if (odd)
-        return tma ? go(zsc_step_kernel<ST, false, true, true, ZG>) : go(zsc_step_kernel<ST, false, true, false, ZG>);
-    return tma ? go(zsc_step_kernel<ST, false, false, true, ZG>) : go(zsc_step_kernel<ST, false, false, false, ZG>);
+    using Yes = std::true_type;
+    using No = std::false_type;
+    auto with = [&](auto deep, auto with_tma) -> cudaError_t {
+        if (f_streamed) {
+            // the streamed initial state is always read by an even step
+            return odd ? cudaErrorInvalidValue : launch(deep, Yes{}, No{}, with_tma);
+        }
+        return odd ? launch(deep, No{}, Yes{}, with_tma) : launch(deep, No{}, No{}, with_tma);
+    };
+    if constexpr (sizeof(ST) == 4)
+        if (plan.deep) return tma ? with(Yes{}, Yes{}) : with(Yes{}, No{});
+    return tma ? with(No{}, Yes{}) : with(No{}, No{});
 }
 
 template <typename ST>
@@ -1394,6 +1444,17 @@ cudaError_t launch_typed(const Box &b, const StepConst &c, const Quant &q, const
 }
 
 }  // namespace
+
+int sm_count()
+{
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return std::max(1, n);
+    }();
+    return sms;
+}
 
 cudaError_t launch_wait_selftest(int *err, cudaStream_t s)
 {
