@@ -557,33 +557,20 @@ adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_co
         fy_b = cur.fy;
         cur = top;
 
-        // moments of the streamed g (16-bit: of the stored values; the shifts
-        // cancel in the momentum's opposite pairs)
-        float rh, m[3];
+        // moments of the streamed g, summed in direction order (as g_moments)
+        float rh = 0.f, m[3] = {0.f, 0.f, 0.f};
         {
             const ST *gs = rg + st * Gm::GSTAGE;
-            auto g = [&](int i) -> float {
+#pragma unroll
+            for (int i = 0; i < kQg; i++) {
                 const int sx = ODD ? -kCx(i) : 0;
                 const int cc = PAIR ? 2 * (sx > 0 ? 1 : sx < 0 ? 3 : 0) + (sx > 0 ? hf_r : sx < 0 ? hf_l : hf) : col(sx);
-                return Fmt<ST>::load(gs[i * TYA * Gm::GP + cc]);
-            };
-            rh = g(0);
-            m[0] = m[1] = m[2] = 0.f;
-#pragma unroll
-            for (int p = 1; p < kQg; p += 2) {    // opposite pairs
-                const float u = g(p), v = g(p + 1), d = u - v;
-                rh += u + v;
-                if (kCx(p)) m[0] += kCx(p) * d;
-                if (kCy(p)) m[1] += kCy(p) * d;
-                if (kCz(p)) m[2] += kCz(p) * d;
-            }
-            if constexpr (Fmt<ST>::kMapped) {
-                float shift = 0.f;
-#pragma unroll
-                for (int i = 0; i < kQg; i++) shift += q.g_shift[i];
-                rh = fmaf(rh, q.g_inv, shift);
-#pragma unroll
-                for (int d = 0; d < 3; d++) m[d] *= q.g_inv;
+                float gi = Fmt<ST>::load(gs[i * TYA * Gm::GP + cc]);
+                if constexpr (Fmt<ST>::kMapped) gi = gi * q.g_inv + q.g_shift[i];
+                rh += gi;
+                if (kCx(i)) m[0] += kCx(i) * gi;
+                if (kCy(i)) m[1] += kCy(i) * gi;
+                if (kCz(i)) m[2] += kCz(i) * gi;
             }
         }
         const float inv = 1.0f / rh;
