@@ -29,10 +29,11 @@
 // chunk of halo columns on each side.
 //
 // Memory pipeline: the global reads go through asynchronous copies into
-// shared-memory stages (L2-cached, no registers held while in flight):
-//   - the 19 g rows of the next plane (2 stages; odd steps stage one extra
-//     chunk per row so the +-x shifted reads stay 16-byte aligned),
-//   - the 7 P_f planes three planes ahead (4 stages),
+// shared-memory stages (L2-cached, no registers held while in flight; the
+// number of stages is Geo's):
+//   - the 19 g rows of the next plane (odd steps stage one extra chunk per row
+//     so the +-x shifted reads stay 16-byte aligned),
+//   - the 7 P_f planes two or three planes ahead,
 // so a block always has about one plane of the step's input in flight while it
 // computes the current plane.  The P_f planes (tile + ragged halo, periodic
 // wrap) and the odd step's shifted g rows are cp.async 16-byte chunks: warps
@@ -134,11 +135,10 @@ struct Dir {
 //   dense 1 g stage, 3 P_f planes (66 KB, 80 registers, three per SM): the next
 //         g rows follow once the current ones are in registers, and the third
 //         block covers the shorter flight.
-// FP32, deep -> dense: 256^3 610 -> 605 us a step, 128^3 84.3 -> 81.0, 160 x 104
-// x 93 65.5 -> 60.7; but 64^3 13.8 -> 14.7, 32^3 4.1 -> 4.5: choose_plan takes
-// one by the box.  (16-bit storage with one
-// g stage and five blocks of 96 registers spills and is slower: 256^3 346 ->
-// 400 us.)
+// FP32, deep -> dense: 256^3 610 -> 600 us a step, 128^3 82.9 -> 80.0, 160 x 104
+// x 93 64.4 -> 59.9; but 64^3 13.5 -> 14.6, 32^3 3.8 -> 4.2: choose_plan takes
+// one by the box.  (16-bit storage with one g stage and five blocks of 96
+// registers spills and is slower: 256^3 346 -> 400 us.)
 // g rows carry one extra chunk (an odd step's shifted rows need it on one side
 // only).
 template <typename ST, bool DEEP>
@@ -161,11 +161,12 @@ struct Geo {
     static constexpr int G_OFF = 0;
     static constexpr int F_OFF = NG * G_STAGE;
     static constexpr int PHI_OFF = F_OFF + NF * F_STAGE;
-    static constexpr int MBAR_OFF = PHI_OFF + NPHI * PHI_STAGE;   // mbarriers: 2 g stages, then NF P_f stages
-    static constexpr int SMEM = MBAR_OFF + 8 * (NG + NF);
+    static constexpr int MBAR_OFF = PHI_OFF + NPHI * PHI_STAGE;   // mbarriers: g stages, P_f stages, the first P_f plane
+    static constexpr int SMEM = MBAR_OFF + 8 * (NG + NF + 1);
     static constexpr int G_TMA_BYTES = kQg * TY * TX * (int)sizeof(ST);   // one plane's tile, 19 fields
     static constexpr int TPD = TY * CM;              // g issuer threads per direction
     static constexpr int D = (NT / 2) / TPD;         // directions per pass of the g issuers
+    static_assert(F_STAGE <= G_STAGE, "the first P_f plane fits a g stage");
     static_assert(G_STAGE % 16 == 0 && F_STAGE % 16 == 0 && F0_BYTES % 16 == 0, "16-byte aligned stages");
     static_assert(G_STAGE % 128 == 0 && G_TMA_BYTES <= G_STAGE, "TMA destinations: 128-byte aligned, inside a stage");
     static_assert(E + TX <= GW, "even-step rows staged from column E fit a g row");
@@ -442,7 +443,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
             return;
         }
         if (tid == 0) {
-            for (int k = 0; k < NG + NF; k++) mbar_init(&mbar[k], 1);
+            for (int k = 0; k < NG + NF + 1; k++) mbar_init(&mbar[k], 1);
             mbar_init_fence();
         }
         __syncthreads();
@@ -472,9 +473,13 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
     // columns left of the tile, tiles at the right seam right of it.
     const bool seam_l = x0 == 0, seam_r = x0 + TX == b.nx;
 
-    // P_f stage of plane p (p >= z0 - 2): planes z0 - 2 + m go to stage m % NF
-    // for their (m / NF)-th use; f_0 part and f_1..f_6 part
-    auto fslot = [&](int p) { return (unsigned)(p - z0 + 2) % (unsigned)NF; };
+    // P_f stage of plane p (p >= z0 - 1): planes z0 - 1 + m go to stage m % NF
+    // for their (m / NF)-th use; f_0 part and f_1..f_6 part.  Plane z0 - 2, read
+    // by the first build only, is staged in the last g stage, which g needs
+    // after that build: so all the planes of the first builds are in flight
+    // together.
+    unsigned char *const f_first = smem + Gm::G_OFF + (NG - 1) * Gm::G_STAGE;
+    auto fslot = [&](int p) { return (unsigned)(p - z0 + 1) % (unsigned)NF; };
     auto fstage = [&](int p) { return F + fslot(p) * Gm::F_STAGE; };
     auto f0part = [&](unsigned char *st) { return reinterpret_cast<float *>(st); };
     auto fqpart = [&](unsigned char *st) { return reinterpret_cast<ST *>(st + Gm::F0_BYTES); };
@@ -513,25 +518,24 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
 
     // P_f stage p's mbarrier and the phase of plane p's use of it
     auto fbar = [&](int p) { return &mbar[NG + fslot(p)]; };
-    auto fphase = [&](int p) { return ((unsigned)(p - z0 + 2) / (unsigned)NF) & 1u; };
+    auto fphase = [&](int p) { return ((unsigned)(p - z0 + 1) / (unsigned)NF) & 1u; };
+    uint64_t *const fbar_first = &mbar[NG + NF];   // plane z0 - 2
     // phi slot of plane p (planes z0 - 1 + m go to slot m % NPHI)
     auto pslot = [&](int p) { return (int)((unsigned)(p - z0 + 1) % (unsigned)NPHI); };
 
-    // Queue the 7 P_f planes of plane p (tile + halo) into its stage.
-    auto issue_f = [&](int p) {
+    // Queue the 7 P_f planes of plane p (tile + halo) into stage st.
+    auto issue_f_to = [&](int p, unsigned char *st, uint64_t *bar) {
         if (tile_tma_f) {
             if (tid == 32) {   // lane 0 of warp 1 (warp 0 issues the g copies)
-                unsigned char *st = fstage(p);
                 const int zp = zf(p);
                 fence_proxy_async();
-                mbar_expect_tx(fbar(p), (unsigned)Gm::F_STAGE);
-                tma_load_3d(f0part(st), &f0map, x0 - 4, y0 - 2, zp, fbar(p));
-                tma_load_4d(fqpart(st), &fqmap, x0 - E, y0 - 2, zp, 0, fbar(p));
+                mbar_expect_tx(bar, (unsigned)Gm::F_STAGE);
+                tma_load_3d(f0part(st), &f0map, x0 - 4, y0 - 2, zp, bar);
+                tma_load_4d(fqpart(st), &fqmap, x0 - E, y0 - 2, zp, 0, bar);
             }
             return;
         }
         const unsigned zb = (unsigned)zf(p) * (unsigned)b.nxy;
-        unsigned char *st = fstage(p);
         if (f0_issuer && in_field((long long)zb + f0_xy, 4, nf, P.err))
             cp_async16(f0part(st) + f0_dst, P.f0in + (zb + (unsigned)f0_xy));
         if (fq_issuer) {
@@ -542,6 +546,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
                 if (in_field(base, E, nf, P.err)) cp_async16(dst + a * FR * W, P.fin[a] + base);
         }
     };
+    auto issue_f = [&](int p) { issue_f_to(p, fstage(p), fbar(p)); };
 
     // Call f(Dir<i>) for the directions this g issuer owns (compile-time
     // direction numbers; the branch is uniform per warp).
@@ -605,9 +610,9 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
         }
     };
 
-    // Streamed D3Q7 values at ring-tile position (lx, ly) of plane p (f_1..f_6
-    // in stored units) and phi (src/update_phi.cu:42-43), from the staged planes.
-    auto phi_at = [&](int p, int lx, int ly, float(&f)[kQf]) -> float {
+    // Streamed D3Q7 values at ring-tile position (lx, ly) of plane p (S0: the
+    // stage of plane p - 1; f_1..f_6 in stored units) and phi (src/update_phi.cu:42-43), from the staged planes.
+    auto phi_at = [&](unsigned char *S0, int p, int lx, int ly, float(&f)[kQf]) -> float {
         const int row = ly + 1;
         const int c0 = lx + 3;          // f_0 column: x - (x0 - 4)
         const int cq = lx - 1 + E;      // f_1..f_6 column: x - (x0 - E)
@@ -624,7 +629,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
 #pragma unroll
             for (int a = 0; a < kQf - 1; a++) f[a + 1] = raw(S1, a, row, cq);
         } else {
-            unsigned char *S0 = fstage(p - 1), *S2 = fstage(p + 1);
+            unsigned char *S2 = fstage(p + 1);
             f[1] = blend(S1, 0, row, cq - 1);
             f[2] = blend(S1, 1, row, cq + 1);
             f[3] = blend(S1, 2, row - 1, cq);
@@ -638,14 +643,14 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
 
     // phi of plane p on the tile + ring into phi slot s; the streamed f of the
     // thread's own node(s) is returned in fo.
-    auto build_plane = [&](int p, int s, float(&fo)[XPT][kQf]) {
+    auto build_plane = [&](unsigned char *S0, int p, int s, float(&fo)[XPT][kQf]) {
         float *ph = PHI + s * (RH * RW);
 #pragma unroll
         for (int k = 0; k < XPT; k++)
-            ph[(ty + 1) * RW + XPT * tx + k + 1] = phi_at(p, XPT * tx + k + 1, ty + 1, fo[k]);
+            ph[(ty + 1) * RW + XPT * tx + k + 1] = phi_at(S0, p, XPT * tx + k + 1, ty + 1, fo[k]);
         if (has_ring) {
             float tmp[kQf];
-            ph[rly * RW + rlx] = phi_at(p, rlx, rly, tmp);
+            ph[rly * RW + rlx] = phi_at(S0, p, rlx, rly, tmp);
         }
     };
 
@@ -678,7 +683,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
         const T2 v = reinterpret_cast<const T2 *>(fqpart(S))[(a * FR + rr) * (W / 2) + cw];
         return Fm::load2(Fm::perm2(v, sel));
     };
-    auto phi_pair = [&](int p, int lx, int ly, const Sel &sw, float2(&f)[kQf]) -> float2 {
+    auto phi_pair = [&](unsigned char *S0, int p, int lx, int ly, const Sel &sw, float2(&f)[kQf]) -> float2 {
         using namespace pk;
         const int row = ly + 1, c0 = lx + 1, cq = lx + 3;
         unsigned char *S1 = fstage(p);
@@ -688,7 +693,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
 #pragma unroll
             for (int a = 0; a < kQf - 1; a++) f[a + 1] = fq_word(S1, a, row, cq, sw.c);
         } else {
-            unsigned char *S0 = fstage(p - 1), *S2 = fstage(p + 1);
+            unsigned char *S2 = fstage(p + 1);
             // eta P(x - c) + (1 - eta) P(x), in stored units
             auto blend = [&](unsigned char *Su, int a, int ru, int cu, unsigned su) {
                 return fma(splat(c.eta), fq_word(Su, a, ru, cu, su), mul(splat(c.eta2), fq_word(S1, a, row, cq, sw.c)));
@@ -702,12 +707,12 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
         }
         return fma(splat(m.f_inv), add(add(add(add(add(f[1], f[2]), f[3]), f[4]), f[5]), f[6]), f[0]);
     };
-    auto build_pair = [&](int p, int s, float2(&fo)[kQf]) {
+    auto build_pair = [&](unsigned char *S0, int p, int s, float2(&fo)[kQf]) {
         float2 *ph = reinterpret_cast<float2 *>(PHI) + s * (RH * RWP);
-        ph[(ty + 1) * RWP + tx + 1] = phi_pair(p, tx + 1, ty + 1, sel_own, fo);
+        ph[(ty + 1) * RWP + tx + 1] = phi_pair(S0, p, tx + 1, ty + 1, sel_own, fo);
         if (has_ring) {
             float2 tmp[kQf];
-            ph[rly * RWP + rlx] = phi_pair(p, rlx, rly, sel_ring, tmp);
+            ph[rly * RWP + rlx] = phi_pair(S0, p, rlx, rly, sel_ring, tmp);
         }
     };
 
@@ -723,42 +728,41 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
     pdl_wait();   // the previous step's writes are complete and visible
     pdl_launch_dependents();
 
-    // prologue: P_f planes z0-2 .. z0+1 (with 3 stages: z0+1 after the first
-    // build), g of plane z0; phi of z0-1 and z0
-    issue_f(z0 - 2);
+    // prologue: P_f planes z0-2 .. z0+1 (4 stages: and z0+2) and, where
+    // another stage than plane z0-2's is there for it, g of plane z0; phi of z0-1
+    // and z0
+    issue_f_to(z0 - 2, f_first, fbar_first);
     issue_f(z0 - 1);
     issue_f(z0);
-    if constexpr (NF == 4) issue_f(z0 + 1);
-    issue_g(z0, 0);
+    issue_f(z0 + 1);
+    if constexpr (NF == 4) issue_f(z0 + 2);
+    if constexpr (NG == 2) issue_g(z0, 0);
     cp_async_commit();
     cp_async_wait_all();
     bool late = false;
     if (tile_tma_f) {
-        for (int p = z0 - 2; p <= z0 - 3 + NF; p++) late |= !mbar_wait(fbar(p), fphase(p));
+        late |= !mbar_wait(fbar_first, 0);
+        for (int p = z0 - 1; p <= z0 + 1; p++) late |= !mbar_wait(fbar(p), fphase(p));
     }
     __syncthreads();
     if constexpr (PAIR) {
         float2 tmp[kQf];
-        build_pair(z0 - 1, pslot(z0 - 1), tmp);
+        build_pair(f_first, z0 - 1, pslot(z0 - 1), tmp);
+        build_pair(fstage(z0 - 1), z0, pslot(z0), fcur2);
     } else {
         float tmp[XPT][kQf];
-        build_plane(z0 - 1, pslot(z0 - 1), tmp);
+        build_plane(f_first, z0 - 1, pslot(z0 - 1), tmp);
+        build_plane(fstage(z0 - 1), z0, pslot(z0), fcur);
     }
     if constexpr (NF == 3) {
-        // the stage of plane z0 - 2 is free once every thread has built z0 - 1
-        __syncthreads();
-        issue_f(z0 + 1);
+        __syncthreads();   // plane z0 - 1 is read (and plane z0 - 2)
+        issue_f(z0 + 2);
         cp_async_commit();
-        cp_async_wait_all();
-        if (tile_tma_f) late |= !mbar_wait(fbar(z0 + 1), fphase(z0 + 1));
-        __syncthreads();
     }
-    if constexpr (PAIR) build_pair(z0, pslot(z0), fcur2);
-    else build_plane(z0, pslot(z0), fcur);
-    __syncthreads();
-    issue_f(z0 + 2);
-    cp_async_commit();
-    if constexpr (NG == 1) cp_async_commit();   // (g of plane z0 has landed: its group is empty)
+    if constexpr (NG == 1) {
+        issue_g(z0, 0);
+        cp_async_commit();
+    }
 
     for (int j = 0; j < nzc; ++j) {
         const int z = z0 + j;
@@ -775,8 +779,8 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
         // P_f plane z + 2 is first read here (a late copy only spoils values:
         // the uniform exit below comes before anything is stored)
         if (tile_tma_f) late |= !mbar_wait(fbar(z + 2), fphase(z + 2));
-        if constexpr (PAIR) build_pair(z + 1, pslot(z + 1), fnext2);
-        else build_plane(z + 1, pslot(z + 1), fnext);
+        if constexpr (PAIR) build_pair(fstage(z), z + 1, pslot(z + 1), fnext2);
+        else build_plane(fstage(z), z + 1, pslot(z + 1), fnext);
         if constexpr (NG == 1) cp_async_wait_all();   // g of plane z (cp.async tiles)
         if constexpr (TMA) {
             // g of plane z: stage j % NG, its (j / NG)-th use (cp.async tiles
@@ -1302,15 +1306,16 @@ bool encode_f_maps(const Box &b, const float *f0, const ST *fq, CUtensorMap *f0m
 // FP32 takes the deep geometry below 16 tile-planes (32 x 8 nodes) per SM, the
 // dense one from there: below, blocks are alone or two on an SM and bound by
 // their own latencies.  Best of each over forced depths, deep / dense: 6.7
-// tile-planes per SM (64^3) 13.9 / 14.7 us, 12.6 (96 x 64 x 80) 21.0 / 21.1,
-// 22.7 (96^3) 35.0 / 34.5, 39.8 (160 x 104 x 93) 64.4 / 60.7.
+// tile-planes per SM (64^3) 13.5 / 14.6 us, 12.6 (96 x 64 x 80) 20.7 / 21.0,
+// 22.7 (96^3) 34.5 / 34.2, 53.9 (128^3) 79.9 / 79.9, 39.8 (160 x 104 x 93)
+// 64.4 / 59.9.
 //
 // The depth comes from march_depth, its constants fitted to forced depths
-// 1 .. 64 on nine boxes from 32^3 to 256^3: the choice is within 1.1% of the
-// best depth on average for the deep and the 16-bit kernels (6.4% at most) and
-// 0.3% for the dense one.  (Depth of at least 4 planes and a cost without the
-// share of an SM, before -> now: 32^3 FP32 8.2 -> 4.1 us, 32 x 64 x 48 FP32
-// 12.1 -> 6.8, FP16 16.0 -> 7.1; 64^3 FP16 16.9 -> 11.0; 192^3 FP16 171 -> 159.)
+// 1 .. 64 on nine boxes from 32^3 to 256^3: the choice is within 1.4% of the
+// best depth on average for the deep and the 16-bit kernels (5.9% at most) and
+// 0.03% for the dense one.  (Depth of at least 4 planes and a cost without the
+// share of an SM, before -> now: 32^3 FP32 8.2 -> 3.8 us, 32 x 64 x 48 FP32
+// 12.1 -> 6.6, FP16 16.0 -> 7.0; 64^3 FP16 16.9 -> 10.9; 192^3 FP16 171 -> 159.)
 struct Plan {
     bool deep;
     int tz;
