@@ -94,11 +94,13 @@ int create_context(lbm_ctx **out, const lbm_params *p, int zghost)
     c->partial_count = lbm::stats_partial_count(c->box);
     // the device buffers, 256-byte aligned pieces of one allocation (the TMA
     // tensor maps need 16-byte aligned field bases)
-    const size_t sizes[7] = {sizeof(float) * 2 * nf, c->esz * 2 * (lbm::kQf - 1) * nf, c->esz * lbm::kQg * ng,
-                             sizeof(float) * 5 * n, sizeof(double) * lbm::kStatsValues * c->partial_count,
-                             sizeof(double) * lbm::kStatsValues, sizeof(int)};
-    size_t offs[7], total = 0;
-    for (int k = 0; k < 7; k++) {
+    // the kernels' error flag follows the statistics' result: one copy reads both
+    constexpr int kPieces = 6;
+    const size_t sizes[kPieces] = {sizeof(float) * 2 * nf, c->esz * 2 * (lbm::kQf - 1) * nf, c->esz * lbm::kQg * ng,
+                                   sizeof(float) * 5 * n, sizeof(double) * lbm::kStatsValues * c->partial_count,
+                                   lbm::kReportBytes};
+    size_t offs[kPieces], total = 0;
+    for (int k = 0; k < kPieces; k++) {
         offs[k] = total;
         total += (sizes[k] + 255) & ~(size_t)255;
     }
@@ -112,9 +114,9 @@ int create_context(lbm_ctx **out, const lbm_params *p, int zghost)
         c->st.mom = reinterpret_cast<float *>(a + offs[3]);
         c->partials = reinterpret_cast<double *>(a + offs[4]);
         c->result = reinterpret_cast<double *>(a + offs[5]);
-        c->err = reinterpret_cast<int *>(a + offs[6]);
+        c->err = reinterpret_cast<int *>(c->result + lbm::kStatsValues);
     }
-    if (e == cudaSuccess) e = cudaMallocHost(&c->result_host, sizeof(double) * lbm::kStatsValues);
+    if (e == cudaSuccess) e = cudaMallocHost(&c->result_host, lbm::kReportBytes);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->err, 0, sizeof(int), c->stream);
     if (e != cudaSuccess) {
         lbm_destroy(c);
@@ -268,10 +270,17 @@ namespace lbm {
 // build found a global index outside its field (LBM_ECUDA).
 int device_error(lbm_ctx *c)
 {
-    int flag = 0;
     // on the context's stream, after the kernels that set it
-    LBM_CUDA(cudaMemcpyAsync(&flag, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "error flag");
+    LBM_CUDA(cudaMemcpyAsync(c->result_host + kStatsValues, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream),
+             "error flag");
     LBM_CUDA(cudaStreamSynchronize(c->stream), "error flag");
+    return flag_status(c);
+}
+
+int flag_status(const lbm_ctx *c)
+{
+    int flag = 0;
+    std::memcpy(&flag, c->result_host + kStatsValues, sizeof(int));
     if (flag & 4) return fail(LBM_ECUDA, "a checked build found a global index outside its field");
     if (flag & 2) return fail(LBM_ECUDA, "a step kernel's shared-memory stage was misaligned for TMA");
     if (flag) return fail(LBM_ETIMEOUT, "a step kernel timed out waiting for its staged data");
@@ -515,17 +524,18 @@ extern "C" int lbm_stats(lbm_ctx *c, lbm_stats_out *s, float *phi, float *rho, f
         cudaError_t e = lbm::launch_stats(c->box, c->d, c->st.mom, c->partials, c->partial_count, c->result,
                                           c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "stats kernel launch");
-        LBM_CUDA(cudaMemcpyAsync(c->result_host, c->result, sizeof(double) * lbm::kStatsValues,
-                                 cudaMemcpyDeviceToHost, c->stream),
-                 "stats copy");
     }
+    // the sums (meaningful with s only) and the error flag in one copy, one
+    // wait for everything: a 32^3 box's call took two copies and two waits
+    LBM_CUDA(cudaMemcpyAsync(c->result_host, c->result, lbm::kReportBytes, cudaMemcpyDeviceToHost, c->stream),
+             "stats copy");
     float *dst[5] = {phi, rho, ux, uy, uz};
     for (int a = 0; a < 5; a++)
         if (dst[a])
             LBM_CUDA(cudaMemcpyAsync(dst[a], c->st.mom + a * n, bytes, cudaMemcpyDeviceToHost, c->stream),
                      "field copy");
     LBM_CUDA(cudaStreamSynchronize(c->stream), "lbm_stats");
-    if (int rc = device_error(c)) return rc;
+    if (int rc = lbm::flag_status(c)) return rc;
     if (!s) return LBM_OK;
     return fill_stats(c, c->result_host, s);
 }

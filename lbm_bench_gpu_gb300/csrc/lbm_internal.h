@@ -216,6 +216,8 @@ cudaError_t launch_init_adjoint(const Box &b, const lbm_derived &d, float Gamma,
 
 // Number of doubles produced by launch_stats in `result`.
 constexpr int kStatsValues = 16;
+// Bytes of a context's report: those doubles and the kernels' error flag.
+constexpr size_t kReportBytes = sizeof(double) * kStatsValues + sizeof(int);
 
 }  // namespace lbm
 
@@ -230,9 +232,9 @@ struct lbm_ctx {
     size_t esz = 4;                // bytes per element of fq / g
     double *partials = nullptr;    // stats scratch: per-block partial sums
     size_t partial_count = 0;
-    double *result = nullptr;      // stats result (device)
-    double *result_host = nullptr; // pinned copy
-    int *err = nullptr;            // device error flag of the kernels (0 = none)
+    double *result = nullptr;      // the report: stats result (device) ...
+    int *err = nullptr;            // ... and behind it the error flag of the kernels (0 = none)
+    double *result_host = nullptr; // pinned copy of the report
     // one device allocation holding st.f0, st.fq, st.g, st.mom, partials,
     // result and err (one cudaMalloc per context instead of seven)
     void *arena = nullptr;
@@ -283,8 +285,10 @@ int fail(int code, const std::string &msg);
 int cuda_fail(cudaError_t e, const char *what);
 // Allocate a context (zghost: a z-slab with ghost planes, lbm_split_z).
 int create_context(lbm_ctx **out, const lbm_params *p, int zghost);
-// The kernels' error flag as a status (LBM_ETIMEOUT, LBM_ECUDA) after a sync.
+// The kernels' error flag as a status (LBM_ETIMEOUT, LBM_ECUDA) after a sync,
+// and the status of the flag a copy of the report has brought to the host.
 int device_error(lbm_ctx *c);
+int flag_status(const lbm_ctx *c);
 // lbm_stats_out from the raw statistics of a box of n nodes.
 int fill_stats_raw(double n, const lbm_params &p, long long steps, const double *raw, lbm_stats_out *s);
 
