@@ -190,26 +190,67 @@ __device__ __forceinline__ double block_sum(double v, double *red)
 
 __device__ __forceinline__ unsigned block_id() { return blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z); }
 
-// phi = sum of the streamed f of a native state.
-template <typename ST>
-__global__ void __launch_bounds__(NTA) adjoint_phi_kernel(Box b, float eta, Quant q, const float *__restrict__ f0,
-                                                          const FQFields fq, int f_streamed,
-                                                          float *__restrict__ phi)
+// phi = sum of the streamed f of a native state (FP32 storage).
+__global__ void __launch_bounds__(NTA) adjoint_phi_kernel(Box b, float eta, const float *__restrict__ f0,
+                                                          const FQFields fq, int f_streamed, float *__restrict__ phi)
 {
     const float eta2 = 1.f - eta;
     const int x = blockIdx.x * TXA + threadIdx.x, y = blockIdx.y * TYA + threadIdx.y;
     for (int z = blockIdx.z * kPlanes, z_end = min(b.nz, z + kPlanes); z < z_end; z++) {
-        const Nb p = state_neighbourhood<ST>(b, x, y, z);
-        const unsigned ts = p.at(0, 0, 0);
-        float s = f0[ts];
+        const Nb p = neighbourhood(b, x, y, z);
+        const unsigned t = p.at(0, 0, 0);
+        float s = f0[t];
 #pragma unroll
         for (int i = 1; i < kQf; i++) {
-            const ST *a = static_cast<const ST *>(fq.f[i - 1]);
-            const float inv = Fmt<ST>::kMapped ? q.f_inv : 1.f;
-            const float here = Fmt<ST>::load(a[ts]) * inv;
-            s += f_streamed ? here : eta * (Fmt<ST>::load(a[dir_at(p, i, -1)]) * inv) + eta2 * here;
+            const float *a = static_cast<const float *>(fq.f[i - 1]);
+            const float here = a[t];
+            s += f_streamed ? here : eta * a[dir_at(p, i, -1)] + eta2 * here;
         }
-        phi[node_index_of(b, x, y, z)] = s;
+        phi[t] = s;
+    }
+}
+
+// The same for 16-bit storage: a thread sums the two nodes of one pair-layout
+// word, so that every load is a whole word (with two-byte loads, 256^3 took 87
+// us; the 20 bytes a node take 49 at the copy bandwidth).
+template <typename ST>
+__global__ void __launch_bounds__(TXA / 2 * TYA) adjoint_phi_pair_kernel(Box b, float eta, float inv,
+                                                                         const float *__restrict__ f0,
+                                                                         const FQFields fq, int f_streamed,
+                                                                         float *__restrict__ phi)
+{
+    using T2 = typename Fmt<ST>::T2;
+    const float eta2 = 1.f - eta;
+    const int h = b.nx / 2, w = blockIdx.x * (TXA / 2) + threadIdx.x, y = blockIdx.y * TYA + threadIdx.y;
+    // the words at x - 1 and x + 1; past the x seam a word's nodes are swapped
+    const int wl = w == 0 ? h - 1 : w - 1, wr = w == h - 1 ? 0 : w + 1;
+    const unsigned sel_l = w == 0 ? kSwap : kKeep, sel_r = w == h - 1 ? kSwap : kKeep;
+    const int yl = y == 0 ? b.ny - 1 : y - 1, yr = y == b.ny - 1 ? 0 : y + 1;
+    for (int z = blockIdx.z * kPlanes, z_end = min(b.nz, z + kPlanes); z < z_end; z++) {
+        const int zl = z == 0 ? b.nz - 1 : z - 1, zr = z == b.nz - 1 ? 0 : z + 1;
+        auto word = [&](int ww, int yy, int zz) { return (unsigned)ww + (unsigned)h * ((unsigned)yy + (unsigned)b.ny * (unsigned)zz); };
+        const unsigned t = word(w, y, z);
+        // where the streamed f_i comes from: x - c_i
+        const unsigned up[kQf - 1] = {word(wl, y, z), word(wr, y, z), word(w, yl, z),
+                                      word(w, yr, z), word(w, y, zl), word(w, y, zr)};
+        float2 s = reinterpret_cast<const float2 *>(f0)[t];
+#pragma unroll
+        for (int i = 0; i < kQf - 1; i++) {
+            const T2 *a = static_cast<const T2 *>(fq.f[i]);
+            const float2 c = Fmt<ST>::load2(a[t]);
+            const float hx = c.x * inv, hy = c.y * inv;
+            if (f_streamed) {
+                s.x += hx;
+                s.y += hy;
+            } else {
+                const float2 v = Fmt<ST>::load2(Fmt<ST>::perm2(a[up[i]], i == 0 ? sel_l : i == 1 ? sel_r : kKeep));
+                s.x += eta * (v.x * inv) + eta2 * hx;
+                s.y += eta * (v.y * inv) + eta2 * hy;
+            }
+        }
+        const unsigned r = (unsigned)b.nx * ((unsigned)y + (unsigned)b.ny * (unsigned)z) + (unsigned)w;
+        phi[r] = s.x;
+        phi[r + (unsigned)h] = s.y;
     }
 }
 
@@ -733,13 +774,14 @@ struct StencilGeo {
     static constexpr int FIELD = P * ROWS, PLANE = 4 * FIELD;
     static constexpr int CHUNKS = PLANE / 4;               // 16-byte chunks of a plane
     static constexpr int PER = (CHUNKS + NTA - 1) / NTA;   // per thread
+    static constexpr int STAGES = 4;
 };
 
 __global__ void __launch_bounds__(NTA, kStencilBlocks)
 adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict__ lphi, int tz)
 {
     using G = StencilGeo;
-    __shared__ __align__(16) float sm[2][G::PLANE];
+    __shared__ __align__(16) float sm[G::STAGES][G::PLANE];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TXA + tx;
     const int ntx = b.nx / TXA, nty = b.ny / TYA;
     const int bx = blockIdx.x % ntx, by = (blockIdx.x / ntx) % nty, bz = blockIdx.x / (ntx * nty);
@@ -784,29 +826,28 @@ adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict_
         p.above = side + sz * kInv12;
         return p;
     };
-    // plane p is staged in stage (p - z0 + 1) & 1
-    issue(z0 - 1, 0);
-    cp_async_commit();
-    issue(z0, 1);
-    cp_async_commit();
+    // plane z0 - 1 + m is staged in stage m % STAGES, two planes ahead of its use
+    auto at = [&](int m) { return (int)((unsigned)m % (unsigned)G::STAGES); };
+#pragma unroll
+    for (int m = 0; m < 3; m++) {
+        issue(z0 - 1 + m, at(m));
+        cp_async_commit();
+    }
+    cp_async_wait_prior<2>();
+    __syncthreads();
+    float from_below = part(at(0)).above;   // what plane z0 - 1 adds to plane z0
     cp_async_wait_prior<1>();
     __syncthreads();
-    float from_below = part(0).above;   // what plane z0 - 1 adds to plane z0
-    __syncthreads();
-    issue(z0 + 1, 0);
-    cp_async_commit();
-    cp_async_wait_prior<1>();
-    __syncthreads();
-    Part cur = part(1);
+    Part cur = part(at(1));
     unsigned t = (unsigned)z0 * nxy + (unsigned)((y0 + ty) * b.nx + x0 + tx);
     for (int j = 0; j < nzc; ++j, t += nxy) {
         const float base = lphi[t];
-        __syncthreads();   // plane z is read: its stage takes plane z + 2
-        if (j + 1 < nzc) issue(z0 + j + 2, (j + 3) & 1);
+        // plane z + 2 takes the stage of plane z - 2, read before the last barrier
+        if (j + 1 < nzc) issue(z0 + j + 2, at(j + 3));
         cp_async_commit();
         cp_async_wait_prior<1>();
         __syncthreads();   // plane z + 1 has landed
-        const Part top = part((j + 2) & 1);
+        const Part top = part(at(j + 2));
         lphi[t] = base + ((cur.own + top.below) + from_below);
         from_below = cur.above;
         cur = top;
@@ -847,7 +888,9 @@ __global__ void __launch_bounds__(NTA) init_adjoint_kernel(Box b, float alpha4, 
         float lfs = 6.f * add, lga = 0.f, lgd = 0.f;
         if (lq)
             for (int i = 1; i < kQf; i++) lfs += lq[i * n + t];
+#pragma unroll
         for (int i = 1; i < 7; i++) lga += lg[i * n + t];
+#pragma unroll
         for (int i = 7; i < kQg; i++) lgd += lg[i * n + t];
         const float lg0 = lg[t];
         const float lmu = -3.f * Gamma * l0 + 0.5f * Gamma * lfs - 6.f * kW0 * ph * lg0 + 3.f * kW1 * ph * lga
@@ -940,14 +983,23 @@ size_t adjoint_blocks(const Box &b) { return blocks_of(adjoint_grid(b)); }
 cudaError_t launch_adjoint_phi(const Box &b, float eta, const Quant &q, const NativeState &st, float *phi,
                                cudaStream_t s)
 {
-    NativeState even = st;
-    even.g_odd = false;   // phi does not read g
-    return dispatch(even, [&](auto tag, auto) {
-        using ST = decltype(tag);
-        adjoint_phi_kernel<ST><<<adjoint_grid(b), kBlock, 0, s>>>(b, eta, q, st.f0, fq_fields(b, st),
-                                                                 st.f_streamed ? 1 : 0, phi);
-        return cudaGetLastError();
-    });
+    const int streamed = st.f_streamed ? 1 : 0;
+    const dim3 pair(TXA / 2, TYA);
+    switch (st.storage) {
+    case LBM_STORAGE_FP32:
+        adjoint_phi_kernel<<<adjoint_grid(b), kBlock, 0, s>>>(b, eta, st.f0, fq_fields(b, st), streamed, phi);
+        break;
+    case LBM_STORAGE_FP16:
+        adjoint_phi_pair_kernel<__half><<<adjoint_grid(b), pair, 0, s>>>(b, eta, q.f_inv, st.f0, fq_fields(b, st),
+                                                                         streamed, phi);
+        break;
+    case LBM_STORAGE_BF16:
+        adjoint_phi_pair_kernel<__nv_bfloat16><<<adjoint_grid(b), pair, 0, s>>>(b, eta, q.f_inv, st.f0,
+                                                                                fq_fields(b, st), streamed, phi);
+        break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t launch_objective(const Box &b, int objective, float phiStar, double scale, const Quant &q,
