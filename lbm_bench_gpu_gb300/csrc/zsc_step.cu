@@ -1303,19 +1303,20 @@ bool encode_f_maps(const Box &b, const float *f0, const ST *fq, CUtensorMap *f0m
 
 // Staging geometry and planes per block of a launch.
 //
-// FP32 takes the deep geometry below 16 tile-planes (32 x 8 nodes) per SM, the
-// dense one from there: below, blocks are alone or two on an SM and bound by
-// their own latencies.  Best of each over forced depths, deep / dense: 6.7
-// tile-planes per SM (64^3) 13.5 / 14.6 us, 12.6 (96 x 64 x 80) 20.7 / 21.0,
-// 22.7 (96^3) 34.5 / 34.2, 53.9 (128^3) 79.9 / 79.9, 39.8 (160 x 104 x 93)
-// 64.4 / 59.9.
+// The depth comes from march_depth.  Its constants were fitted to forced depths
+// 1 .. 64 on 24 boxes from 32^3 to 256^3, 15 of them drawn at random: the depth
+// taken is within 0.4% of the best on average (4.0% at most) for the 16-bit
+// kernel, 0.2% (2.1%) for the dense one and 0.6% (7.5%) for the deep one.
 //
-// The depth comes from march_depth, its constants fitted to forced depths
-// 1 .. 64 on nine boxes from 32^3 to 256^3: the choice is within 1.4% of the
-// best depth on average for the deep and the 16-bit kernels (5.9% at most) and
-// 0.03% for the dense one.  (Depth of at least 4 planes and a cost without the
-// share of an SM, before -> now: 32^3 FP32 8.2 -> 3.8 us, 32 x 64 x 48 FP32
-// 12.1 -> 6.6, FP16 16.0 -> 7.0; 64^3 FP16 16.9 -> 10.9; 192^3 FP16 171 -> 159.)
+// FP32 takes the geometry with the lower estimate: on each of the 17 boxes of
+// up to 1.2 million nodes the faster one of the two at their depths.  Deep /
+// dense in us: 64^3 13.4 / 14.5, 128 x 64 x 44 15.8 / 17.6, 96 x 64 x 80 20.6 /
+// 20.8; 32 x 96 x 110 14.6 / 13.5, 128 x 112 x 37 22.6 / 20.9, 96 x 88 x 100
+// 33.6 / 32.7.  Larger boxes take the dense one.
+//
+// (Depth of at least 4 planes and a cost without the share of an SM, before ->
+// now: 32^3 FP32 8.2 -> 3.8 us, 32 x 64 x 48 FP32 12.1 -> 6.6, FP16 16.0 -> 6.7;
+// 64^3 FP16 16.9 -> 10.9; 160 x 104 x 93 FP16 41.8 -> 38.3; 192^3 FP16 171 -> 159.)
 struct Plan {
     bool deep;
     int tz;
@@ -1344,13 +1345,16 @@ Plan choose_plan(const Box &b)
     const long long tiles = (long long)(b.nx / TX) * (b.ny / TY);
     const int sms = sm_count();
     if constexpr (sizeof(ST) == 2) {
-        constexpr MarchCost cost = {1.25, 0.88, {0.0, 1.0, 1.43, 1.90, 2.28}};
-        plan.tz = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), cost);
+        constexpr MarchCost cost = {1.45, {0.0, 1.0, 1.33, 1.97, 2.10}, {0.30, 0.79, 1.22, 1.62, 1.77}};
+        plan.tz = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), cost).tz;
     } else {
-        constexpr MarchCost deep = {1.25, 0.88, {0.0, 1.0, 1.40}}, dense = {3.0, 0.84, {0.0, 1.0, 1.60, 1.71}};
-        plan.deep = tiles * b.nz < 16LL * sms;
-        plan.tz = plan.deep ? march_depth(tiles, b.nz, sms, resident_blocks<ST, true>(), deep)
-                            : march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), dense);
+        constexpr MarchCost deep = {1.16, {0.0, 1.0, 1.50}, {0.30, 0.97, 1.54}};
+        constexpr MarchCost dense = {3.28, {0.0, 1.0, 1.53, 1.71}, {0.91, 1.39, 1.51, 1.56}};
+        const Depth d = march_depth(tiles, b.nz, sms, resident_blocks<ST, true>(), deep);
+        const Depth e = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), dense);
+        // the two costs in one unit
+        plan.deep = d.cost <= 0.9 * e.cost - 0.5;
+        plan.tz = plan.deep ? d.tz : e.tz;
     }
     last[0] = b.nx;
     last[1] = b.ny;
