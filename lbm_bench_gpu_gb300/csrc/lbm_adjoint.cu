@@ -119,7 +119,6 @@ struct Adjoint {
     // lambda: L, the 19 lg and, when tauPhi is not 1, the seven q (AdjointBuffers)
     float *lam_L[2] = {nullptr, nullptr}, *lam_g[2] = {nullptr, nullptr}, *lam_q[2] = {nullptr, nullptr};
     float *lsrc = nullptr;        // 4 x n
-    float *phi0 = nullptr, *mom_save = nullptr;
     double *partials = nullptr, *dgrav = nullptr, *ab = nullptr, *acc = nullptr;
     unsigned char *slots = nullptr;   // the context's checkpoint pool
     std::vector<Snapshot> snaps;
@@ -249,7 +248,8 @@ struct Adjoint {
     {
         if (nsteps <= 0) return LBM_OK;
         fwd_steps += nsteps;
-        return lbm_step(c, (int)nsteps, o.grav);
+        // (the context's phi, rho, u fields stay those of its initial state)
+        return lbm::queue_steps(c, (int)nsteps, o.grav, false);
     }
 
     // One step of the state src (at step `step`) with its output in the
@@ -542,11 +542,10 @@ struct Adjoint {
     }
 
     // the work buffers, carved from the context's arena; the objective alone
-    // needs only phi, mom_save and the sums
+    // needs only phi and the sums
     void carve(Carver &w, bool gradient, size_t nblocks)
     {
         phi = w.take<float>(2 * n);
-        mom_save = w.take<float>(5 * n);
         partials = w.take<double>(2 * nblocks);
         ab = w.take<double>(8);
         acc = w.take<double>(2);
@@ -557,7 +556,6 @@ struct Adjoint {
             if (k.invTauPhiOne != 0.f) lam_q[i] = w.take<float>((size_t)lbm::kQf * n);
         }
         lsrc = w.take<float>(4 * n);
-        phi0 = w.take<float>(n);
         dgrav = w.take<double>(lbm::adjoint_dgrav_parts(c->box));
     }
 };
@@ -653,15 +651,12 @@ extern "C" int lbm_objective(lbm_ctx *c, const lbm_adjoint_opts *o, double *J)
     LBM_ON_DEVICE(c->p.device);
     Adjoint A;
     setup(A, c, o);
-    const size_t n = A.n;
     if ((rc = workspace(c, A, false, "lbm_objective: work buffers")) ||
         (rc = ensure(c->adj_slots, c->adj_slot_bytes, A.snap_bytes, "lbm_objective: snapshot")))
         return rc;
     A.slots = static_cast<unsigned char *>(c->adj_slots);
     A.snaps.assign(1, Snapshot());
     cudaError_t e = cudaMemsetAsync(A.acc, 0, sizeof(double) * 2, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(A.mom_save, c->st.mom, sizeof(float) * 5 * n, cudaMemcpyDeviceToDevice, c->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "lbm_objective: setup");
     if (!rc) rc = A.save(0, 0);
     if (!rc) rc = A.forward(A.first_source);
@@ -679,8 +674,6 @@ extern "C" int lbm_objective(lbm_ctx *c, const lbm_adjoint_opts *o, double *J)
     if (!rc) {
         e = cudaMemcpyAsync(acc, A.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) rc = A.restore(0);
-        if (e == cudaSuccess && !rc)
-            e = cudaMemcpyAsync(c->st.mom, A.mom_save, sizeof(float) * 5 * n, cudaMemcpyDeviceToDevice, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess && !rc) rc = cuda_fail(e, "lbm_objective: results");
     }
@@ -749,9 +742,6 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
     e = cudaMemsetAsync(A.acc, 0, sizeof(double) * 2, c->stream);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(A.dgrav, 0, sizeof(double) * lbm::adjoint_dgrav_parts(c->box), c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(A.phi0, c->st.mom, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(A.mom_save, c->st.mom, sizeof(float) * 5 * n, cudaMemcpyDeviceToDevice, c->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "lbm_step_adjoint: setup");
     if (!rc) rc = A.create_streams((int)nslots);
     if (!rc) rc = A.save(0, 0);
@@ -762,7 +752,7 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
     if (!rc) {
         e = lbm::launch_dgrav_fold(c->box, A.dgrav, A.acc, c->stream);
         if (e == cudaSuccess)
-            e = lbm::launch_init_adjoint(c->box, c->d, c->p.Gamma, A.phi0, A.lam_q[A.cur], A.lam_L[A.cur],
+            e = lbm::launch_init_adjoint(c->box, c->d, c->p.Gamma, c->st.mom, A.lam_q[A.cur], A.lam_L[A.cur],
                                          A.lam_g[A.cur], lphi0, A.phi, c->stream);
         if (e != cudaSuccess) rc = cuda_fail(e, "lbm_step_adjoint: initial-state adjoint");
     }
@@ -772,10 +762,8 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
         e = cudaMemcpyAsync(acc, A.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess && out->dJ_dphi0)
             e = cudaMemcpyAsync(out->dJ_dphi0, lphi0, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream);
-        // leave the context at its initial state with its initial fields
+        // leave the context at its initial state (its fields were not touched)
         if (e == cudaSuccess) rc = A.restore(0);
-        if (e == cudaSuccess && !rc)
-            e = cudaMemcpyAsync(c->st.mom, A.mom_save, sizeof(float) * 5 * n, cudaMemcpyDeviceToDevice, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess && !rc) rc = cuda_fail(e, "lbm_step_adjoint: results");
     }

@@ -491,6 +491,24 @@ extern "C" int lbm_slab_init_bubbles(lbm_ctx **out, const lbm_params *p, const f
     return LBM_OK;
 }
 
+namespace lbm {
+int queue_steps(lbm_ctx *c, int nsteps, float grav, bool moments)
+{
+    const StepConst k = step_const(c->d, c->p, grav);
+    for (int s = 0; s < nsteps; s++) {
+        const int in = c->st.f_cur;
+        cudaError_t e = launch_step(c->box, k, c->q, view(c, in), c->st.f_streamed, c->st.g_odd_next,
+                                    moments && s == nsteps - 1, c->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
+        c->st.f_cur = 1 - in;
+        c->st.f_streamed = false;
+        c->st.g_odd_next = !c->st.g_odd_next;
+        c->st.steps++;
+    }
+    return LBM_OK;
+}
+}  // namespace lbm
+
 extern "C" int lbm_step(lbm_ctx *c, int nsteps, float grav)
 {
     const lbm::Range nvtx_range("lbm_step");
@@ -499,18 +517,7 @@ extern "C" int lbm_step(lbm_ctx *c, int nsteps, float grav)
     if (!std::isfinite(grav)) return fail(LBM_EINVAL, "grav is not finite");
     if (c->box.zghost) return fail(LBM_EINVAL, "lbm_step: a z-slab steps with lbm_slab_step / lbm_slab_step_local");
     LBM_ON_DEVICE(c->p.device);
-    const lbm::StepConst k = lbm::step_const(c->d, c->p, grav);
-    for (int s = 0; s < nsteps; s++) {
-        const int in = c->st.f_cur;
-        cudaError_t e = lbm::launch_step(c->box, k, c->q, view(c, in), c->st.f_streamed, c->st.g_odd_next,
-                                         s == nsteps - 1, c->stream);
-        if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
-        c->st.f_cur = 1 - in;
-        c->st.f_streamed = false;
-        c->st.g_odd_next = !c->st.g_odd_next;
-        c->st.steps++;
-    }
-    return LBM_OK;
+    return lbm::queue_steps(c, nsteps, grav, true);
 }
 
 extern "C" int lbm_stats(lbm_ctx *c, lbm_stats_out *s, float *phi, float *rho, float *ux, float *uy, float *uz)

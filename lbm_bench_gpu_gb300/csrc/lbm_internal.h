@@ -292,6 +292,9 @@ int fail(int code, const std::string &msg);
 int cuda_fail(cudaError_t e, const char *what);
 // Allocate a context (zghost: a z-slab with ghost planes, lbm_split_z).
 int create_context(lbm_ctx **out, const lbm_params *p, int zghost);
+// Queue nsteps >= 0 steps of a whole-box context, whose device is current;
+// moments: the last one writes the phi, rho, u fields.
+int queue_steps(lbm_ctx *c, int nsteps, float grav, bool moments);
 // The kernels' error flag as a status (LBM_ETIMEOUT, LBM_ECUDA) after a sync,
 // and the status of the flag a copy of the report has brought to the host.
 int device_error(lbm_ctx *c);
