@@ -22,8 +22,8 @@ namespace lbm {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int SX = 32, SY = kThreads / 32;   // columns of a block's tile
-constexpr int kBlocksPerSm = 3;              // resident blocks the launch bounds ask for (80 registers)
+constexpr int SX = 32, SY = 2 * kThreads / 32;   // columns of a block's tile (two rows a thread)
+constexpr int kBlocksPerSm = 2;              // resident blocks the launch bounds ask for (128 registers)
 constexpr int kMaxBlocks = 152 * kBlocksPerSm;
 constexpr float kInv6 = 0.16666666666666666667f;
 constexpr float kInv12 = 0.08333333333333333333f;
@@ -80,25 +80,27 @@ struct Plane {
     float mid, gx, gy;        // e4 + 2 f4 - 24 c; own-plane parts of the x and y gradient
 };
 
-// One block: eight warps, a 32 x 8 tile of columns; item `it` is one tile and
-// a run of kz planes, which every thread marches at its column.  Plane z + 2
-// of phi and plane z + 1 of the other fields are loaded while plane z is
-// computed.  |u|^2 and the pressure are evaluated in float as the reference
-// does (src/stats.c:45, src/logsave.c:94-137); sums are compensated, counts
-// exact.  phi_lo / phi_hi: the phi planes just below and above a z-slab (NULL
-// for a periodic box, whose z neighbours wrap).  The pressure is summed over
-// the reference's region only, so x and y need no wrap.
+// One block: eight warps, a 32 x 16 tile of columns; item `it` is one tile and
+// a run of kz planes, which every thread marches at its two columns (rows y and
+// y + 1, which share 6 of the 18 values of phi they need).  Plane z + 2 of phi
+// and plane z + 1 of the other fields are loaded while plane z is computed.
+// |u|^2 and the pressure are evaluated in float as the reference does
+// (src/stats.c:45, src/logsave.c:94-137); sums are compensated, counts exact.
+// phi_lo / phi_hi: the phi planes just below and above a z-slab (NULL for a
+// periodic box, whose z neighbours wrap).  The pressure is summed over the
+// reference's region only, so x and y need no wrap.
 //
 // Bound by instruction issue: the 20 bytes a node must be read take 49 us at
-// 256^3 at the copy bandwidth, the kernel's 223 instructions per node (100 of
-// them FP32, 51 in the compensated sums of a node outside the bubbles) 97 us
-// at one per cycle and scheduler; 72% of the cycles issue.  Measured, 256^3:
-// 351 -> 136 us, 32^3 with the fold 78 -> 12 us, against one thread per node reading 19
-// points, with 15 FP64 values per thread reduced over the block (FP64 runs at
-// a 60th of the FP32 rate: that reduction was most of a small box's time).
-// Two nodes a thread in f32x2 was slower (143 us: the packed operations issue
-// at half rate and their constants take register pairs); four resident blocks
-// (64 registers, spills) 175 us.
+// 256^3 at the copy bandwidth, its 100 FP32 instructions (51 of them in the
+// compensated sums of a node outside the bubbles) 45 us at one per cycle and
+// scheduler, of about 180 in all.  Measured, lbm_stats_noalloc with its fold,
+// 256^3: 368 -> 127 us, 128^3 36.9, 32^3 78 -> 12 us, against one thread per
+// node reading 19 points, with 15 FP64 values per thread reduced over the block
+// (FP64 runs at a 60th of the FP32 rate: that reduction was most of a small
+// box's time).  Also measured at 256^3: one column a thread 145 us (223
+// instructions a node), two nodes a thread in f32x2 147 (the packed operations
+// issue at half rate and their constants take register pairs), the planes
+// staged by cp.async 133.
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
 stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__restrict__ rho,
              const float *__restrict__ ux, const float *__restrict__ uy, const float *__restrict__ uz,
@@ -114,112 +116,125 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
 
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int tile = it % (ntx * nty), z0 = (it / (ntx * nty)) * kz;
-        const int x = (tile % ntx) * SX + lane, y = (tile / ntx) * SY + warp;
+        const int x = (tile % ntx) * SX + lane, y = (tile / ntx) * SY + 2 * warp;
         if (x >= b.nx || y >= b.ny) continue;   // (no barrier in this loop)
-        const bool region = x >= 1 && x <= b.nx - 2 && y >= 1 && y <= b.ny - 2;
-        const unsigned xy = (unsigned)y * nx + (unsigned)x;
+        const bool two = y + 1 < b.ny;          // the row y + 1 is in the box
+        const bool x_in = x >= 1 && x <= b.nx - 2;
+        const bool in_a = x_in && y >= 1 && y <= b.ny - 2, in_b = x_in && y + 1 <= b.ny - 2;
         const int n_z = min(kz, b.nz - z0);
+        // rows y - 1 .. y + 2, clamped to the box (a clamped row is not used)
+        const unsigned o0 = (unsigned)y * nx + (unsigned)x;
+        const unsigned om = y > 0 ? o0 - nx : o0, o1 = two ? o0 + nx : o0, o2 = y + 2 < b.ny ? o0 + 2 * nx : o0;
 
-        // phi around (x, y) on plane z (one past the box: its periodic or ghost neighbour)
-        float r[9];
+        // phi around the two nodes on plane z (one past the box: its periodic or ghost neighbour)
+        float c4[4], e4[4], w4[4];
         auto load_phi = [&](int z) {
             const float *p = phi;
-            unsigned t = xy;
+            unsigned t = 0;
             if (z < 0 && phi_lo) p = phi_lo;
             else if (z >= b.nz && phi_hi) p = phi_hi;
-            else t += (unsigned)(z < 0 ? b.nz - 1 : (z >= b.nz ? 0 : z)) * nxy;
-            const float *m = p + t;
-            r[0] = __ldg(m);
-            if (region) {
-                const float *n = p + (t + nx), *s = p + (t - nx);
-                r[1] = __ldg(m + 1);
-                r[2] = __ldg(m - 1);
-                r[3] = __ldg(n);
-                r[4] = __ldg(s);
-                r[5] = __ldg(n + 1);
-                r[6] = __ldg(s - 1);
-                r[7] = __ldg(s + 1);
-                r[8] = __ldg(n - 1);
+            else t = (unsigned)(z < 0 ? b.nz - 1 : (z >= b.nz ? 0 : z)) * nxy;
+            const float *const rows[4] = {p + (t + om), p + (t + o0), p + (t + o1), p + (t + o2)};
+#pragma unroll
+            for (int k = 0; k < 4; k++) c4[k] = __ldg(rows[k]);
+            if (x_in) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    e4[k] = __ldg(rows[k] + 1);
+                    w4[k] = __ldg(rows[k] - 1);
+                }
             }
         };
-        auto derive = [&]() -> Plane {
+        auto derive = [&](int k) -> Plane {   // of row k of the four
             Plane p;
-            p.c = r[0];
-            const float f4 = (r[1] + r[2]) + (r[3] + r[4]);
-            const float d1 = r[5] - r[6], d2 = r[7] - r[8];
-            p.fx = r[1] - r[2];
-            p.fy = r[3] - r[4];
-            p.a = fmaf(2.f, r[0], f4);
-            p.mid = fmaf(2.f, fmaf(-12.f, r[0], f4), (r[5] + r[6]) + (r[7] + r[8]));
+            const float f4 = (e4[k] + w4[k]) + (c4[k + 1] + c4[k - 1]);
+            const float d1 = e4[k + 1] - w4[k - 1], d2 = e4[k - 1] - w4[k + 1];
+            p.c = c4[k];
+            p.fx = e4[k] - w4[k];
+            p.fy = c4[k + 1] - c4[k - 1];
+            p.a = fmaf(2.f, p.c, f4);
+            p.mid = fmaf(2.f, fmaf(-12.f, p.c, f4), (e4[k + 1] + w4[k - 1]) + (e4[k - 1] + w4[k + 1]));
             p.gx = fmaf(2.f, p.fx, d1 + d2);
             p.gy = fmaf(2.f, p.fy, d1 - d2);
             return p;
         };
-        float f_rho, f_ux, f_uy, f_uz;
+        struct Fields {
+            float rho, ux, uy, uz;
+        };
+        Fields fa, fb;
         auto load_fields = [&](int z) {
-            const unsigned t = (unsigned)z * nxy + xy;
-            f_rho = __ldg(rho + t);
-            f_ux = __ldg(ux + t);
-            f_uy = __ldg(uy + t);
-            f_uz = __ldg(uz + t);
+            const unsigned ta = (unsigned)z * nxy + o0, tb = (unsigned)z * nxy + o1;
+            fa = Fields{__ldg(rho + ta), __ldg(ux + ta), __ldg(uy + ta), __ldg(uz + ta)};
+            fb = Fields{__ldg(rho + tb), __ldg(ux + tb), __ldg(uy + tb), __ldg(uz + tb)};
+        };
+        // one node: cur its plane, top and (a_b, fx_b, fy_b) the ones above and below
+        auto node = [&](const Plane &cur, const Plane &top, float a_b, float fx_b, float fy_b, const Fields &f,
+                        bool region) {
+            const float ph = cur.c;
+            // 0 * x summed over the fields is 0 if all are finite, else NaN
+            const float t =
+                fmaf(0.f, f.uz, fmaf(0.f, f.uy, fmaf(0.f, f.ux, fmaf(0.f, f.rho, __fmul_rn(0.f, ph)))));
+            if (t != 0.f) {   // NaN
+                cnt_bad++;
+                return;
+            }
+            const float u2 = fmaf(f.uz, f.uz, fmaf(f.uy, f.uy, f.ux * f.ux));
+            s_phi.add(ph);
+            s_rho.add(f.rho);
+            s_mx.add_product(f.rho, f.ux);
+            s_my.add_product(f.rho, f.uy);
+            s_mz.add_product(f.rho, f.uz);
+            const bool heavy = ph >= 0.f;
+            cnt_all += heavy;
+            umax_all = fmaxf(umax_all, u2);
+            if (!region) return;
+            umax_c = fmaxf(umax_c, u2);
+            const float lap = ((cur.mid + top.a) + a_b) * kInv6;
+            // 12 grad; z: 2 (ct - cb) + f4t - f4b, with a = f4 + 2 c
+            const float gx = cur.gx + (top.fx + fx_b), gy = cur.gy + (top.fy + fy_b), gz = top.a - a_b;
+            const float ph2 = ph * ph;
+            const float bulk = fmaf(ph2, fmaf(3.f, ph2, -2.f * c.phiStarSq), -c.phiStarSq * c.phiStarSq);
+            const float g2 = fmaf(gz, gz, fmaf(gy, gy, gx * gx));
+            const float surf = fmaf(-0.5f * kInv12 * kInv12, g2, ph * lap);
+            const float pres = fmaf(kCsSq, f.rho, fmaf(c.alpha, bulk, -c.kappa * surf));
+            if (heavy) {
+                cnt_in++;
+                s_ux.add(f.ux);
+                s_uy.add(f.uy);
+                s_uz.add(f.uz);
+                s_in.add(pres);
+            } else {
+                s_out.add(pres);
+            }
         };
 
 #pragma unroll
-        for (int k = 1; k < 9; k++) r[k] = 0.f;   // (outside the region: not used)
+        for (int k = 0; k < 4; k++) e4[k] = w4[k] = 0.f;   // (outside the region: not used)
         load_phi(z0 - 1);
-        const Plane below = derive();
-        float a_b = below.a, fx_b = below.fx, fy_b = below.fy;
+        Plane p = derive(1), q = derive(2);
+        float a_a = p.a, fx_a = p.fx, fy_a = p.fy, a_b = q.a, fx_b = q.fx, fy_b = q.fy;
         load_phi(z0);
-        Plane cur = derive();
+        Plane cur_a = derive(1), cur_b = derive(2);
         load_phi(z0 + 1);
         load_fields(z0);
+#pragma unroll 2
         for (int k = 0; k < n_z; k++) {
-            const Plane top = derive();
-            const float ph = cur.c, rh = f_rho, vx = f_ux, vy = f_uy, vz = f_uz;
+            const Plane top_a = derive(1), top_b = derive(2);
+            const Fields f0 = fa, f1 = fb;
             if (k + 1 < n_z) {
                 load_phi(z0 + k + 2);
                 load_fields(z0 + k + 1);
             }
-            // 0 * x summed over the fields is 0 if all are finite, else NaN
-            const float t =
-                fmaf(0.f, vz, fmaf(0.f, vy, fmaf(0.f, vx, fmaf(0.f, rh, __fmul_rn(0.f, ph)))));
-            if (t == 0.f) {
-                const float u2 = fmaf(vz, vz, fmaf(vy, vy, vx * vx));
-                s_phi.add(ph);
-                s_rho.add(rh);
-                s_mx.add_product(rh, vx);
-                s_my.add_product(rh, vy);
-                s_mz.add_product(rh, vz);
-                const bool heavy = ph >= 0.f;
-                cnt_all += heavy;
-                umax_all = fmaxf(umax_all, u2);
-                if (region) {
-                    umax_c = fmaxf(umax_c, u2);
-                    const float lap = ((cur.mid + top.a) + a_b) * kInv6;
-                    // 12 grad; z: 2 (ct - cb) + f4t - f4b, with a = f4 + 2 c
-                    const float gx = cur.gx + (top.fx + fx_b), gy = cur.gy + (top.fy + fy_b), gz = top.a - a_b;
-                    const float ph2 = ph * ph;
-                    const float bulk = fmaf(ph2, fmaf(3.f, ph2, -2.f * c.phiStarSq), -c.phiStarSq * c.phiStarSq);
-                    const float g2 = fmaf(gz, gz, fmaf(gy, gy, gx * gx));
-                    const float surf = fmaf(-0.5f * kInv12 * kInv12, g2, ph * lap);
-                    const float pres = fmaf(kCsSq, rh, fmaf(c.alpha, bulk, -c.kappa * surf));
-                    cnt_in += heavy;
-                    if (heavy) {
-                        s_ux.add(vx);
-                        s_uy.add(vy);
-                        s_uz.add(vz);
-                        s_in.add(pres);
-                    } else {
-                        s_out.add(pres);
-                    }
-                }
-            } else {
-                cnt_bad++;
-            }
-            a_b = cur.a;
-            fx_b = cur.fx;
-            fy_b = cur.fy;
-            cur = top;
+            node(cur_a, top_a, a_a, fx_a, fy_a, f0, in_a);
+            if (two) node(cur_b, top_b, a_b, fx_b, fy_b, f1, in_b);
+            a_a = cur_a.a;
+            fx_a = cur_a.fx;
+            fy_a = cur_a.fy;
+            a_b = cur_b.a;
+            fx_b = cur_b.fx;
+            fy_b = cur_b.fy;
+            cur_a = top_a;
+            cur_b = top_b;
         }
     }
 
