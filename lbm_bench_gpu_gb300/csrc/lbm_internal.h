@@ -119,9 +119,10 @@ struct AdjointBuffers {
 // are, then a last, partly filled one, which overlaps the end of the others:
 // x blocks per SM of it add tail[x] (interpolated; tail[0] is what the first of
 // them adds) of their time, which is that of the last, shorter run of planes
-// if there are no others among them.  The depth that minimises the sum is
-// taken; cost is in plane-times of a lone block.
+// if there are no others among them.  The depth up to `deepest` that minimises
+// the sum is taken; cost is in plane-times of a lone block.
 struct MarchCost {
+    int deepest;
     double prologue;
     double share[7], tail[7];
 };
@@ -133,7 +134,7 @@ inline Depth march_depth(long long tiles, int planes, int sms, int per_sm, const
 {
     const long long slots = (long long)sms * per_sm;
     Depth best = {1, -1.0};
-    for (int tz = 1; tz <= 64; tz++) {
+    for (int tz = 1; tz <= m.deepest; tz++) {
         const int runs = (planes + tz - 1) / tz, last = planes - (runs - 1) * tz;
         const long long blocks = tiles * runs, full = blocks / slots, rest = blocks % slots;
         double cost = (double)full * m.share[per_sm] * (tz + m.prologue);

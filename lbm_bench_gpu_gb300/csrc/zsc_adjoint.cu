@@ -927,7 +927,7 @@ struct March {
 };
 March march_of(const Box &b)
 {
-    constexpr MarchCost cost = {1.0, {0.0, 1.0, 1.4}, {0.88, 0.88, 1.23}};
+    constexpr MarchCost cost = {32, 1.0, {0.0, 1.0, 1.4}, {0.88, 0.88, 1.23}};
     const int tiles = (b.nx / TXA) * (b.ny / TYA);
     const int tz = march_depth(tiles, b.nz, sm_count(), 2, cost).tz;
     return March{tz, tiles * ((b.nz + tz - 1) / tz)};
@@ -935,7 +935,7 @@ March march_of(const Box &b)
 // The stencil kernel's: a prologue of two planes, kStencilBlocks blocks on an SM.
 March stencil_march(const Box &b)
 {
-    constexpr MarchCost cost = {2.0, {0.0, 1.0, 1.2, 1.5, 1.8, 2.2}, {0.88, 0.88, 1.06, 1.32, 1.58, 1.94}};
+    constexpr MarchCost cost = {32, 2.0, {0.0, 1.0, 1.2, 1.5, 1.8, 2.2}, {0.88, 0.88, 1.06, 1.32, 1.58, 1.94}};
     const int tiles = (b.nx / TXA) * (b.ny / TYA);
     const int tz = march_depth(tiles, b.nz, sm_count(), kStencilBlocks, cost).tz;
     return March{tz, tiles * ((b.nz + tz - 1) / tz)};

@@ -1304,9 +1304,12 @@ bool encode_f_maps(const Box &b, const float *f0, const ST *fq, CUtensorMap *f0m
 // Staging geometry and planes per block of a launch.
 //
 // The depth comes from march_depth.  Its constants were fitted to forced depths
-// 1 .. 64 on 24 boxes from 32^3 to 256^3, 15 of them drawn at random: the depth
+// 1 .. 64 on 33 boxes from 32^3 to 512^3, 15 of them drawn at random: the depth
 // taken is within 0.4% of the best on average (4.0% at most) for the 16-bit
-// kernel, 0.2% (2.1%) for the dense one and 0.6% (7.5%) for the deep one.
+// kernel, 0.2% (1.7%) for the dense one and 0.5% (7.4%) for the deep one.  No
+// large box gained from more than 24 planes (their blocks drift apart, and
+// neighbouring tiles then share fewer halo rows in L2): 512^3 FP16 2777 us at
+// 22 planes, 2831 at 37, 3069 at 64; FP32 4814, 4862, 4936.
 //
 // FP32 takes the geometry with the lower estimate: on each of the 17 boxes of
 // up to 1.2 million nodes the faster one of the two at their depths.  Deep /
@@ -1345,15 +1348,15 @@ Plan choose_plan(const Box &b)
     const long long tiles = (long long)(b.nx / TX) * (b.ny / TY);
     const int sms = sm_count();
     if constexpr (sizeof(ST) == 2) {
-        constexpr MarchCost cost = {1.45, {0.0, 1.0, 1.33, 1.97, 2.10}, {0.30, 0.79, 1.22, 1.62, 1.77}};
+        constexpr MarchCost cost = {22, 1.45, {0.0, 1.0, 1.33, 1.97, 2.10}, {0.30, 0.79, 1.22, 1.62, 1.77}};
         plan.tz = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), cost).tz;
     } else {
-        constexpr MarchCost deep = {1.16, {0.0, 1.0, 1.50}, {0.30, 0.97, 1.54}};
-        constexpr MarchCost dense = {3.28, {0.0, 1.0, 1.53, 1.71}, {0.91, 1.39, 1.51, 1.56}};
+        constexpr MarchCost deep = {22, 1.16, {0.0, 1.0, 1.50}, {0.30, 0.97, 1.54}};
+        constexpr MarchCost dense = {24, 3.19, {0.0, 1.0, 1.42, 1.58}, {1.16, 1.17, 1.08, 1.41}};
         const Depth d = march_depth(tiles, b.nz, sms, resident_blocks<ST, true>(), deep);
         const Depth e = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), dense);
         // the two costs in one unit
-        plan.deep = d.cost <= 0.9 * e.cost - 0.5;
+        plan.deep = d.cost <= 1.12 * e.cost - 2.25;
         plan.tz = plan.deep ? d.tz : e.tz;
     }
     last[0] = b.nx;
