@@ -119,7 +119,7 @@ struct Adjoint {
     // lambda: L, the 19 lg and, when tauPhi is not 1, the seven q (AdjointBuffers)
     float *lam_L[2] = {nullptr, nullptr}, *lam_g[2] = {nullptr, nullptr}, *lam_q[2] = {nullptr, nullptr};
     float *lsrc = nullptr;        // 4 x n
-    double *partials = nullptr, *dgrav = nullptr, *ab = nullptr, *acc = nullptr;
+    double *partials = nullptr, *dgrav = nullptr, *wuz = nullptr, *ab = nullptr, *acc = nullptr;
     unsigned char *slots = nullptr;   // the context's checkpoint pool
     std::vector<Snapshot> snaps;
     unsigned char *host = nullptr;    // pinned host checkpoints (second tier), slot layout
@@ -131,8 +131,8 @@ struct Adjoint {
     lbm::StepConst k;
     int first_source;            // first state index with an objective term
     double scale;
-    // Side stream: phi and the objective of state n depend only on that
-    // state, so they run there as soon as it exists, overlapping the main
+    // Side stream: phi of state n and the objective's weight sum depend only on
+    // that state, so they run there as soon as it exists, overlapping the main
     // stream's adjoint kernels of step n + 1.  Events order the two streams:
     // slot_ev[s] / ctx_ev mark a state written, buf_free[b] the main stream's
     // last read of phi / ab buffer b, side_done the side work of a step.
@@ -352,12 +352,11 @@ struct Adjoint {
         cudaError_t e = cudaStreamWaitEvent(side, ready, 0);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(side, buf_free[b], 0);
         if (e != cudaSuccess) return cuda_fail(e, "adjoint: stream order");
-        int rc = prepare(st, ph, side);
-        if (rc) return rc;
-        if (src)
-            e = lbm::launch_objective(c->box, o.objective, c->d.phiStar, scale, c->q, st, ph, partials, abs_, acc,
-                                      side);
-        if (e == cudaSuccess) e = cudaEventRecord(side_done, side);
+        // (only the u_z objective has states before the last in its window)
+        e = lbm::launch_adjoint_phi(c->box, c->d.eta, c->q, st, ph, side, c->d.phiStar, scale, partials,
+                                    src ? abs_ : nullptr);
+        if (e != cudaSuccess) return cuda_fail(e, "adjoint: phi");
+        e = cudaEventRecord(side_done, side);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, side_done, 0);
         if (e != cudaSuccess) return cuda_fail(e, "adjoint: side stream");
         lbm::AdjointBuffers a;
@@ -370,8 +369,10 @@ struct Adjoint {
         a.L_out = lam_L[1 - cur];
         a.lsrc = lsrc;
         a.dgrav = dgrav;
+        a.wuz = wuz;
         a.ab = abs_;
-        e = lbm::launch_adjoint_step(c->box, k, c->d.phiStar, c->q, st, a, src, o.objective, scale, c->stream);
+        a.acc = acc;
+        e = lbm::launch_adjoint_step(c->box, k, c->d.phiStar, c->q, st, a, src, scale, c->stream);
         if (e != cudaSuccess) return cuda_fail(e, "adjoint step");
         cur = 1 - cur;
         adj_steps++;
@@ -557,6 +558,7 @@ struct Adjoint {
         }
         lsrc = w.take<float>(4 * n);
         dgrav = w.take<double>(lbm::adjoint_dgrav_parts(c->box));
+        wuz = w.take<double>(lbm::adjoint_dgrav_parts(c->box));
     }
 };
 

@@ -108,7 +108,9 @@ struct AdjointBuffers {
     float *lq_out, *lg_out, *L_out;    // lambda^n
     float *lsrc;                       // scratch: lambda_lap and mu lambda_F, four fields
     double *dgrav;                     // per-warp running sums of the dJ/dgrav terms
-    const double *ab;                  // objective sums of s^n
+    double *wuz;                       // per-warp sums of the step's w u_z (window steps)
+    double *ab;                        // objective sums of s^n (window steps)
+    double *acc;                       // acc[0] += its term of J (window steps)
 };
 
 // Planes per block of a kernel whose blocks march `planes` planes on `tiles`
@@ -206,17 +208,22 @@ cudaError_t launch_pressure(const Box &b, const lbm_derived &d, const float *mom
 size_t adjoint_blocks(const Box &b);
 // Length of the dgrav array: one running sum per warp of the march kernel's grid.
 size_t adjoint_dgrav_parts(const Box &b);
+// phi of a native state; with ab also B = ab[1], the sum of the objective's
+// weights, and ab[3] = scale / B (partials: scratch of adjoint_blocks doubles).
 cudaError_t launch_adjoint_phi(const Box &b, float eta, const Quant &q, const NativeState &st, float *phi,
-                               cudaStream_t s);
+                               cudaStream_t s, float phiStar = 1.f, double scale = 0.0, double *partials = nullptr,
+                               double *ab = nullptr);
 cudaError_t launch_objective(const Box &b, int objective, float phiStar, double scale, const Quant &q,
                              const NativeState &st, const float *phi, double *partials, double *ab, double *acc,
                              cudaStream_t s);
 cudaError_t launch_source_init(const Box &b, int objective, double scale, const double *ab, float phiStar,
                                const Quant &q, const NativeState &st, const float *phi, float *lq, float *lg,
                                float *L, cudaStream_t s);
+// One adjoint step; add_source: s^n is in the averaging window of the u_z
+// objective (a.ab then holds B of it; A and the term of J are found here).
 cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar, const Quant &q,
-                                const NativeState &st, const AdjointBuffers &a, bool add_source, int objective,
-                                double scale, cudaStream_t s);
+                                const NativeState &st, const AdjointBuffers &a, bool add_source, double scale,
+                                cudaStream_t s);
 // acc[1] = sum of the per-warp dgrav sums.
 cudaError_t launch_dgrav_fold(const Box &b, const double *dgrav, double *acc, cudaStream_t s);
 cudaError_t launch_init_adjoint(const Box &b, const lbm_derived &d, float Gamma, const float *phi0, const float *lq,

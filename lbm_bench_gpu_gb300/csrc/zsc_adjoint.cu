@@ -190,11 +190,33 @@ __device__ __forceinline__ double block_sum(double v, double *red)
 
 __device__ __forceinline__ unsigned block_id() { return blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z); }
 
-// phi = sum of the streamed f of a native state (FP32 storage).
-__global__ void __launch_bounds__(NTA) adjoint_phi_kernel(Box b, float eta, const float *__restrict__ f0,
-                                                          const FQFields fq, int f_streamed, float *__restrict__ phi)
+// The light phase's weight sum of one block of a phi kernel (NT threads, linear
+// thread number tid) into *out.
+template <int NT>
+__device__ __forceinline__ void weight_sum(double v, int tid, double *out)
 {
-    const float eta2 = 1.f - eta;
+    __shared__ double red[NT / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((tid & 31) == 0) red[tid >> 5] = v;
+    __syncthreads();
+    if (tid == 0) {
+        double r = 0.0;
+        for (int w = 0; w < NT / 32; w++) r += red[w];
+        *out = r;
+    }
+}
+
+// phi = sum of the streamed f of a native state (FP32 storage).  With SUM also
+// the per-block sums of w = (phiStar - phi) / (2 phiStar), the objective's
+// weight, which an adjoint step of the averaging window needs.
+template <bool SUM>
+__global__ void __launch_bounds__(NTA) adjoint_phi_kernel(Box b, float eta, const float *__restrict__ f0,
+                                                          const FQFields fq, int f_streamed, float *__restrict__ phi,
+                                                          float phiStar, double *__restrict__ partials)
+{
+    const float eta2 = 1.f - eta, half_inv = 0.5f / phiStar;
+    double B = 0.0;
     const int x = blockIdx.x * TXA + threadIdx.x, y = blockIdx.y * TYA + threadIdx.y;
     for (int z = blockIdx.z * kPlanes, z_end = min(b.nz, z + kPlanes); z < z_end; z++) {
         const Nb p = neighbourhood(b, x, y, z);
@@ -207,20 +229,24 @@ __global__ void __launch_bounds__(NTA) adjoint_phi_kernel(Box b, float eta, cons
             s += f_streamed ? here : eta * a[dir_at(p, i, -1)] + eta2 * here;
         }
         phi[t] = s;
+        if (SUM) B += (double)((phiStar - s) * half_inv);
     }
+    if (SUM) weight_sum<NTA>(B, threadIdx.y * TXA + threadIdx.x, partials + block_id());
 }
 
 // The same for 16-bit storage: a thread sums the two nodes of one pair-layout
 // word, so that every load is a whole word (with two-byte loads, 256^3 took 87
 // us; the 20 bytes a node take 49 at the copy bandwidth).
-template <typename ST>
+template <typename ST, bool SUM>
 __global__ void __launch_bounds__(TXA / 2 * TYA) adjoint_phi_pair_kernel(Box b, float eta, float inv,
                                                                          const float *__restrict__ f0,
                                                                          const FQFields fq, int f_streamed,
-                                                                         float *__restrict__ phi)
+                                                                         float *__restrict__ phi, float phiStar,
+                                                                         double *__restrict__ partials)
 {
     using T2 = typename Fmt<ST>::T2;
-    const float eta2 = 1.f - eta;
+    const float eta2 = 1.f - eta, half_inv = 0.5f / phiStar;
+    double B = 0.0;
     const int h = b.nx / 2, w = blockIdx.x * (TXA / 2) + threadIdx.x, y = blockIdx.y * TYA + threadIdx.y;
     // the words at x - 1 and x + 1; past the x seam a word's nodes are swapped
     const int wl = w == 0 ? h - 1 : w - 1, wr = w == h - 1 ? 0 : w + 1;
@@ -251,7 +277,9 @@ __global__ void __launch_bounds__(TXA / 2 * TYA) adjoint_phi_pair_kernel(Box b, 
         const unsigned r = (unsigned)b.nx * ((unsigned)y + (unsigned)b.ny * (unsigned)z) + (unsigned)w;
         phi[r] = s.x;
         phi[r + (unsigned)h] = s.y;
+        if (SUM) B += (double)((phiStar - s.x) * half_inv) + (double)((phiStar - s.y) * half_inv);
     }
+    if (SUM) weight_sum<TXA / 2 * TYA>(B, threadIdx.y * (TXA / 2) + threadIdx.x, partials + block_id());
 }
 
 // Objective sums of one state: A = sum w q, B = sum w, with
@@ -307,6 +335,46 @@ __global__ void __launch_bounds__(NTA) objective_fold_kernel(const double *__res
         ab[2] = A / B;
         ab[3] = scale / B;
         acc[0] += scale * A / B;
+    }
+}
+
+// ab[1] = B = sum of the phi kernel's weight sums, ab[3] = scale / B.
+__global__ void __launch_bounds__(NTA) weight_fold_kernel(const double *__restrict__ partials, int nparts, double scale,
+                                                          double *__restrict__ ab)
+{
+    __shared__ double red[NTA / 32];
+    double B = 0.0;
+    for (int p = threadIdx.y * TXA + threadIdx.x; p < nparts; p += NTA) B += partials[p];
+    B = block_sum(B, red);
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        ab[1] = B;
+        ab[3] = scale / B;
+    }
+}
+
+// ab[0] = A = sum of the march kernel's sums of w u_z, ab[2] = A / B; acc[0] (J)
+// += scale A / B.
+__global__ void __launch_bounds__(1024) velocity_fold_kernel(const double *__restrict__ parts, int nparts, double scale,
+                                                             double *__restrict__ ab, double *__restrict__ acc)
+{
+    __shared__ double red[32];
+    const int tid = threadIdx.x;
+    double A = 0.0;
+#pragma unroll 4
+    for (int p = tid; p < nparts; p += 1024) A += parts[p];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) A += __shfl_down_sync(0xffffffffu, A, o);
+    if ((tid & 31) == 0) red[tid >> 5] = A;
+    __syncthreads();
+    if (tid < 32) {
+        A = red[tid];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) A += __shfl_down_sync(0xffffffffu, A, o);
+        if (tid == 0) {
+            ab[0] = A;
+            ab[2] = A / ab[1];
+            acc[0] += scale * A / ab[1];
+        }
     }
 }
 
@@ -385,9 +453,9 @@ struct AdjIn {
     float *lphi;                           // lambda_phi^n (L^n without its stencil part)
     float *lsrc[4];                        // lambda_lap, mu lambda_F at every node
     double *dgrav;                         // per warp of each block, accumulated over steps
-    const double *ab;                      // objective sums of s^n (when add_source)
-    double scale;
-    int objective, add_source;
+    double *wuz;                           // per warp: sum of w u_z of s^n (when add_source)
+    const double *ab;                      // objective sums of s^n: ab[3] = scale / B (when add_source)
+    int add_source;                        // s^n is in the averaging window of the u_z objective
 };
 
 __device__ __forceinline__ int wrap_to(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
@@ -575,7 +643,7 @@ adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_co
     float a_b = below.a, fx_b = below.fx, fy_b = below.fy;
     PlaneSums cur = plane_sums<Gm::HP>(SP + hslot(z0));
     float L_m = SF[hslot(z0 - 1)], L_c = SF[hslot(z0)];
-    double dg = 0.0;
+    double dg = 0.0, wuz = 0.0;
 
     for (int j = 0; j < nzc; ++j) {
         const int z = z0 + j, st = j & 1;
@@ -731,11 +799,15 @@ adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_co
 #pragma unroll
         for (int k = 0; k < 3; k++) a.lsrc[1 + k][t] = mu * lF[k];
         if (a.add_source) {
-            float dphi, drho, dmz;
-            objective_source(z, a.objective, source_coef(a.ab, phiStar), phiStar, ph, rh, m[2], dphi, drho, dmz);
-            lphi += dphi;
-            lrho += drho;
-            lm[2] += dmz;
+            // the objective's source but for its part of A / B, which is the
+            // same at every node and which the stencil kernel adds when A is
+            // known (objective_source with ratio 0)
+            const float half_inv = 0.5f / phiStar, s_over_b = (float)a.ab[3];
+            const float w = (phiStar - ph) * half_inv, uz = m[2] * inv, duz = s_over_b * w;
+            wuz += (double)(w * (m[2] / rh));
+            lphi += -half_inv * s_over_b * uz;
+            lrho += -duz * uz * inv;
+            lm[2] += duz * inv;
         }
         a.lphi[t] = lphi;
         if constexpr (LQ) {
@@ -755,6 +827,11 @@ adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_co
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dg += __shfl_down_sync(0xffffffffu, dg, o);
     if (tx == 0) a.dgrav[blockIdx.x * (NTA / 32) + ty] += dg;
+    if (a.add_source) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) wuz += __shfl_down_sync(0xffffffffu, wuz, o);
+        if (tx == 0) a.wuz[blockIdx.x * (NTA / 32) + ty] = wuz;
+    }
 }
 
 // L = lambda_phi + Lap[lambda_lap] - sum_k D_k[lambda_grad_k]: the transposed
@@ -778,8 +855,11 @@ struct StencilGeo {
 };
 
 __global__ void __launch_bounds__(NTA, kStencilBlocks)
-adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict__ lphi, int tz)
+adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict__ lphi, int tz,
+                       const double *__restrict__ ab, float phiStar)
 {
+    // the objective's source common to all nodes (see the march kernel)
+    const float common = ab ? 0.5f / phiStar * (float)ab[3] * (float)ab[2] : 0.f;
     using G = StencilGeo;
     __shared__ __align__(16) float sm[G::STAGES][G::PLANE];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TXA + tx;
@@ -848,7 +928,7 @@ adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict_
         cp_async_wait_prior<1>();
         __syncthreads();   // plane z + 1 has landed
         const Part top = part(at(j + 2));
-        lphi[t] = base + ((cur.own + top.below) + from_below);
+        lphi[t] = (base + common) + ((cur.own + top.below) + from_below);
         from_below = cur.above;
         cur = top;
     }
@@ -981,24 +1061,33 @@ size_t adjoint_dgrav_parts(const Box &b) { return (size_t)march_of(b).blocks * (
 size_t adjoint_blocks(const Box &b) { return blocks_of(adjoint_grid(b)); }
 
 cudaError_t launch_adjoint_phi(const Box &b, float eta, const Quant &q, const NativeState &st, float *phi,
-                               cudaStream_t s)
+                               cudaStream_t s, float phiStar, double scale, double *partials, double *ab)
 {
     const int streamed = st.f_streamed ? 1 : 0;
-    const dim3 pair(TXA / 2, TYA);
-    switch (st.storage) {
-    case LBM_STORAGE_FP32:
-        adjoint_phi_kernel<<<adjoint_grid(b), kBlock, 0, s>>>(b, eta, st.f0, fq_fields(b, st), streamed, phi);
-        break;
-    case LBM_STORAGE_FP16:
-        adjoint_phi_pair_kernel<__half><<<adjoint_grid(b), pair, 0, s>>>(b, eta, q.f_inv, st.f0, fq_fields(b, st),
-                                                                         streamed, phi);
-        break;
-    case LBM_STORAGE_BF16:
-        adjoint_phi_pair_kernel<__nv_bfloat16><<<adjoint_grid(b), pair, 0, s>>>(b, eta, q.f_inv, st.f0,
-                                                                                fq_fields(b, st), streamed, phi);
-        break;
-    default: return cudaErrorInvalidValue;
-    }
+    const dim3 grid = adjoint_grid(b), pair(TXA / 2, TYA);
+    const FQFields fq = fq_fields(b, st);
+    auto go = [&](auto sum) {
+        constexpr bool SUM = decltype(sum)::value;
+        switch (st.storage) {
+        case LBM_STORAGE_FP32:
+            adjoint_phi_kernel<SUM><<<grid, kBlock, 0, s>>>(b, eta, st.f0, fq, streamed, phi, phiStar, partials);
+            break;
+        case LBM_STORAGE_FP16:
+            adjoint_phi_pair_kernel<__half, SUM><<<grid, pair, 0, s>>>(b, eta, q.f_inv, st.f0, fq, streamed, phi,
+                                                                       phiStar, partials);
+            break;
+        case LBM_STORAGE_BF16:
+            adjoint_phi_pair_kernel<__nv_bfloat16, SUM><<<grid, pair, 0, s>>>(b, eta, q.f_inv, st.f0, fq, streamed,
+                                                                              phi, phiStar, partials);
+            break;
+        default: return cudaErrorInvalidValue;
+        }
+        return cudaGetLastError();
+    };
+    if (!ab) return go(std::false_type{});
+    const cudaError_t e = go(std::true_type{});
+    if (e != cudaSuccess) return e;
+    weight_fold_kernel<<<1, kBlock, 0, s>>>(partials, (int)blocks_of(grid), scale, ab);
     return cudaGetLastError();
 }
 
@@ -1030,8 +1119,8 @@ cudaError_t launch_source_init(const Box &b, int objective, double scale, const 
 }
 
 cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar, const Quant &q,
-                                const NativeState &st, const AdjointBuffers &a, bool add_source, int objective,
-                                double scale, cudaStream_t s)
+                                const NativeState &st, const AdjointBuffers &a, bool add_source, double scale,
+                                cudaStream_t s)
 {
     AdjIn in;
     std::memset(&in, 0, sizeof(in));
@@ -1050,9 +1139,8 @@ cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar,
     }
     for (int k = 0; k < 4; k++) in.lsrc[k] = a.lsrc + (size_t)k * n;
     in.dgrav = a.dgrav;
+    in.wuz = a.wuz;
     in.ab = a.ab;
-    in.scale = scale;
-    in.objective = objective;
     in.add_source = add_source ? 1 : 0;
     const March march = march_of(b);
     cudaError_t e = dispatch(st, [&](auto tag, auto odd) {
@@ -1068,8 +1156,13 @@ cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar,
                        : go(adjoint_march_kernel<ST, decltype(odd)::value, false>);
     });
     if (e != cudaSuccess) return e;
+    if (add_source) {
+        velocity_fold_kernel<<<1, 1024, 0, s>>>(a.wuz, march.blocks * (NTA / 32), scale, a.ab, a.acc);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     const March sten = stencil_march(b);
-    adjoint_stencil_kernel<<<(unsigned)sten.blocks, kBlock, 0, s>>>(b, a.lsrc, a.L_out, sten.tz);
+    adjoint_stencil_kernel<<<(unsigned)sten.blocks, kBlock, 0, s>>>(b, a.lsrc, a.L_out, sten.tz,
+                                                                         add_source ? a.ab : nullptr, phiStar);
     return cudaGetLastError();
 }
 
