@@ -379,6 +379,23 @@ struct StepBox {
     long long nxy, n;
 };
 
+// Element idx of a field.  16-bit storage takes it by a 32-bit byte offset: a
+// field is below 4 GB (19 n < 2^32 elements; a z-slab's, with its ghost planes,
+// 2.1 GB), and a 64-bit base plus a 32-bit offset is one operand of a load or
+// store, where an element index needs a multiplication of its own.  The kernel
+// runs at half the issue rate with 16 warps on an SM, so its time follows the
+// instruction count: odd steps 107.4 -> 102.6 M warp instructions at 192^3,
+// FP16 342 -> 334 us a step at 256^3, 51.4 -> 49.8 at 128^3.  FP32 keeps the
+// element index: its odd kernel has no registers for the offsets (256^3
+// 600 -> 637 us).
+template <typename ST, typename T>
+__device__ __forceinline__ T *elem(T *field, unsigned idx)
+{
+    if constexpr (sizeof(ST) == 2)
+        return reinterpret_cast<T *>(reinterpret_cast<unsigned long long>(field) + idx * (unsigned)sizeof(T));
+    else
+        return field + idx;
+}
 __device__ __forceinline__ unsigned node_index(const StepBox &b, int x, int y, int z)
 {
     return (unsigned)x + (unsigned)b.nx * ((unsigned)y + (unsigned)b.ny * (unsigned)z);
@@ -537,13 +554,13 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
         }
         const unsigned zb = (unsigned)zf(p) * (unsigned)b.nxy;
         if (f0_issuer && in_field((long long)zb + f0_xy, 4, nf, P.err))
-            cp_async16(f0part(st) + f0_dst, P.f0in + (zb + (unsigned)f0_xy));
+            cp_async16(f0part(st) + f0_dst, elem<ST>(P.f0in, zb + (unsigned)f0_xy));
         if (fq_issuer) {
             ST *dst = fqpart(st) + fq_dst;
             const unsigned base = zb + (unsigned)fq_xy;
 #pragma unroll
             for (int a = 0; a < kQf - 1; a++)
-                if (in_field(base, E, nf, P.err)) cp_async16(dst + a * FR * W, P.fin[a] + base);
+                if (in_field(base, E, nf, P.err)) cp_async16(dst + a * FR * W, elem<ST>(P.fin[a], base));
         }
     };
     auto issue_f = [&](int p) { issue_f_to(p, fstage(p), fbar(p)); };
@@ -581,7 +598,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
             const unsigned base = (unsigned)zg0(z) * (unsigned)b.nxy + (unsigned)(g_row_0 + g_x_hi);
             for_my_dirs([&](auto d) {
                 constexpr int i = decltype(d)::value;
-                if (in_field(base, E, ng, P.err)) cp_async16(dst + i * TY * GW + E + E * g_k, P.gin[i] + base);
+                if (in_field(base, E, ng, P.err)) cp_async16(dst + i * TY * GW + E + E * g_k, elem<ST>(P.gin[i], base));
             });
         } else {
             const unsigned zb0 = (unsigned)zg0(z) * (unsigned)b.nxy;
@@ -592,19 +609,24 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
                 constexpr int cx = kCx(i), cy = kCy(i), cz = kCz(i);
                 const unsigned zb = cz > 0 ? zbp : (cz < 0 ? zbm : zb0);
                 const int row = cy > 0 ? g_row_p : (cy < 0 ? g_row_m : g_row_0);
-                const ST *src = P.gin[kOpp(i)] + (zb + (unsigned)row);
+                const unsigned zr = zb + (unsigned)row;
+                const ST *row_src = P.gin[kOpp(i)] + zr;
+                auto src = [&](int col) {
+                    if constexpr (PAIR) return elem<ST>(P.gin[kOpp(i)], zr + (unsigned)col);
+                    else return row_src + col;
+                };
                 ST *d_row = dst + i * TY * GW;
                 const long long r0 = (long long)zb + row;   // row start in the field
                 if (cx > 0) {
                     // columns 0 .. TX + E - 1 hold x0 - E .. x0 + TX - 1
-                    if (in_field(r0 + g_x_lo, E, ng, P.err)) cp_async16(d_row + E * g_k, src + g_x_lo);
+                    if (in_field(r0 + g_x_lo, E, ng, P.err)) cp_async16(d_row + E * g_k, src(g_x_lo));
                     if (g_k == 0 && in_field(r0 + x0 + TX - E, E, ng, P.err))
-                        cp_async16(d_row + TX, src + (x0 + TX - E));
+                        cp_async16(d_row + TX, src(x0 + TX - E));
                 } else {
                     // columns GX0 .. hold x0 .. x0 + TX (+ E for cx < 0)
-                    if (in_field(r0 + g_x_hi, E, ng, P.err)) cp_async16(d_row + GX0 + E * g_k, src + g_x_hi);
+                    if (in_field(r0 + g_x_hi, E, ng, P.err)) cp_async16(d_row + GX0 + E * g_k, src(g_x_hi));
                     if (cx < 0 && g_k == 0 && in_field(r0 + g_x_wrap, E, ng, P.err))
-                        cp_async16(d_row + TX + GX0, src + g_x_wrap);
+                        cp_async16(d_row + TX + GX0, src(g_x_wrap));
                 }
             });
         }
@@ -1118,12 +1140,12 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
                 auto fc = [&](int k) { return fcur2[k]; };
                 const float2 Af = mul(splat(0.5f * c.Gamma * c.invTauPhi), mu);
                 if (in_field(idf, 2, nf, P.err))
-                    *reinterpret_cast<float2 *>(P.f0out + idf) =
+                    *reinterpret_cast<float2 *>(elem<ST>(P.f0out, idf)) =
                         fma(a2, fc(0), fma(splat(-6.f), Af, mul(splat(c.invTauPhi), pc)));
                 const float2 Afk = mul(splat(m.Af), mu), Cf = mul(splat(m.Cf), pc);
                 const float2 cux = mul(Cf, usx), cuy = mul(Cf, usy), cuz = mul(Cf, usz);
                 auto put2 = [&](int k, float2 v) {
-                    if (in_field(idf, 2, nf, P.err)) *reinterpret_cast<T2 *>(P.fout[k] + idf) = Fm::store2(v);
+                    if (in_field(idf, 2, nf, P.err)) *reinterpret_cast<T2 *>(elem<ST>(P.fout[k], idf)) = Fm::store2(v);
                 };
                 put2(0, fma(a2, fc(1), add(Afk, cux)));
                 put2(1, fma(a2, fc(2), sub(Afk, cux)));
@@ -1177,7 +1199,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
 #pragma unroll
                     for (int i = 0; i < kQg; i++)
                         if (in_field(idg, 2, ng, P.err))
-                            *reinterpret_cast<T2 *>(P.g[kOpp(i)] + idg) = Fm::store2(qv[i]);
+                            *reinterpret_cast<T2 *>(elem<ST>(P.g[kOpp(i)], idg)) = Fm::store2(qv[i]);
                 } else {
                     // odd: downstream neighbours x + c_i, natural slot i.  Both
                     // nodes of the word move to the neighbouring word together;
@@ -1194,7 +1216,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
                                       (kCz(i) > 0 ? o_zp : kCz(i) < 0 ? o_zm : 0);
                         T2 h = Fm::store2(qv[i]);
                         if (kCx(i) != 0) h = Fm::perm2(h, kCx(i) > 0 ? sel_r : sel_l);
-                        if (in_field((long long)idg + o, 2, ng, P.err)) *reinterpret_cast<T2 *>(P.g[i] + idg + o) = h;
+                        if (in_field((long long)idg + o, 2, ng, P.err)) *reinterpret_cast<T2 *>(elem<ST>(P.g[i], idg + (unsigned)o)) = h;
                     }
                 }
             }
