@@ -731,65 +731,68 @@ adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_co
             lmu += 0.5f * c.Gamma * c.invTauPhi * lAf;
         }
         // D3Q19 collision with forcing
-        float ls = 0.f, lvsq6 = 0.f, lUF = 0.f, lv[3] = {0.f, 0.f, 0.f};
+        float ls, lvsq6, lUF, lv[3];
         {
-            ls += -2.f * c.K0 * lQ[0];
-            lrho += c.K0 * (1.f - vsq6) * lQ[0];
-            lvsq6 += -c.K0 * rh * lQ[0];
-            lUF += -c.KC0 * lQ[0];
-            float ltemp1 = 0.f;
+            // A weight class's constants are taken out of its sums, and the sums
+            // over lambda_Q that several terms share are formed once: the kernel
+            // runs at half the issue rate, and with every term written out it
+            // took 825 instructions a node and plane in place of 737 (192^3 FP16
+            // state 306 -> 290 us, FP32 297 -> 287).
+            const float K1r = c.K1 * rh, K2r = c.K2 * rh;
+            const float G1[3] = {c.KC1 * F[0], c.KC1 * F[1], c.KC1 * F[2]};
+            const float G2[3] = {c.KC2 * F[0], c.KC2 * F[1], c.KC2 * F[2]};
+            float ltemp1 = 0.f, lrho1 = 0.f, lF1[3];
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 const float S = lQ[1 + 2 * k] + lQ[2 + 2 * k], A = lQ[1 + 2 * k] - lQ[2 + 2 * k];
+                const float SA = S + A, vS = v[k] * S;
                 ltemp1 += S;
-                lrho += 0.5f * c.K1 * v[k] * v[k] * S + c.K1 * v[k] * A;
-                lv[k] += c.K1 * rh * v[k] * S + c.KC1 * F[k] * S + (c.K1 * rh + c.KC1 * F[k]) * A;
-                lF[k] += c.KC1 * v[k] * (S + A);
-                lUF += -c.KC1 * S;
+                lrho1 += v[k] * (0.5f * vS + A);
+                lv[k] = K1r * (vS + A) + G1[k] * SA;
+                lF1[k] = v[k] * SA;
             }
-            ls += c.K1 * ltemp1;
-            lrho += c.K1 * (1.f - vsq6) * ltemp1;
-            lvsq6 += -c.K1 * rh * ltemp1;
             // pairs (7,8) x+y, (9,10) x-y, (11,12) x+z, (13,14) x-z, (15,16) y+z, (17,18) y-z
             constexpr int PA[6] = {0, 0, 0, 0, 1, 1}, PB[6] = {1, 1, 2, 2, 2, 2};
             constexpr float SG[6] = {1.f, -1.f, 1.f, -1.f, 1.f, -1.f};
-            float ltemp2 = 0.f;
+            float ltemp2 = 0.f, lrho2 = 0.f, lF2[3] = {0.f, 0.f, 0.f};
 #pragma unroll
             for (int pp = 0; pp < 6; pp++) {
                 const int ia = PA[pp], ib = PB[pp];
                 const float sg = SG[pp];
-                const float w = v[ia] + sg * v[ib], Gs = F[ia] + sg * F[ib];
+                const float w = v[ia] + sg * v[ib], Gs = G2[ia] + sg * G2[ib];
                 const float S = lQ[7 + 2 * pp] + lQ[8 + 2 * pp], A = lQ[7 + 2 * pp] - lQ[8 + 2 * pp];
+                const float wS = w * S, B = wS + A;
                 ltemp2 += S;
-                lrho += 0.5f * c.K2 * w * w * S + c.K2 * w * A;
-                const float lw = c.K2 * rh * w * S + c.KC2 * Gs * S + c.K2 * rh * A;
-                const float lG = c.KC2 * w * S + c.KC2 * A;
-                lUF += -c.KC2 * S;
+                lrho2 += w * (0.5f * wS + A);
+                const float lw = K2r * B + Gs * S;
                 lv[ia] += lw;
                 lv[ib] += sg * lw;
-                lF[ia] += lG;
-                lF[ib] += sg * lG;
+                lF2[ia] += B;
+                lF2[ib] += sg * B;
             }
-            ls += c.K2 * ltemp2;
-            lrho += c.K2 * (1.f - vsq6) * ltemp2;
-            lvsq6 += -c.K2 * rh * ltemp2;
+#pragma unroll
+            for (int k = 0; k < 3; k++) lF[k] = c.KC1 * lF1[k] + c.KC2 * lF2[k];
+            const float T0 = c.K0 * lQ[0], T = c.K2 * ltemp2 + (c.K1 * ltemp1 + T0);
+            ls = T - 3.f * T0;
+            lUF = -(c.KC2 * ltemp2 + (c.KC1 * ltemp1 + c.KC0 * lQ[0]));
+            lvsq6 = -rh * T * (1.f / 3.f);
+            lrho += (1.f - vsq6) * T + (c.K1 * lrho1 + c.K2 * lrho2);
         }
 #pragma unroll
-        for (int k = 0; k < 3; k++) lv[k] += lvsq6 * v[k] * (1.f / 3.f);
-#pragma unroll
         for (int k = 0; k < 3; k++) {
+            lv[k] += lvsq6 * v[k];
             lus[k] += lUF * F[k] + 3.f * lv[k];
             lF[k] += lUF * us[k];
         }
-        lphi += 3.f * mu * ls;
-        lmu += 3.f * ph * ls;
+        const float ls3 = 3.f * ls;
+        lphi += mu * ls3;
+        lmu += ph * ls3;
         float lm[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            lF[k] += 0.5f * lus[k] * inv;
-            lrho += -0.5f * lus[k] * F[k] * inv * inv;
             lm[k] = lus[k] * inv;
-            lrho += -lus[k] * u[k] * inv;
+            lF[k] += 0.5f * lm[k];
+            lrho -= lm[k] * us[k];   // us = u + F / (2 rho)
         }
 #pragma unroll
         for (int k = 0; k < 3; k++) lmu += gr[k] * lF[k];
