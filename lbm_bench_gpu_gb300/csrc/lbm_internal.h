@@ -126,7 +126,7 @@ struct AdjointBuffers {
 struct MarchCost {
     int deepest;
     double prologue;
-    double share[7], tail[7];
+    double share[9], tail[9];
 };
 struct Depth {
     int tz;

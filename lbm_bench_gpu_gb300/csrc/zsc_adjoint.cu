@@ -46,7 +46,7 @@ constexpr int TXA = 32, TYA = 8, NTA = TXA * TYA;
 #define ZSC_ADJ_PLANES 4
 #endif
 constexpr int kPlanes = ZSC_ADJ_PLANES;
-constexpr int kStencilBlocks = 5;   // resident blocks of the stencil kernel per SM
+constexpr int kStencilBlocks = 8;   // resident blocks of the stencil kernel per SM
 constexpr float kInv6 = 0.16666666666666666667f;
 constexpr float kInv12 = 0.08333333333333333333f;
 constexpr float kW0 = 0.33333333333333333333f, kW1 = 0.05555555555555555556f, kW2 = 0.02777777777777777778f;
@@ -843,21 +843,26 @@ adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_co
 // 1/12 on edges.
 //
 // A block marches tz planes of a 32 x 8 tile.  The four source fields of a
-// plane (the tile plus one node) are staged one plane ahead with 16-byte
+// plane (the tile plus one node) are staged two planes ahead with 16-byte
 // cp.async copies.  Regrouped by plane, a node takes three numbers from each:
 // what it adds to the node in it, to the node above and to the node below,
-// which two registers carry down the march; a plane is read at 26 scalars per
-// node, not 49 in three planes.  Bound by DRAM at 24 bytes a node (59 us at
-// 256^3 at the copy bandwidth).
+// which two registers carry down the march.  A thread has two rows of the
+// tile, which share the rows between them: 20 shared-memory reads a node and
+// plane (31 with one row, 49 without the regrouping), and eight blocks of 128
+// threads stay on an SM.  24 bytes a node, 59 us at 256^3 at the copy
+// bandwidth; 84 us (one row a thread and lambda_phi read where it is used
+// 104, the kernel before with no staging 152), 128^3 16 us (20, 24): bound by
+// the latency of its shared-memory reads and barriers beside DRAM at 70 %.
 struct StencilGeo {
     static constexpr int P = TXA + 8, ROWS = TYA + 2;      // staged row and rows (floats)
     static constexpr int FIELD = P * ROWS, PLANE = 4 * FIELD;
     static constexpr int CHUNKS = PLANE / 4;               // 16-byte chunks of a plane
-    static constexpr int PER = (CHUNKS + NTA - 1) / NTA;   // per thread
+    static constexpr int NT = NTA / 2;                     // threads of a block, two rows each
+    static constexpr int PER = (CHUNKS + NT - 1) / NT;     // per thread
     static constexpr int STAGES = 4;
 };
 
-__global__ void __launch_bounds__(NTA, kStencilBlocks)
+__global__ void __launch_bounds__(StencilGeo::NT, kStencilBlocks)
 adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict__ lphi, int tz,
                        const double *__restrict__ ab, float phiStar)
 {
@@ -875,7 +880,7 @@ adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict_
     unsigned off[G::PER];
 #pragma unroll
     for (int q = 0; q < G::PER; q++) {
-        const int e = tid + q * NTA, f = e / (G::FIELD / 4), r = e % (G::FIELD / 4);
+        const int e = tid + q * G::NT, f = e / (G::FIELD / 4), r = e % (G::FIELD / 4);
         const int row = r / (G::P / 4), kk = r % (G::P / 4);
         off[q] = (unsigned)f * n + (unsigned)(b.nx * wrap_to(y0 - 1 + row, b.ny) + wrap_to(x0 - 4 + 4 * kk, b.nx));
     }
@@ -883,30 +888,44 @@ adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict_
         const unsigned zo = (unsigned)wrap_to(z, b.nz) * nxy;
 #pragma unroll
         for (int q = 0; q < G::PER; q++) {
-            const int e = tid + q * NTA;
+            const int e = tid + q * G::NT;
             if (e < G::CHUNKS) cp_async16(&sm[stage][4 * e], lsrc + zo + off[q]);
         }
     };
-    // contributions of plane values at this node: to its own plane, to the
-    // plane below it (it is the plane above that one) and to the plane above
-    const int cell = (ty + 1) * G::P + tx + 4;
+    // contributions of plane values at this thread's nodes (rows 2 ty and
+    // 2 ty + 1 of the tile): to their own plane, to the plane below it (it is
+    // the plane above that one) and to the plane above
+    const int cell = (2 * ty + 1) * G::P + tx + 4;
     struct Part {
-        float own, below, above;
+        float own[2], below[2], above[2];
     };
     auto part = [&](int stage) -> Part {
-        const float *l = sm[stage] + cell, *gx = l + G::FIELD, *gy = gx + G::FIELD, *gz = gy + G::FIELD;
         constexpr int N = G::P;
-        const float lc = l[0], lf = (l[1] + l[-1]) + (l[N] + l[-N]);
-        const float le = (l[N + 1] + l[-N - 1]) + (l[-N + 1] + l[N - 1]);
-        const float sx = gx[1] - gx[-1], sy = gy[N] - gy[-N];
-        const float dx = (gx[N + 1] - gx[-N - 1]) + (gx[-N + 1] - gx[N - 1]);
-        const float dy = (gy[N + 1] - gy[-N - 1]) - (gy[-N + 1] - gy[N - 1]);
-        const float sz = ((gz[1] + gz[-1]) + (gz[N] + gz[-N])) + 2.f * gz[0];
+        const float *l = sm[stage] + cell - N, *gx = l + G::FIELD, *gy = gx + G::FIELD, *gz = gy + G::FIELD;
+        // rows -1 .. 2 about row 2 ty: sums over x - 1, x + 1 and differences
+        float lc[4], ls[4], xd[4], yc[4], yd[4], ys[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            lc[r] = l[r * N];
+            ls[r] = l[r * N + 1] + l[r * N - 1];
+            xd[r] = gx[r * N + 1] - gx[r * N - 1];
+            yc[r] = gy[r * N];
+            ys[r] = gy[r * N + 1] + gy[r * N - 1];
+        }
         Part p;
-        p.own = (le + 2.f * (lf - 12.f * lc)) * kInv6 - (2.f * (sx + sy) + (dx + dy)) * kInv12;
-        const float side = (lf + 2.f * lc) * kInv6 - (sx + sy) * kInv12;
-        p.below = side - sz * kInv12;   // c_z = +1 of the node below
-        p.above = side + sz * kInv12;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int c = k + 1;
+            const float lf = ls[c] + (lc[c + 1] + lc[c - 1]), le = ls[c + 1] + ls[c - 1];
+            const float sx = xd[c], sy = yc[c + 1] - yc[c - 1];
+            const float dx = xd[c + 1] + xd[c - 1], dy = ys[c + 1] - ys[c - 1];
+            const float *g = gz + c * N;
+            const float sz = ((g[1] + g[-1]) + (g[N] + g[-N])) + 2.f * g[0];
+            p.own[k] = (le + 2.f * (lf - 12.f * lc[c])) * kInv6 - (2.f * (sx + sy) + (dx + dy)) * kInv12;
+            const float side = (lf + 2.f * lc[c]) * kInv6 - (sx + sy) * kInv12;
+            p.below[k] = side - sz * kInv12;   // c_z = +1 of the node below
+            p.above[k] = side + sz * kInv12;
+        }
         return p;
     };
     // plane z0 - 1 + m is staged in stage m % STAGES, two planes ahead of its use
@@ -916,23 +935,33 @@ adjoint_stencil_kernel(Box b, const float *__restrict__ lsrc, float *__restrict_
         issue(z0 - 1 + m, at(m));
         cp_async_commit();
     }
+    unsigned t = (unsigned)z0 * nxy + (unsigned)((y0 + 2 * ty) * b.nx + x0 + tx);
+    const unsigned row = (unsigned)b.nx;
+    float next[2] = {lphi[t], lphi[t + row]};
     cp_async_wait_prior<2>();
     __syncthreads();
-    float from_below = part(at(0)).above;   // what plane z0 - 1 adds to plane z0
+    Part cur = part(at(0));
+    float from_below[2] = {cur.above[0], cur.above[1]};   // what plane z0 - 1 adds to plane z0
     cp_async_wait_prior<1>();
     __syncthreads();
-    Part cur = part(at(1));
-    unsigned t = (unsigned)z0 * nxy + (unsigned)((y0 + ty) * b.nx + x0 + tx);
+    cur = part(at(1));
     for (int j = 0; j < nzc; ++j, t += nxy) {
-        const float base = lphi[t];
+        const float base[2] = {next[0], next[1]};
         // plane z + 2 takes the stage of plane z - 2, read before the last barrier
-        if (j + 1 < nzc) issue(z0 + j + 2, at(j + 3));
+        if (j + 1 < nzc) {
+            issue(z0 + j + 2, at(j + 3));
+            next[0] = lphi[t + nxy];
+            next[1] = lphi[t + nxy + row];
+        }
         cp_async_commit();
         cp_async_wait_prior<1>();
         __syncthreads();   // plane z + 1 has landed
         const Part top = part(at(j + 2));
-        lphi[t] = (base + common) + ((cur.own + top.below) + from_below);
-        from_below = cur.above;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            lphi[t + (unsigned)k * row] = (base[k] + common) + ((cur.own[k] + top.below[k]) + from_below[k]);
+            from_below[k] = cur.above[k];
+        }
         cur = top;
     }
 }
@@ -1015,10 +1044,13 @@ March march_of(const Box &b)
     const int tz = march_depth(tiles, b.nz, sm_count(), 2, cost).tz;
     return March{tz, tiles * ((b.nz + tz - 1) / tz)};
 }
-// The stencil kernel's: a prologue of two planes, kStencilBlocks blocks on an SM.
+// The stencil kernel's: a prologue of two planes, kStencilBlocks blocks on an
+// SM.  Depths from 2 to 32 measured on seven boxes: the choice is within 5 % of
+// the best (64^3 2 planes 5.7 us, best 3 planes 5.5; 128^3 16.1, best; 256^3
+// 20 to 24 planes 84, 16 85, 32 86.5, 8 91.5).
 March stencil_march(const Box &b)
 {
-    constexpr MarchCost cost = {32, 2.0, {0.0, 1.0, 1.2, 1.5, 1.8, 2.2}, {0.88, 0.88, 1.06, 1.32, 1.58, 1.94}};
+    constexpr MarchCost cost = {24, 2.0, {0.0, 1.0, 1.05, 1.15, 1.3, 1.45, 1.65, 1.85, 2.1}, {0.88, 0.88, 0.93, 1.02, 1.15, 1.28, 1.46, 1.64, 1.85}};
     const int tiles = (b.nx / TXA) * (b.ny / TYA);
     const int tz = march_depth(tiles, b.nz, sm_count(), kStencilBlocks, cost).tz;
     return March{tz, tiles * ((b.nz + tz - 1) / tz)};
@@ -1164,7 +1196,7 @@ cudaError_t launch_adjoint_step(const Box &b, const StepConst &c, float phiStar,
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     const March sten = stencil_march(b);
-    adjoint_stencil_kernel<<<(unsigned)sten.blocks, kBlock, 0, s>>>(b, a.lsrc, a.L_out, sten.tz,
+    adjoint_stencil_kernel<<<(unsigned)sten.blocks, dim3(TXA, TYA / 2), 0, s>>>(b, a.lsrc, a.L_out, sten.tz,
                                                                          add_source ? a.ab : nullptr, phiStar);
     return cudaGetLastError();
 }
