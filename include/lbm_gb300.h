@@ -264,7 +264,7 @@ long long lbm_adjoint_forward_steps(long long nsteps, int slots);
  *   nodes of that region; 7 sum phi; 8 sum rho; 9..11 sum rho u;
  *   12 number of nodes with phi >= 0; 13 max |u|^2; 14 number of nodes with a
  *   non-finite value (full domain for 7..14); 15 zero.
- * The per-block partial sums use a 57 KiB array in the library's static device
+ * The per-block partial sums use a 38 KiB array in the library's static device
  * memory, which every GPU that loads the library keeps until the process
  * exits.  More than LBM_NOALLOC_MAX_NODES nodes is rejected with LBM_EINVAL,
  * and so are parameters whose constants cannot be

@@ -235,8 +235,9 @@ __global__ void __launch_bounds__(NTA) adjoint_phi_kernel(Box b, float eta, cons
 }
 
 // The same for 16-bit storage: a thread sums the two nodes of one pair-layout
-// word, so that every load is a whole word (with two-byte loads, 256^3 took 87
-// us; the 20 bytes a node take 49 at the copy bandwidth).
+// word, so that every load is a whole word: 60 us at 256^3 (with two-byte loads
+// 87; the 20 bytes a node take 49 at the copy bandwidth).  Bound by the latency
+// of its loads at 85 % of the warps.
 template <typename ST, bool SUM>
 __global__ void __launch_bounds__(TXA / 2 * TYA) adjoint_phi_pair_kernel(Box b, float eta, float inv,
                                                                          const float *__restrict__ f0,
@@ -339,6 +340,8 @@ __global__ void __launch_bounds__(NTA) objective_fold_kernel(const double *__res
 }
 
 // ab[1] = B = sum of the phi kernel's weight sums, ab[3] = scale / B.
+// One block, bound by the latency of its reads: 4 us at 128^3 (cold), on the
+// side stream.
 __global__ void __launch_bounds__(NTA) weight_fold_kernel(const double *__restrict__ partials, int nparts, double scale,
                                                           double *__restrict__ ab)
 {
@@ -353,7 +356,8 @@ __global__ void __launch_bounds__(NTA) weight_fold_kernel(const double *__restri
 }
 
 // ab[0] = A = sum of the march kernel's sums of w u_z, ab[2] = A / B; acc[0] (J)
-// += scale A / B.
+// += scale A / B.  One block, 7 us at 128^3 (cold); with the two it takes the
+// place of a pass over the state's g (42 us).
 __global__ void __launch_bounds__(1024) velocity_fold_kernel(const double *__restrict__ parts, int nparts, double scale,
                                                              double *__restrict__ ab, double *__restrict__ acc)
 {
@@ -539,6 +543,14 @@ struct Geo {
 // (own slots, or in the odd AA layout the reversed slots of x - c_i), and phi
 // and L on the tile plus one node; phi of the plane above is reduced to the
 // sums its stencils need (PlaneSums) once and carried down the march.
+//
+// 256 bytes a node with an FP32 state, 218 with a 16-bit one: 632 and 538 us at
+// 256^3 at the copy bandwidth.  It takes 651 and 652 (DRAM bounds the first,
+// the instructions and the shared-memory pipe of two blocks of 128 registers
+// the second); read straight from global memory, with all seven lambda_f kept,
+// the step took 1055 and 1066.  128^3 FP32 86 us (126 before), 64^3 16 (22).
+// Two blocks, not more: the state's and lambda's two stages of rows take 83 to
+// 95 KB, and one plane ahead hides the latency of a plane.
 template <typename ST, bool ODD, bool LQ>
 __global__ void __launch_bounds__(NTA, 2)
 adjoint_march_kernel(Box b, StepConst c, float phiStar, Quant q, const __grid_constant__ AdjIn a, int tz)

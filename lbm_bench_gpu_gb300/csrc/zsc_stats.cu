@@ -414,7 +414,7 @@ cudaError_t launch_pressure(const Box &b, const lbm_derived &d, const float *mom
 // already owns; this entry point adds nothing to them.
 //
 // The per-block partial sums live in a fixed array in the library's static
-// device memory (57 KiB, one row per resident block, reserved on every GPU that
+// device memory (38 KiB, one row per resident block, reserved on every GPU that
 // loads the library until the process exits).  Boxes of more than 512^3 nodes
 // are rejected (LBM_NOALLOC_MAX_NODES).  Every row the final fold reads is
 // written earlier in the same call, so no part of the array has to be cleared
