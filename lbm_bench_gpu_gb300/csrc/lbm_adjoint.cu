@@ -119,6 +119,8 @@ struct Adjoint {
     // lambda: L, the 19 lg and, when tauPhi is not 1, the seven q (AdjointBuffers)
     float *lam_L[2] = {nullptr, nullptr}, *lam_g[2] = {nullptr, nullptr}, *lam_q[2] = {nullptr, nullptr};
     float *lsrc = nullptr;        // 4 x n
+    lbm::State home;              // the context's state (s^0) while it steps elsewhere (begin)
+    bool away = false;
     double *partials = nullptr, *dgrav = nullptr, *wuz = nullptr, *ab = nullptr, *acc = nullptr;
     unsigned char *slots = nullptr;   // the context's checkpoint pool
     std::vector<Snapshot> snaps;
@@ -169,9 +171,33 @@ struct Adjoint {
 
     unsigned char *slot_ptr(int s) { return slots + (size_t)s * snap_bytes; }
 
+    // The context's own state is s^0, and slot 0 is that state, read in place:
+    // while the adjoint runs, the context steps in the pool's first slot and in
+    // the half of f that s^0 does not use.  So s^0 is copied neither into a
+    // slot nor back (two copies of the state a call), and the context is at s^0
+    // again after an error too.
+    void begin()
+    {
+        home = c->st;
+        away = true;
+        snaps[0] = Snapshot{0, home.f_streamed, home.g_odd_next};
+        const size_t b0 = sizeof(float) * n, bq = c->esz * (lbm::kQf - 1) * n;
+        unsigned char *d = slot_ptr(0);
+        c->st.f0 = reinterpret_cast<float *>(d);
+        c->st.fq = d + b0;
+        c->st.g = d + b0 + bq;
+        c->st.f0_1 = home.f0 + (size_t)(1 - home.f_cur) * n;
+        c->st.fq_1 = static_cast<unsigned char *>(home.fq) + (size_t)(1 - home.f_cur) * bq;
+    }
+
     // the state in slot s, read in place
     lbm::NativeState slot_state(int s)
     {
+        if (s == 0)
+            return lbm::NativeState{c->p.storage, home.f0 + (size_t)home.f_cur * n,
+                                    static_cast<const unsigned char *>(home.fq) +
+                                        (size_t)home.f_cur * (lbm::kQf - 1) * n * c->esz,
+                                    home.g, home.f_streamed, home.g_odd_next};
         const unsigned char *d = slot_ptr(s);
         const size_t b0 = sizeof(float) * n, bq = c->esz * (lbm::kQf - 1) * n;
         return lbm::NativeState{c->p.storage, reinterpret_cast<const float *>(d), d + b0, d + b0 + bq,
@@ -225,23 +251,6 @@ struct Adjoint {
         if (e != cudaSuccess) return cuda_fail(e, "adjoint: host checkpoint restore");
         snaps[s] = hsnaps[h];
         return slot_ev.empty() ? LBM_OK : record(slot_ev[s], c->stream);
-    }
-
-    int restore(int s)
-    {
-        lbm::StepView v = lbm::state_view(c, 0);
-        const unsigned char *d = slot_ptr(s);
-        const size_t b0 = sizeof(float) * n, bq = c->esz * (lbm::kQf - 1) * n, bg = c->esz * lbm::kQg * n;
-        cudaError_t e = cudaMemcpyAsync(c->st.f0, d, b0, cudaMemcpyDeviceToDevice, c->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(const_cast<void *>(v.fq_in), d + b0, bq, cudaMemcpyDeviceToDevice, c->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(c->st.g, d + b0 + bq, bg, cudaMemcpyDeviceToDevice, c->stream);
-        if (e != cudaSuccess) return cuda_fail(e, "adjoint: restore");
-        c->st.f_cur = 0;
-        c->st.f_streamed = snaps[s].f_streamed;
-        c->st.g_odd_next = snaps[s].g_odd_next;
-        c->st.steps = snaps[s].step;
-        return LBM_OK;
     }
 
     int forward(long long nsteps)
@@ -468,7 +477,7 @@ struct Adjoint {
         };
         // sweep: s^{kL} of k = 1 .. K - 2 to host slot k - 1 through b[k & 1]
         for (long long k = 1; k < K && !rc; k++) {
-            rc = forward(L);
+            rc = k == 1 ? advance(0, 0, L) : forward(L);
             if (rc || k == K - 1) continue;
             const int i = (int)(k & 1);
             if (!(rc = wait(c->stream, done[i])) && !(rc = save(b[i], k * L)) && !(rc = rec(saved, c->stream)) &&
@@ -516,7 +525,7 @@ struct Adjoint {
         if (base < 0) return fail(LBM_ESTATE, "adjoint: checkpoint pool exhausted");
         int rc = LBM_OK;
         for (long long k = 1; k < K && !rc; k++) {
-            rc = forward(L);                               // the context: s^{(k - 1) L} -> s^{k L}
+            rc = k == 1 ? advance(0, 0, L) : forward(L);   // the context: s^{(k - 1) L} -> s^{k L}
             if (!rc && k < K - 1) rc = to_host((int)(k - 1), k * L);
         }
         if (!rc) rc = save(base, (K - 1) * L);
@@ -532,6 +541,8 @@ struct Adjoint {
     void release()
     {
         cudaStreamSynchronize(c->stream);
+        if (away) c->st = home;
+        away = false;
         if (side) {
             cudaStreamSynchronize(side);
             cudaStreamDestroy(side);
@@ -660,8 +671,8 @@ extern "C" int lbm_objective(lbm_ctx *c, const lbm_adjoint_opts *o, double *J)
     A.snaps.assign(1, Snapshot());
     cudaError_t e = cudaMemsetAsync(A.acc, 0, sizeof(double) * 2, c->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "lbm_objective: setup");
-    if (!rc) rc = A.save(0, 0);
-    if (!rc) rc = A.forward(A.first_source);
+    if (!rc) A.begin();
+    if (!rc) rc = A.advance(0, 0, A.first_source);
     for (long long k = A.first_source; !rc && k <= o->nsteps; k++) {
         const lbm::NativeState st = A.ctx_state();
         rc = A.prepare(st, A.phi, c->stream);
@@ -675,9 +686,8 @@ extern "C" int lbm_objective(lbm_ctx *c, const lbm_adjoint_opts *o, double *J)
     double acc[2] = {0.0, 0.0};
     if (!rc) {
         e = cudaMemcpyAsync(acc, A.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) rc = A.restore(0);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess && !rc) rc = cuda_fail(e, "lbm_objective: results");
+        if (e != cudaSuccess) rc = cuda_fail(e, "lbm_objective: results");
     }
     A.release();
     if (rc) return rc;
@@ -746,7 +756,8 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
         e = cudaMemsetAsync(A.dgrav, 0, sizeof(double) * lbm::adjoint_dgrav_parts(c->box), c->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "lbm_step_adjoint: setup");
     if (!rc) rc = A.create_streams((int)nslots);
-    if (!rc) rc = A.save(0, 0);
+    if (!rc) A.begin();
+    if (!rc) rc = A.record(A.slot_ev[0], c->stream);
     if (!rc) rc = hslots >= 1 ? A.two_level(hslots, nslots) : A.revolve(0, o->nsteps, 0, (int)(nslots - 1));
     // lambda^0 -> dJ/dphi0 through the initial equilibrium (output in the
     // lsrc buffer, phi as the scratch for the Laplacian's adjoint)
@@ -764,10 +775,8 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
         e = cudaMemcpyAsync(acc, A.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess && out->dJ_dphi0)
             e = cudaMemcpyAsync(out->dJ_dphi0, lphi0, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream);
-        // leave the context at its initial state (its fields were not touched)
-        if (e == cudaSuccess) rc = A.restore(0);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess && !rc) rc = cuda_fail(e, "lbm_step_adjoint: results");
+        if (e != cudaSuccess) rc = cuda_fail(e, "lbm_step_adjoint: results");
     }
     A.release();
     if (rc) return rc;

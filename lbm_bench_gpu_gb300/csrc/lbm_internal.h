@@ -67,6 +67,8 @@ struct State {
     void *fq = nullptr;
     void *g = nullptr;
     float *mom = nullptr;
+    float *f0_1 = nullptr;    // half 1 of f0 / fq where it is not behind half 0
+    void *fq_1 = nullptr;
     int f_cur = 0;            // which half of f0 / fq holds the current values
     bool f_streamed = true;
     bool g_odd_next = false;  // the next step reads g in the AA "odd" layout
@@ -282,14 +284,18 @@ namespace lbm {
 inline StepView state_view(lbm_ctx *c, int in)
 {
     const int out = 1 - in;
-    unsigned char *fq = static_cast<unsigned char *>(c->st.fq);
+    const size_t nf = (size_t)c->box.nf;
+    auto f0 = [&](int half) { return half && c->st.f0_1 ? c->st.f0_1 : c->st.f0 + (size_t)half * nf; };
+    auto fq = [&](int half) -> void * {
+        if (half && c->st.fq_1) return c->st.fq_1;
+        return static_cast<unsigned char *>(c->st.fq) + (size_t)half * (kQf - 1) * nf * c->esz;
+    };
     StepView v;
     v.storage = c->p.storage;
-    const size_t nf = (size_t)c->box.nf;
-    v.f0_in = c->st.f0 + (size_t)in * nf;
-    v.f0_out = c->st.f0 + (size_t)out * nf;
-    v.fq_in = fq + (size_t)in * (kQf - 1) * nf * c->esz;
-    v.fq_out = fq + (size_t)out * (kQf - 1) * nf * c->esz;
+    v.f0_in = f0(in);
+    v.f0_out = f0(out);
+    v.fq_in = fq(in);
+    v.fq_out = fq(out);
     v.g = c->st.g;
     v.g_in = nullptr;
     v.mom = c->st.mom;
