@@ -991,6 +991,8 @@ __global__ void __launch_bounds__(NTA) dgrav_fold_kernel(const double *__restric
 
 // dJ/dphi0 through the initial equilibrium (src/init_f.cu:57-78,
 // src/init_g.cu:69-91), local part; llap receives lambda of the Laplacian.
+// The 19 lambda_g are loaded before anything waits for phi: 256^3 450 -> 275 us
+// (92 bytes a node, 227 us at the copy bandwidth), 128^3 65 -> 38, 64^3 17 -> 8.5.
 __global__ void __launch_bounds__(NTA) init_adjoint_kernel(Box b, float alpha4, float kappa, float phiStarSq,
                                                            float Gamma, const float *__restrict__ phi0,
                                                            const float *__restrict__ lq,
@@ -1003,20 +1005,23 @@ __global__ void __launch_bounds__(NTA) init_adjoint_kernel(Box b, float alpha4, 
     for (int z = blockIdx.z * kPlanes, z_end = min(b.nz, z + kPlanes); z < z_end; z++) {
         const Nb p = neighbourhood(b, x, y, z);
         const unsigned t = p.at(0, 0, 0);
+        float l[kQg];
+#pragma unroll
+        for (int i = 0; i < kQg; i++) l[i] = __ldg(lg + (i * n + t));
+        const float add = L[t];   // lf_i = q_i + L
         float lap, gx, gy, gz;
         stencil19(phi0, p, lap, gx, gy, gz);
         const float ph = phi0[t];
         const float mu = alpha4 * ph * (ph * ph - phiStarSq) - kappa * lap;
-        const float add = L[t];   // lf_i = q_i + L
         const float l0 = lq ? lq[t] + add : add;
         float lfs = 6.f * add, lga = 0.f, lgd = 0.f;
         if (lq)
             for (int i = 1; i < kQf; i++) lfs += lq[i * n + t];
 #pragma unroll
-        for (int i = 1; i < 7; i++) lga += lg[i * n + t];
+        for (int i = 1; i < 7; i++) lga += l[i];
 #pragma unroll
-        for (int i = 7; i < kQg; i++) lgd += lg[i * n + t];
-        const float lg0 = lg[t];
+        for (int i = 7; i < kQg; i++) lgd += l[i];
+        const float lg0 = l[0];
         const float lmu = -3.f * Gamma * l0 + 0.5f * Gamma * lfs - 6.f * kW0 * ph * lg0 + 3.f * kW1 * ph * lga
                           + 3.f * kW2 * ph * lgd;
         float lphi = l0 - 6.f * kW0 * mu * lg0 + 3.f * kW1 * mu * lga + 3.f * kW2 * mu * lgd;
