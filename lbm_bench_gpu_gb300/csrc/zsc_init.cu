@@ -162,6 +162,17 @@ __device__ __forceinline__ Eq equilibrium_at(const Box &b, const EqConst &c, con
 // that and its conversion took 700, 289 and 498.
 constexpr int EQZ = 4;
 
+// The block's tile and first plane.  The grid has one dimension: a box's y or z
+// may need more blocks than the 65535 of a grid's second and third.
+struct EqTile {
+    int bx, by, z0;
+};
+__device__ __forceinline__ EqTile eq_tile(const Box &b)
+{
+    const unsigned ntx = (unsigned)b.nx / 32u, nty = (unsigned)b.ny / 8u, t = blockIdx.x;
+    return EqTile{(int)(t % ntx), (int)(t / ntx % nty), (int)(t / (ntx * nty)) * EQZ};
+}
+
 // FP32 storage: the streamed natural layout is the equilibrium itself.
 __global__ void __launch_bounds__(256) equilibrium_kernel(Box b, EqConst c, const float *__restrict__ phi,
                                                           const float *__restrict__ rho,
@@ -169,9 +180,10 @@ __global__ void __launch_bounds__(256) equilibrium_kernel(Box b, EqConst c, cons
                                                           const float *__restrict__ ghost_hi, float *__restrict__ f0,
                                                           float *__restrict__ fq, float *__restrict__ g)
 {
-    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    const EqTile tile = eq_tile(b);
+    const int i = tile.bx * 32 + threadIdx.x, j = tile.by * 8 + threadIdx.y;
 #pragma unroll 1
-    for (int k = blockIdx.z * EQZ, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
+    for (int k = tile.z0, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
         const Eq e = equilibrium_at(b, c, phi, rho, ghost_lo, ghost_hi, i, j, k);
         const size_t t = (size_t)k * b.nxy + j * b.nx + i;
         f0[t] = e.f0;
@@ -196,9 +208,10 @@ __global__ void __launch_bounds__(128) equilibrium_store_kernel(Box b, EqConst c
                                                                 ST *__restrict__ g)
 {
     using T2 = typename Fmt<ST>::T2;
-    const int w = blockIdx.x * 16 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    const EqTile tile = eq_tile(b);
+    const int w = tile.bx * 16 + threadIdx.x, j = tile.by * 8 + threadIdx.y;
 #pragma unroll 1
-    for (int k = blockIdx.z * EQZ, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
+    for (int k = tile.z0, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
         const Eq a = equilibrium_at(b, c, phi, rho, ghost_lo, ghost_hi, w, j, k);
         const Eq d = equilibrium_at(b, c, phi, rho, ghost_lo, ghost_hi, w + b.nx / 2, j, k);
         const size_t t = (size_t)k * b.nxy + j * b.nx + 2 * w;   // the word's first element
@@ -227,10 +240,11 @@ __global__ void __launch_bounds__(256) equilibrium_maxabs_kernel(Box b, EqConst 
                                                                  unsigned *__restrict__ out_bits)
 {
     __shared__ unsigned red[8][5];
-    const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    const EqTile tile = eq_tile(b);
+    const int i = tile.bx * 32 + threadIdx.x, j = tile.by * 8 + threadIdx.y;
     float m[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-    for (int k = blockIdx.z * EQZ, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
+    for (int k = tile.z0, k_end = min(b.nz, k + EQZ); k < k_end; k++) {
         const Eq e = equilibrium_at(b, c, phi, rho, ghost_lo, ghost_hi, i, j, k);
         m[0] = fmaxf(m[0], fabsf(e.f0));
         m[1] = fmaxf(m[1], fabsf(e.f1));
@@ -283,9 +297,9 @@ cudaError_t launch_bubble_phi(const Box &b, const float *bubbles_dev, int nbubbl
 
 namespace {
 EqConst eq_const(const lbm_derived &d, float Gamma) { return EqConst{d.alpha4, d.kappa, d.phiStarSq, Gamma}; }
-dim3 eq_grid(const Box &b)
+unsigned eq_grid(const Box &b)
 {
-    return dim3((unsigned)(b.nx / 32), (unsigned)(b.ny / 8), (unsigned)((b.nz + EQZ - 1) / EQZ));
+    return (unsigned)(b.nx / 32) * (unsigned)(b.ny / 8) * (unsigned)((b.nz + EQZ - 1) / EQZ);
 }
 }  // namespace
 
