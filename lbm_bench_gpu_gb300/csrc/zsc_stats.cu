@@ -5,8 +5,8 @@
 // compensated float sums (a float pair hi + lo updated with Knuth's two-sum,
 // products split exactly with an FMA), which hold ~48 bits like an FP64 sum
 // at FP32 throughput (GB300's FP64 rate is a small fraction of its FP32 rate);
-// the same pairs through the warp reduction, FP64 across warps and blocks in
-// a fixed order (deterministic for a given box).
+// FP64 across threads, warps and blocks in a fixed order (deterministic for a
+// given box).
 //
 // Partial / result layout (doubles):
 //   0 max |u|^2 (compat)    1 #phi>=0 (compat)   2..4 sum u over phi>=0 (compat)
@@ -58,16 +58,8 @@ struct Sum2 {
         add(p);
         lo = __fadd_rn(lo, fmaf(a, b, -p));
     }
+    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
-
-// (h, l) += (h2, l2) of float pairs
-__device__ __forceinline__ void pair_add(float &h, float &l, float h2, float l2)
-{
-    const float s = __fadd_rn(h, h2);
-    const float bp = __fsub_rn(s, h);
-    l = __fadd_rn(__fadd_rn(l, l2), __fadd_rn(__fsub_rn(h, __fsub_rn(s, bp)), __fsub_rn(h2, bp)));
-    h = s;
-}
 
 // What a node needs of one plane of phi for the 19-point Laplacian, the
 // gradient and its own value: with f4 = e + w + n + s and e4 the four diagonal
@@ -238,30 +230,27 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
         }
     }
 
-    // The block's sums.  Ten float pairs per thread through a recursive halving
-    // over the warp (16 value slots: after offsets 16, 8, 4, 2 a lane holds one
-    // value of 16 lanes, then offset 1), 16 pair additions per thread instead of
-    // 50, and no FP64 until one value per warp is left.
-    float h[16], l[16];
+    // The block's sums: each thread's ten float pairs go to FP64 and through a
+    // recursive halving over the warp (16 value slots: after offsets 16, 8, 4, 2
+    // a lane holds one value of 16 lanes, then offset 1), 16 FP64 additions per
+    // thread in place of 50.  Float pairs through the warp took 11.5, 16.8 and
+    // 35.2 us at 32^3, 64^3 and 128^3 (now 13.6, 22.9 and 38.0), but kept 48 bits
+    // and left FP32's range where the FP64 sums of the threads' pairs do not.
+    double d[16];
     const Sum2 *const all[10] = {&s_ux, &s_uy, &s_uz, &s_in, &s_out, &s_phi, &s_rho, &s_mx, &s_my, &s_mz};
 #pragma unroll
-    for (int v = 0; v < 16; v++) {
-        h[v] = v < 10 ? all[v < 10 ? v : 0]->hi : 0.f;
-        l[v] = v < 10 ? all[v < 10 ? v : 0]->lo : 0.f;
-    }
+    for (int v = 0; v < 16; v++) d[v] = v < 10 ? all[v < 10 ? v : 0]->value() : 0.0;
 #pragma unroll
     for (int half = 8; half >= 1; half >>= 1) {
         const bool up = lane & (2 * half);
 #pragma unroll
         for (int v = 0; v < half; v++) {
-            const float gh = __shfl_xor_sync(0xffffffffu, up ? h[v] : h[v + half], 2 * half);
-            const float gl = __shfl_xor_sync(0xffffffffu, up ? l[v] : l[v + half], 2 * half);
-            h[v] = up ? h[v + half] : h[v];
-            l[v] = up ? l[v + half] : l[v];
-            pair_add(h[v], l[v], gh, gl);
+            if (v >= 10) continue;   // (both slots of the pair are empty)
+            const double other = __shfl_xor_sync(0xffffffffu, up ? d[v] : d[v + half], 2 * half);
+            d[v] = (up ? d[v + half] : d[v]) + other;
         }
     }
-    pair_add(h[0], l[0], __shfl_xor_sync(0xffffffffu, h[0], 1), __shfl_xor_sync(0xffffffffu, l[0], 1));
+    d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
     cnt_in = __reduce_add_sync(0xffffffffu, cnt_in);
     cnt_all = __reduce_add_sync(0xffffffffu, cnt_all);
     cnt_bad = __reduce_add_sync(0xffffffffu, cnt_bad);
@@ -270,7 +259,7 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
     const unsigned mx_a = __reduce_max_sync(0xffffffffu, __float_as_uint(umax_all));
     __shared__ double red[kThreads / 32][kStatsValues];
     // lane 2 v (of each pair of lanes) holds sum v: result entries 2..6 and 7..11
-    if ((lane & 1) == 0 && lane < 20) red[warp][2 + (lane >> 1)] = (double)h[0] + (double)l[0];
+    if ((lane & 1) == 0 && lane < 20) red[warp][2 + (lane >> 1)] = d[0];
     if (lane == 31) {
         red[warp][0] = __uint_as_float(mx_c);
         red[warp][1] = cnt_in;
