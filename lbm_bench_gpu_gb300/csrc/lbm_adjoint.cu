@@ -686,8 +686,9 @@ extern "C" int lbm_objective(lbm_ctx *c, const lbm_adjoint_opts *o, double *J)
     double acc[2] = {0.0, 0.0};
     if (!rc) {
         e = cudaMemcpyAsync(acc, A.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = lbm::queue_flag(c);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) rc = cuda_fail(e, "lbm_objective: results");
+        rc = e == cudaSuccess ? lbm::flag_status(c) : cuda_fail(e, "lbm_objective: results");
     }
     A.release();
     if (rc) return rc;
@@ -775,8 +776,9 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
         e = cudaMemcpyAsync(acc, A.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess && out->dJ_dphi0)
             e = cudaMemcpyAsync(out->dJ_dphi0, lphi0, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = lbm::queue_flag(c);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) rc = cuda_fail(e, "lbm_step_adjoint: results");
+        rc = e == cudaSuccess ? lbm::flag_status(c) : cuda_fail(e, "lbm_step_adjoint: results");
     }
     A.release();
     if (rc) return rc;

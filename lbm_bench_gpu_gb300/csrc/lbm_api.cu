@@ -270,11 +270,15 @@ namespace lbm {
 // build found a global index outside its field (LBM_ECUDA).
 int device_error(lbm_ctx *c)
 {
-    // on the context's stream, after the kernels that set it
-    LBM_CUDA(cudaMemcpyAsync(c->result_host + kStatsValues, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream),
-             "error flag");
+    LBM_CUDA(queue_flag(c), "error flag");
     LBM_CUDA(cudaStreamSynchronize(c->stream), "error flag");
     return flag_status(c);
+}
+
+cudaError_t queue_flag(lbm_ctx *c)
+{
+    // on the context's stream, after the kernels that set it
+    return cudaMemcpyAsync(c->result_host + kStatsValues, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
 }
 
 int flag_status(const lbm_ctx *c)
@@ -791,6 +795,19 @@ extern "C" int lbm_wait_selftest(lbm_ctx *c)
     if (rc == LBM_OK) return fail(LBM_ESTATE, "lbm_wait_selftest: the bounded wait did not give up");
     return rc;
 }
+
+#if defined(ZSC_CHECKED) && ZSC_CHECKED
+// Checked build only: set the kernels' error flag, as a step kernel that gave
+// up would, for the tests of the calls that report it.
+extern "C" int lbm_checked_raise_flag(lbm_ctx *c, int flag)
+{
+    if (!c) return fail(LBM_EINVAL, "context is NULL");
+    LBM_ON_DEVICE(c->p.device);
+    LBM_CUDA(cudaMemcpyAsync(c->err, &flag, sizeof(int), cudaMemcpyHostToDevice, c->stream), "error flag");
+    LBM_CUDA(cudaStreamSynchronize(c->stream), "error flag");
+    return LBM_OK;
+}
+#endif
 
 extern "C" void lbm_destroy(lbm_ctx *c)
 {
