@@ -153,7 +153,7 @@ inline Depth march_depth(long long tiles, int planes, int sms, int per_sm, const
     }
     return best;
 }
-int sm_count();   // SMs of the current device (read once per process)
+int sm_count();   // SMs of the current device
 
 void set_error(const std::string &msg);
 const std::string &last_error();

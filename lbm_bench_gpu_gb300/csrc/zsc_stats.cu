@@ -413,6 +413,8 @@ cudaError_t launch_pressure(const Box &b, const lbm_derived &d, const float *mom
 // ---------------------------------------------------------------------------
 #include <mutex>
 
+#include "per_device.h"
+
 namespace lbm {
 namespace {
 
@@ -420,7 +422,6 @@ constexpr long long kNoAllocMaxNodes = LBM_NOALLOC_MAX_NODES;
 
 static __device__ __align__(256) double g_noalloc_partials[kMaxBlocks * kStatsValues];
 
-constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mutex;
 double *g_noalloc_ptr[kMaxDevices] = {};
 

@@ -56,6 +56,7 @@
 #include <utility>
 
 #include "lattice.cuh"
+#include "per_device.h"
 
 namespace lbm {
 namespace {
@@ -1234,19 +1235,26 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
     }
 }
 
+// The shared-memory limit and carveout of an instance belong to the device's
+// copy of it: set once per device (which must be current).
 template <typename ST, bool DEEP, bool S, bool O, bool T, bool Z>
-cudaError_t configure()
+cudaError_t configure(int device)
 {
-    static bool done = false;   // per template instance, per process
-    if (done) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(zsc_step_kernel<ST, DEEP, S, O, T, Z>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Geo<ST, DEEP>::SMEM);
-    // all of the unified L1 / shared storage as shared memory: the resident
-    // blocks per SM the launch bounds ask for need it
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(zsc_step_kernel<ST, DEEP, S, O, T, Z>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess) done = true;
+    static PerDevice<int> set;
+    cudaError_t e = cudaSuccess;
+    int unused;
+    set.get(device, unused, [&](int &v) {
+        v = 1;
+        e = cudaFuncSetAttribute(zsc_step_kernel<ST, DEEP, S, O, T, Z>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 Geo<ST, DEEP>::SMEM);
+        // all of the unified L1 / shared storage as shared memory: the resident
+        // blocks per SM the launch bounds ask for need it
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(zsc_step_kernel<ST, DEEP, S, O, T, Z>,
+                                     cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     (int)cudaSharedmemCarveoutMaxShared);
+        return e == cudaSuccess;
+    });
     return e;
 }
 
@@ -1350,35 +1358,39 @@ struct Plan {
 };
 
 template <typename ST, bool DEEP>
-int resident_blocks()   // per SM; per instance, per process
+int resident_blocks(int device)   // per SM, of the current device
 {
-    static const int blocks = [] {
-        int n = 0;
-        configure<ST, DEEP, false, false, false, false>();   // its shared memory above the default limit
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, zsc_step_kernel<ST, DEEP, false, false, false, false>,
-                                                      threads_of<ST>(), Geo<ST, DEEP>::SMEM);
-        return std::max(1, std::min(n, Geo<ST, DEEP>::kMinBlocks));
-    }();
+    static PerDevice<int> found;
+    int blocks = 1;
+    found.get(device, blocks, [&](int &n) {
+        // its shared memory above the default limit first
+        if (configure<ST, DEEP, false, false, false, false>(device) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, zsc_step_kernel<ST, DEEP, false, false, false, false>,
+                                                          threads_of<ST>(), Geo<ST, DEEP>::SMEM) != cudaSuccess)
+            return false;
+        n = std::max(1, std::min(n, Geo<ST, DEEP>::kMinBlocks));
+        return true;
+    });
     return blocks;
 }
 
 template <typename ST>
-Plan choose_plan(const Box &b)
+Plan choose_plan(const Box &b, int device)
 {
-    // a thread's steps are mostly on one box: its last answer is kept
-    static thread_local int last[3] = {0, 0, 0};
+    // a thread's steps are mostly on one box of one device: its last answer is kept
+    static thread_local int last[4] = {0, 0, 0, -1};
     static thread_local Plan plan = {false, 1};
-    if (last[0] == b.nx && last[1] == b.ny && last[2] == b.nz) return plan;
+    if (last[0] == b.nx && last[1] == b.ny && last[2] == b.nz && last[3] == device) return plan;
     const long long tiles = (long long)(b.nx / TX) * (b.ny / TY);
     const int sms = sm_count();
     if constexpr (sizeof(ST) == 2) {
         constexpr MarchCost cost = {22, 1.45, {0.0, 1.0, 1.33, 1.97, 2.10}, {0.30, 0.79, 1.22, 1.62, 1.77}};
-        plan.tz = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), cost).tz;
+        plan.tz = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(device), cost).tz;
     } else {
         constexpr MarchCost deep = {22, 1.16, {0.0, 1.0, 1.50}, {0.30, 0.97, 1.54}};
         constexpr MarchCost dense = {24, 3.19, {0.0, 1.0, 1.42, 1.58}, {1.16, 1.17, 1.08, 1.41}};
-        const Depth d = march_depth(tiles, b.nz, sms, resident_blocks<ST, true>(), deep);
-        const Depth e = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(), dense);
+        const Depth d = march_depth(tiles, b.nz, sms, resident_blocks<ST, true>(device), deep);
+        const Depth e = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(device), dense);
         // the two costs in one unit
         plan.deep = d.cost <= 1.12 * e.cost - 2.25;
         plan.tz = plan.deep ? d.tz : e.tz;
@@ -1386,6 +1398,7 @@ Plan choose_plan(const Box &b)
     last[0] = b.nx;
     last[1] = b.ny;
     last[2] = b.nz;
+    last[3] = device;
     return plan;
 }
 
@@ -1442,7 +1455,10 @@ cudaError_t launch_typed(const Box &b, const StepConst &c, const Quant &q, const
     if (tma && use_tma_f<ST>()) tma = encode_f_maps<ST>(b, P.f0in, fin, &f0map, &fqmap);
     Box range = b;   // the chunk depth for the planes this launch covers
     range.nz = zhi - zlo;
-    const Plan plan = choose_plan<ST>(range);
+    int device = 0;
+    const cudaError_t ed = cudaGetDevice(&device);
+    if (ed != cudaSuccess) return ed;
+    const Plan plan = choose_plan<ST>(range, device);
     const int tz = plan.tz;
     const int nchunks = (range.nz + tz - 1) / tz;
     const unsigned nblocks = (unsigned)((b.nx / TX) * (b.ny / TY) * nchunks);
@@ -1452,7 +1468,7 @@ cudaError_t launch_typed(const Box &b, const StepConst &c, const Quant &q, const
     auto launch = [&](auto deep, auto streamed, auto is_odd, auto with_tma) -> cudaError_t {
         constexpr bool D = decltype(deep)::value, S = decltype(streamed)::value, O = decltype(is_odd)::value,
                        T = decltype(with_tma)::value;
-        const cudaError_t e = configure<ST, D, S, O, T, ZG>();
+        const cudaError_t e = configure<ST, D, S, O, T, ZG>(device);
         if (e != cudaSuccess) return e;
         return launch_step_kernel(zsc_step_kernel<ST, D, S, O, T, ZG>, nblocks, block, Geo<ST, D>::SMEM, s, P, kb, c,
                                   m, tz, wm, zlo, zhi, gmap, f0map, fqmap);
@@ -1483,13 +1499,15 @@ cudaError_t launch_typed(const Box &b, const StepConst &c, const Quant &q, const
 
 int sm_count()
 {
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return std::max(1, n);
-    }();
-    return sms;
+    static PerDevice<int> found;
+    int device = -1, sms = 1;
+    if (cudaGetDevice(&device) != cudaSuccess) return 1;
+    found.get(device, sms, [&](int &n) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return false;
+        n = std::max(1, n);
+        return true;
+    });
+    return std::max(1, sms);
 }
 
 cudaError_t launch_wait_selftest(int *err, cudaStream_t s)
