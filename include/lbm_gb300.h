@@ -191,7 +191,7 @@ typedef struct lbm_adjoint_opts {
 typedef struct lbm_adjoint_out {
     double J;                 /* objective (FP64 accumulation) */
     double dJ_dgrav;          /* dJ / d grav (FP64 accumulation) */
-    float *dJ_dphi0;          /* caller's nx*ny*nz host buffer for dJ / d phi0 (undefined unless LBM_OK), or NULL */
+    float *dJ_dphi0;          /* caller's nx*ny*nz host buffer for dJ / d phi0, or NULL */
     int slots;                /* checkpoints held, the initial state included */
     long long forward_steps;  /* forward steps run, recomputation included */
     long long adjoint_steps;  /* = nsteps */
