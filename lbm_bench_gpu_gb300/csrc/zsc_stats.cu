@@ -22,7 +22,8 @@ namespace lbm {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int SX = 32, SY = 2 * kThreads / 32;   // columns of a block's tile (two rows a thread)
+constexpr int kWarps = kThreads / 32;
+constexpr int SX = 32;                       // columns of a warp, two rows a thread
 constexpr int kBlocksPerSm = 2;              // resident blocks the launch bounds ask for (128 registers)
 constexpr int kMaxBlocks = 152 * kBlocksPerSm;
 constexpr float kInv6 = 0.16666666666666666667f;
@@ -72,10 +73,12 @@ struct Plane {
     float mid, gx, gy;        // e4 + 2 f4 - 24 c; own-plane parts of the x and y gradient
 };
 
-// One block: eight warps, a 32 x 16 tile of columns; item `it` is one tile and
-// a run of kz planes, which every thread marches at its two columns (rows y and
-// y + 1, which share 6 of the 18 values of phi they need).  Plane z + 2 of phi
-// and plane z + 1 of the other fields are loaded while plane z is computed.
+// One block: eight warps, a 32 x 2 WY tile of columns (WY = 8, fewer in a box
+// of fewer rows, whose other warps take the next runs of planes); item `it` is
+// one tile and 8 / WY runs of kz planes, one of which every thread marches at
+// its two columns (rows y and y + 1, which share 6 of the 18 values of phi they
+// need).  Plane z + 2 of phi and plane z + 1 of the other fields are loaded
+// while plane z is computed.
 // |u|^2 and the pressure are evaluated in float as the reference does
 // (src/stats.c:45, src/logsave.c:94-137); sums are compensated, counts exact.
 // phi_lo / phi_hi: the phi planes just below and above a z-slab (NULL for a
@@ -86,13 +89,14 @@ struct Plane {
 // 256^3 at the copy bandwidth, its 100 FP32 instructions (51 of them in the
 // compensated sums of a node outside the bubbles) 45 us at one per cycle and
 // scheduler, of about 180 in all.  Measured, lbm_stats_noalloc with its fold,
-// 256^3: 368 -> 127 us, 128^3 36.9, 32^3 78 -> 12 us, against one thread per
+// 256^3: 368 -> 124 us, 128^3 38, 32^3 78 -> 14 us, against one thread per
 // node reading 19 points, with 15 FP64 values per thread reduced over the block
 // (FP64 runs at a 60th of the FP32 rate: that reduction was most of a small
 // box's time).  Also measured at 256^3: one column a thread 145 us (223
 // instructions a node), two nodes a thread in f32x2 147 (the packed operations
 // issue at half rate and their constants take register pairs), the planes
 // staged by cp.async 133.
+template <int WY>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
 stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__restrict__ rho,
              const float *__restrict__ ux, const float *__restrict__ uy, const float *__restrict__ uz,
@@ -100,16 +104,16 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
              int items)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ntx = (b.nx + SX - 1) / SX, nty = (b.ny + SY - 1) / SY;
+    const int ntx = (b.nx + SX - 1) / SX, nty = (b.ny + 2 * WY - 1) / (2 * WY);
     const unsigned nx = (unsigned)b.nx, nxy = (unsigned)b.nxy;
     Sum2 s_phi, s_rho, s_mx, s_my, s_mz, s_ux, s_uy, s_uz, s_in, s_out;
     unsigned cnt_in = 0, cnt_all = 0, cnt_bad = 0;
     float umax_c = 0.f, umax_all = 0.f;
 
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int tile = it % (ntx * nty), z0 = (it / (ntx * nty)) * kz;
-        const int x = (tile % ntx) * SX + lane, y = (tile / ntx) * SY + 2 * warp;
-        if (x >= b.nx || y >= b.ny) continue;   // (no barrier in this loop)
+        const int tile = it % (ntx * nty), z0 = (it / (ntx * nty) * (kWarps / WY) + warp / WY) * kz;
+        const int x = (tile % ntx) * SX + lane, y = (tile / ntx) * 2 * WY + 2 * (warp % WY);
+        if (x >= b.nx || y >= b.ny || z0 >= b.nz) continue;   // (no barrier in this loop)
         const bool two = y + 1 < b.ny;          // the row y + 1 is in the box
         const bool x_in = x >= 1 && x <= b.nx - 2;
         const bool in_a = x_in && y >= 1 && y <= b.ny - 2, in_b = x_in && y + 1 <= b.ny - 2;
@@ -257,7 +261,7 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
     // |u|^2 >= 0: floats order like their bits
     const unsigned mx_c = __reduce_max_sync(0xffffffffu, __float_as_uint(umax_c));
     const unsigned mx_a = __reduce_max_sync(0xffffffffu, __float_as_uint(umax_all));
-    __shared__ double red[kThreads / 32][kStatsValues];
+    __shared__ double red[kWarps][kStatsValues];
     // lane 2 v (of each pair of lanes) holds sum v: result entries 2..6 and 7..11
     if ((lane & 1) == 0 && lane < 20) red[warp][2 + (lane >> 1)] = d[0];
     if (lane == 31) {
@@ -272,7 +276,7 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
     if (threadIdx.x < kStatsValues) {
         const int v = threadIdx.x;
         double s = red[0][v];
-        for (int w = 1; w < kThreads / 32; w++) s = is_max(v) ? fmax(s, red[w][v]) : s + red[w][v];
+        for (int w = 1; w < kWarps; w++) s = is_max(v) ? fmax(s, red[w][v]) : s + red[w][v];
         partials[(size_t)blockIdx.x * kStatsValues + v] = s;
     }
 }
@@ -336,28 +340,40 @@ __global__ void __launch_bounds__(kThreads) pressure_kernel(Box b, StatsConst c,
     }
 }
 
-// How a box is cut: items of one tile and kz planes, the deepest (up to 16)
-// that still give every resident block four of them, so that uneven items
-// even out; a small box takes single planes.
+// How a box is cut: wy warps of a block side by side in y (8, 4 or 2, no more
+// than the box's row pairs fill), and items of one tile and 8 / wy runs of
+// kz planes, the deepest (up to 16) that still give every resident block four of
+// them, so that uneven items even out; a small box takes single planes.  With
+// all eight warps in y a box of 3 or 4 rows used two of them: 2048 x 3 x 2048
+// 371 -> 128 us, 4096 x 4 x 1024 380 -> 136, 5 x 5 x 100000 251 -> 177
+// (before the marching columns 216, 271 and 2652).
 struct Cut {
-    int kz, items, blocks;
+    int wy, kz, items, blocks;
 };
 Cut stats_cut(const Box &b)
 {
-    const long long tiles = (long long)((b.nx + SX - 1) / SX) * ((b.ny + SY - 1) / SY);
-    auto items_of = [&](int kz) { return tiles * ((b.nz + kz - 1) / kz); };
+    int wy = kWarps;
+    while (wy > 2 && 2 * (wy / 2) >= b.ny) wy /= 2;
+    const int runs = kWarps / wy;
+    const long long tiles = (long long)((b.nx + SX - 1) / SX) * ((b.ny + 2 * wy - 1) / (2 * wy));
+    auto items_of = [&](int kz) { return tiles * ((b.nz + kz * runs - 1) / (kz * runs)); };
     int kz = 16;
     while (kz > 1 && items_of(kz) < 4 * kMaxBlocks) kz /= 2;
     const long long items = items_of(kz);
-    return Cut{kz, (int)items, (int)std::min<long long>(items, kMaxBlocks)};
+    return Cut{wy, kz, (int)items, (int)std::min<long long>(items, kMaxBlocks)};
 }
 
 cudaError_t launch_stats_kernels(const Box &b, const StatsConst &c, const float *const f[5], const float *phi_lo,
                                  const float *phi_hi, double *partials, double *result, cudaStream_t s)
 {
     const Cut k = stats_cut(b);
-    stats_kernel<<<(unsigned)k.blocks, kThreads, 0, s>>>(b, c, f[0], f[1], f[2], f[3], f[4], partials, phi_lo,
-                                                         phi_hi, k.kz, k.items);
+    auto launch = [&](auto kernel) {
+        kernel<<<(unsigned)k.blocks, kThreads, 0, s>>>(b, c, f[0], f[1], f[2], f[3], f[4], partials, phi_lo, phi_hi,
+                                                       k.kz, k.items);
+    };
+    if (k.wy == 8) launch(stats_kernel<8>);
+    else if (k.wy == 4) launch(stats_kernel<4>);
+    else launch(stats_kernel<2>);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     fold_kernel<<<1, kThreads, 0, s>>>(partials, k.blocks, result);

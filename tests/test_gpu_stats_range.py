@@ -75,3 +75,15 @@ def _node_pressure(p, fields, at):
     lap, g = lap / 6.0, g / 12.0
     star = float(d.phiStarSq)
     return float(d.alpha) * (c**2 * (3 * c**2 - 2 * star) - star**2) - float(d.kappa) * (c * lap - 0.5 * g @ g) + rho / 3.0
+
+
+# Boxes of few rows: a block's warps share its tile's rows and several runs of planes.
+@pytest.mark.parametrize("shape", [(70, 3, 50), (40, 4, 37), (33, 5, 19), (64, 8, 70), (5, 6, 333), (65, 8, 3),
+                                   (32, 3, 3), (700, 4, 1100)])
+def test_statistics_of_thin_boxes(lib, shape):
+    from lbm_bench_gpu_gb300 import capi
+    p = capi.make_params(*shape, **PHYS)
+    fields = _fields(shape, 9)
+    got = _raw(lib, p, fields)
+    want, tol = _want(p, fields)
+    assert np.all(np.abs(got - want) <= tol), (got, want, tol)
