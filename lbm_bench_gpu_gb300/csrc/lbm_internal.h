@@ -7,6 +7,7 @@
 #include <string>
 
 #include "lbm_gb300.h"
+#include "march_plan.h"
 #include <nvtx3/nvToolsExt.h>   // header-only; no-ops unless a profiler is attached
 
 namespace lbm {
@@ -115,44 +116,6 @@ struct AdjointBuffers {
     double *acc;                       // acc[0] += its term of J (window steps)
 };
 
-// Planes per block of a kernel whose blocks march `planes` planes on `tiles`
-// column tiles, per_sm of them resident on each of sms SMs.  A block's time is
-// about (tz + prologue) plane-times, and r blocks that share an SM slow each
-// other down by share[r] (less than r: a lone block is bound by its own
-// latencies).  The launch takes as many full rounds of resident blocks as there
-// are, then a last, partly filled one, which overlaps the end of the others:
-// x blocks per SM of it add tail[x] (interpolated; tail[0] is what the first of
-// them adds) of their time, which is that of the last, shorter run of planes
-// if there are no others among them.  The depth up to `deepest` that minimises
-// the sum is taken; cost is in plane-times of a lone block.
-struct MarchCost {
-    int deepest;
-    double prologue;
-    double share[9], tail[9];
-};
-struct Depth {
-    int tz;
-    double cost;
-};
-inline Depth march_depth(long long tiles, int planes, int sms, int per_sm, const MarchCost &m)
-{
-    const long long slots = (long long)sms * per_sm;
-    Depth best = {1, -1.0};
-    for (int tz = 1; tz <= m.deepest; tz++) {
-        const int runs = (planes + tz - 1) / tz, last = planes - (runs - 1) * tz;
-        const long long blocks = tiles * runs, full = blocks / slots, rest = blocks % slots;
-        double cost = (double)full * m.share[per_sm] * (tz + m.prologue);
-        if (full == 0) {
-            cost = m.share[(rest + sms - 1) / sms] * (tz + m.prologue);
-        } else if (rest > 0) {
-            const long long i = rest / sms;   // < per_sm
-            const double t = m.tail[i] + (m.tail[i + 1] - m.tail[i]) * (double)(rest - i * sms) / (double)sms;
-            cost += t * ((rest <= tiles ? last : tz) + m.prologue);
-        }
-        if (best.cost < 0.0 || cost < best.cost) best = {tz, cost};
-    }
-    return best;
-}
 int sm_count();   // SMs of the current device
 
 void set_error(const std::string &msg);

@@ -137,8 +137,8 @@ struct Dir {
 //         g rows follow once the current ones are in registers, and the third
 //         block covers the shorter flight.
 // FP32, deep -> dense: 256^3 610 -> 600 us a step, 128^3 82.9 -> 80.0, 160 x 104
-// x 93 64.4 -> 59.9; but 64^3 13.5 -> 14.6, 32^3 3.8 -> 4.2: choose_plan takes
-// one by the box.  (16-bit storage with one g stage and five blocks of 96
+// x 93 64.4 -> 59.9; but 64^3 13.5 -> 14.6, 32^3 3.8 -> 4.2: step_plan_fp32 takes
+// one by the box.  (The dense odd kernel spills 16 bytes, a z-slab's 48.)  (16-bit storage with one g stage and five blocks of 96
 // registers spills and is slower: 256^3 346 -> 400 us.)
 // g rows carry one extra chunk (an odd step's shifted rows need it on one side
 // only).
@@ -827,7 +827,7 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
         }
         // with one g stage plane z + 1's rows follow once every thread holds
         // its g values of plane z in registers
-        auto g_is_read = [&]() {
+        auto g_is_read = [&]() {   // (FP32 only: 16-bit storage has two)
             if constexpr (NG == 1) {
                 __syncthreads();
                 if (j + 1 < nzc) issue_g(z + 1, 0);
@@ -1104,7 +1104,6 @@ zsc_step_kernel(const StepPtrs<ST> P, const StepBox b, const StepConst c, const 
                     g[i] = Fm::load2(Fm::perm2(v, kCx(i) > 0 ? sel_l : sel_r));
                 }
             }
-            g_is_read();
 
             // moments (stored units: rho = g_inv sum + sum of shifts)
             float2 rho = g[0];
@@ -1331,32 +1330,6 @@ bool encode_f_maps(const Box &b, const float *f0, const ST *fq, CUtensorMap *f0m
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Staging geometry and planes per block of a launch.
-//
-// The depth comes from march_depth.  Its constants were fitted to forced depths
-// 1 .. 64 on 33 boxes from 32^3 to 512^3, 15 of them drawn at random: the depth
-// taken is within 0.4% of the best on average (4.0% at most) for the 16-bit
-// kernel, 0.2% (1.7%) for the dense one and 0.5% (7.4%) for the deep one.  No
-// large box gained from more than 24 planes (their blocks drift apart, and
-// neighbouring tiles then share fewer halo rows in L2): 512^3 FP16 2777 us at
-// 22 planes, 2831 at 37, 3069 at 64; FP32 4814, 4862, 4936.
-//
-// FP32 takes the geometry with the lower estimate: on each of the 17 boxes of
-// up to 1.2 million nodes the faster one of the two at their depths.  Deep /
-// dense in us: 64^3 13.4 / 14.5, 128 x 64 x 44 15.8 / 17.6, 96 x 64 x 80 20.6 /
-// 20.8; 32 x 96 x 110 14.6 / 13.5, 128 x 112 x 37 22.6 / 20.9, 96 x 88 x 100
-// 33.6 / 32.7.  Larger boxes take the dense one.
-//
-// (Depth of at least 4 planes and a cost without the share of an SM, before ->
-// now: 32^3 FP32 8.2 -> 3.8 us, 32 x 64 x 48 FP32 12.1 -> 6.6, FP16 16.0 -> 6.7;
-// 64^3 FP16 16.9 -> 10.9; 160 x 104 x 93 FP16 41.8 -> 38.3; 192^3 FP16 171 -> 159.
-// The 16-bit figures are those of the kernel before its byte offsets, with which
-// these boxes take 2 to 4 % less: 192^3 153, 512^3 2692.)
-struct Plan {
-    bool deep;
-    int tz;
-};
-
 template <typename ST, bool DEEP>
 int resident_blocks(int device)   // per SM, of the current device
 {
@@ -1374,31 +1347,31 @@ int resident_blocks(int device)   // per SM, of the current device
     return blocks;
 }
 
+// The plan of a launch over b's planes (march_plan.h).
 template <typename ST>
-Plan choose_plan(const Box &b, int device)
+StepPlan choose_plan(const Box &b, int device)
 {
-    // a thread's steps are mostly on one box of one device: its last answer is kept
-    static thread_local int last[4] = {0, 0, 0, -1};
-    static thread_local Plan plan = {false, 1};
-    if (last[0] == b.nx && last[1] == b.ny && last[2] == b.nz && last[3] == device) return plan;
+    // a thread's steps are mostly on a few boxes or plane ranges of one device:
+    // its last answers are kept
+    struct Kept {
+        int last[4] = {0, 0, 0, -1};
+        StepPlan plan = {false, 1};
+    };
+    constexpr unsigned kKept = 8;
+    static thread_local Kept kept[kKept];
+    static thread_local unsigned next = 0;
+    for (const Kept &k : kept) {
+        const int *last = k.last;
+        if (last[0] == b.nx && last[1] == b.ny && last[2] == b.nz && last[3] == device) return k.plan;
+    }
     const long long tiles = (long long)(b.nx / TX) * (b.ny / TY);
     const int sms = sm_count();
-    if constexpr (sizeof(ST) == 2) {
-        constexpr MarchCost cost = {22, 1.45, {0.0, 1.0, 1.33, 1.97, 2.10}, {0.30, 0.79, 1.22, 1.62, 1.77}};
-        plan.tz = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(device), cost).tz;
-    } else {
-        constexpr MarchCost deep = {22, 1.16, {0.0, 1.0, 1.50}, {0.30, 0.97, 1.54}};
-        constexpr MarchCost dense = {24, 3.19, {0.0, 1.0, 1.42, 1.58}, {1.16, 1.17, 1.08, 1.41}};
-        const Depth d = march_depth(tiles, b.nz, sms, resident_blocks<ST, true>(device), deep);
-        const Depth e = march_depth(tiles, b.nz, sms, resident_blocks<ST, false>(device), dense);
-        // the two costs in one unit
-        plan.deep = d.cost <= 1.12 * e.cost - 2.25;
-        plan.tz = plan.deep ? d.tz : e.tz;
-    }
-    last[0] = b.nx;
-    last[1] = b.ny;
-    last[2] = b.nz;
-    last[3] = device;
+    StepPlan plan;
+    if constexpr (sizeof(ST) == 2)
+        plan = step_plan_16bit(tiles, b.nz, sms, resident_blocks<ST, false>(device));
+    else
+        plan = step_plan_fp32(tiles, b.nz, sms, resident_blocks<ST, true>(device), resident_blocks<ST, false>(device));
+    kept[next++ % kKept] = Kept{{b.nx, b.ny, b.nz, device}, plan};
     return plan;
 }
 
@@ -1458,7 +1431,7 @@ cudaError_t launch_typed(const Box &b, const StepConst &c, const Quant &q, const
     int device = 0;
     const cudaError_t ed = cudaGetDevice(&device);
     if (ed != cudaSuccess) return ed;
-    const Plan plan = choose_plan<ST>(range, device);
+    const StepPlan plan = choose_plan<ST>(range, device);
     const int tz = plan.tz;
     const int nchunks = (range.nz + tz - 1) / tz;
     const unsigned nblocks = (unsigned)((b.nx / TX) * (b.ny / TY) * nchunks);
