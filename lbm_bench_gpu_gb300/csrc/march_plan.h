@@ -51,35 +51,36 @@ inline Depth march_depth(long long tiles, int planes, int sms, int per_sm, const
 
 // Staging geometry (FP32 storage) and planes per block of a step launch.
 //
-// Fitted to forced depths 1 .. 60 of each geometry on 222 boxes from 64 x 40 x 6
-// to 512 x 512 x 256, most of them drawn at random, a third of them flat, with
-// the boxes of up to 256 x 256 columns and 26 planes or more weighted 2.5 fold.
-// On those the plan taken is within 1.2 % of the best one measured on average
-// (at most 8.6 % FP32, 384 x 448 x 11 16 % 16-bit). Before, with constants
-// fitted to boxes of up to 1.2 million nodes and at most 24 planes, it was 3.0 and
-// 2.1 %, and flat boxes lost against the single geometry with its older rule:
-// FP32 384 x 320 x 40 194 us by the older rule, 203 before, 191 now; 384 x 384
-// x 32 181, 188, 179; 32 x 104 x 72 12.9, 14.6, 12.0; FP16 448 x 256 x 30 81.3,
-// 85.6, 78.2; 352 x 480 x 14 62.5, 67.9, 61.0.  On 216 boxes of other draws no
-// plan is slower than the older rule's by more than 0.5 %.
+// Fitted to forced depths 1 .. 60 of each geometry on 379 boxes from 64 x 40 x 6
+// to 512 x 512 x 512, most of them drawn at random, a third of them flat, with
+// more weight on boxes of up to 256 x 256 columns and 26 planes or more and on
+// large ones.  The plan taken is within 1.0 % of the best one measured on average.
+// Before, with constants fitted to boxes of up to 1.2 million nodes and at most
+// 24 planes, it was 3.0 (FP32) and 1.9 % (16-bit), and 52 and 18 of the boxes took
+// longer than with the single geometry and its older rule, by up to 17 and 12 %;
+// now 5 and 3, by up to 3.1 and 5.4 % (the worst are FP32 160 x 232 x 41 60.6 ->
+// 62.5 us, FP16 384 x 448 x 11 51.7 -> 54.5).  On 81 boxes of another draw one is slower than
+// by the older rule (288 x 520 x 32 FP32, 0.8 %).  Older rule, before, now: FP32 384 x
+// 320 x 40 194, 203, 191 us; 32 x 104 x 72 12.9, 14.6, 12.0; 256^3 615, 604, 607;
+// FP16 448 x 256 x 30 81.3, 85.6, 78.2; 352 x 480 x 14 62.5, 67.9, 61.0.
 struct StepPlan {
     bool deep;
     int tz;
 };
 inline StepPlan step_plan_16bit(long long tiles, int planes, int sms, int per_sm)
 {
-    constexpr MarchCost cost = {22, 0.854, {0.0, 1.0, 1.356, 2.344, 2.371}, {0.431, 1.257, 1.978, 1.982, 2.385}, 0.182};
+    constexpr MarchCost cost = {22, 0.87, {0.0, 1.0, 1.398, 2.292, 2.459}, {0.588, 1.168, 1.729, 2.125, 2.569}, 0.438};
     return {false, march_depth(tiles, planes, sms, per_sm, cost).tz};
 }
 inline StepPlan step_plan_fp32(long long tiles, int planes, int sms, int per_sm_deep, int per_sm_dense)
 {
-    constexpr MarchCost deep = {60, 1.531, {0.0, 1.0, 1.62}, {0.884, 1.799, 1.836}, 1.825, 0.002};
-    constexpr MarchCost dense = {60, 1.402, {0.0, 1.0, 1.589, 1.755}, {0.880, 1.531, 1.738, 2.126}, 1.741, 0.037};
+    constexpr MarchCost deep = {60, 1.52, {0.0, 1.0, 1.618}, {0.891, 1.816, 1.838}, 1.863, 0.002};
+    constexpr MarchCost dense = {60, 1.383, {0.0, 1.0, 1.653, 1.757}, {0.888, 1.438, 1.825, 2.112}, 1.724, 0.032};
     const Depth d = march_depth(tiles, planes, sms, per_sm_deep, deep);
     const Depth e = march_depth(tiles, planes, sms, per_sm_dense, dense);
     // the two costs in one unit: a plane of the dense geometry takes a lone block
     // 1.35 times as long
-    if (d.cost <= 1.355 * e.cost - 0.644) return {true, d.tz};
+    if (d.cost <= 1.354 * e.cost - 0.642) return {true, d.tz};
     return {false, e.tz};
 }
 
