@@ -5,8 +5,8 @@
 // compensated float sums (a float pair hi + lo updated with Knuth's two-sum,
 // products split exactly with an FMA), which hold ~48 bits like an FP64 sum
 // at FP32 throughput (GB300's FP64 rate is a small fraction of its FP32 rate);
-// FP64 across threads, warps and blocks in a fixed order (deterministic for a
-// given box).
+// the sums of a warp in three floats, FP64 across warps and blocks, all in a
+// fixed order (deterministic for a given box).
 //
 // Partial / result layout (doubles):
 //   0 max |u|^2 (compat)    1 #phi>=0 (compat)   2..4 sum u over phi>=0 (compat)
@@ -59,7 +59,33 @@ struct Sum2 {
         add(p);
         lo = __fadd_rn(lo, fmaf(a, b, -p));
     }
-    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
+
+// s + e = a + b exactly (Knuth's two-sum)
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
+{
+    s = __fadd_rn(a, b);
+    const float bp = __fsub_rn(s, a);
+    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp));
+}
+
+// A sum in three floats, for the sums of the threads' pairs.
+struct Sum3 {
+    float hi, lo, rest;
+    __device__ __forceinline__ void add(const Sum3 &o)
+    {
+        float e1, e2, e3;
+        two_sum(hi, o.hi, hi, e1);
+        two_sum(lo, o.lo, lo, e2);
+        two_sum(lo, e1, lo, e3);
+        rest = __fadd_rn(__fadd_rn(rest, o.rest), __fadd_rn(e2, e3));
+    }
+    __device__ __forceinline__ Sum3 shuffled(int offset) const   // the value of the lane `offset` away
+    {
+        return Sum3{__shfl_xor_sync(0xffffffffu, hi, offset), __shfl_xor_sync(0xffffffffu, lo, offset),
+                    __shfl_xor_sync(0xffffffffu, rest, offset)};
+    }
+    __device__ __forceinline__ double value() const { return (double)hi + ((double)lo + (double)rest); }
 };
 
 // What a node needs of one plane of phi for the 19-point Laplacian, the
@@ -89,7 +115,7 @@ struct Plane {
 // 256^3 at the copy bandwidth, its 100 FP32 instructions (51 of them in the
 // compensated sums of a node outside the bubbles) 45 us at one per cycle and
 // scheduler, of about 180 in all.  Measured, lbm_stats_noalloc with its fold,
-// 256^3: 368 -> 124 us, 128^3 38, 32^3 78 -> 14 us, against one thread per
+// 256^3: 368 -> 123 us, 128^3 35, 32^3 78 -> 12 us, against one thread per
 // node reading 19 points, with 15 FP64 values per thread reduced over the block
 // (FP64 runs at a 60th of the FP32 rate: that reduction was most of a small
 // box's time).  Also measured at 256^3: one column a thread 145 us (223
@@ -234,27 +260,37 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
         }
     }
 
-    // The block's sums: each thread's ten float pairs go to FP64 and through a
-    // recursive halving over the warp (16 value slots: after offsets 16, 8, 4, 2
-    // a lane holds one value of 16 lanes, then offset 1), 16 FP64 additions per
-    // thread in place of 50.  Float pairs through the warp took 11.5, 16.8 and
-    // 35.2 us at 32^3, 64^3 and 128^3 (now 13.6, 22.9 and 38.0), but kept 48 bits
-    // and left FP32's range where the FP64 sums of the threads' pairs do not.
-    double d[16];
+    // The block's sums: the threads' ten float pairs as three floats each through
+    // a recursive halving over the warp (16 value slots: after offsets 16, 8, 4, 2
+    // a lane holds one value of 16 lanes, then offset 1), 16 additions per thread
+    // in place of 50, and FP64 from one value per warp on.  Three floats keep more
+    // than FP64's 53 bits (two kept 48).  A warp with a sum of 2^122 or more is
+    // scaled by 2^-5, so that no sum over it leaves FP32's range; what that can
+    // shift out is 2^-149.  With FP64 from each thread on, whose additions run at
+    // a 60th of the rate, 32^3, 64^3 and 128^3 took 13.6, 22.8 and
+    // 37.5 us, so 11.5, 18.7 and 35.2 (as two floats 11.5, 16.7 and 35.2).
     const Sum2 *const all[10] = {&s_ux, &s_uy, &s_uz, &s_in, &s_out, &s_phi, &s_rho, &s_mx, &s_my, &s_mz};
+    float most = 0.f;
 #pragma unroll
-    for (int v = 0; v < 16; v++) d[v] = v < 10 ? all[v < 10 ? v : 0]->value() : 0.0;
+    for (int v = 0; v < 10; v++) most = fmaxf(most, fabsf(all[v]->hi));
+    const bool wide = __reduce_max_sync(0xffffffffu, __float_as_uint(most)) >= __float_as_uint(0x1p122f);
+    const float scale = wide ? 0x1p-5f : 1.f;
+    Sum3 t[16];
+#pragma unroll
+    for (int v = 0; v < 16; v++)
+        t[v] = v < 10 ? Sum3{all[v < 10 ? v : 0]->hi * scale, all[v < 10 ? v : 0]->lo * scale, 0.f} : Sum3{0.f, 0.f, 0.f};
 #pragma unroll
     for (int half = 8; half >= 1; half >>= 1) {
         const bool up = lane & (2 * half);
 #pragma unroll
         for (int v = 0; v < half; v++) {
             if (v >= 10) continue;   // (both slots of the pair are empty)
-            const double other = __shfl_xor_sync(0xffffffffu, up ? d[v] : d[v + half], 2 * half);
-            d[v] = (up ? d[v + half] : d[v]) + other;
+            const Sum3 give = up ? t[v] : t[v + half];
+            t[v] = up ? t[v + half] : t[v];
+            t[v].add(give.shuffled(2 * half));
         }
     }
-    d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
+    t[0].add(t[0].shuffled(1));
     cnt_in = __reduce_add_sync(0xffffffffu, cnt_in);
     cnt_all = __reduce_add_sync(0xffffffffu, cnt_all);
     cnt_bad = __reduce_add_sync(0xffffffffu, cnt_bad);
@@ -263,7 +299,7 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
     const unsigned mx_a = __reduce_max_sync(0xffffffffu, __float_as_uint(umax_all));
     __shared__ double red[kWarps][kStatsValues];
     // lane 2 v (of each pair of lanes) holds sum v: result entries 2..6 and 7..11
-    if ((lane & 1) == 0 && lane < 20) red[warp][2 + (lane >> 1)] = d[0];
+    if ((lane & 1) == 0 && lane < 20) red[warp][2 + (lane >> 1)] = t[0].value() * (wide ? 32.0 : 1.0);
     if (lane == 31) {
         red[warp][0] = __uint_as_float(mx_c);
         red[warp][1] = cnt_in;
