@@ -559,7 +559,6 @@ struct Adjoint {
         phi = w.take<float>(2 * n);
         partials = w.take<double>(2 * nblocks);
         ab = w.take<double>(8);
-        acc = w.take<double>(2);
         if (!gradient) return;
         for (int i = 0; i < 2; i++) {
             lam_g[i] = w.take<float>((size_t)lbm::kQg * n);
@@ -642,6 +641,7 @@ void setup(Adjoint &A, lbm_ctx *c, const lbm_adjoint_opts *o)
     A.n = (size_t)c->box.n;
     A.snap_bytes = sizeof(float) * A.n + c->esz * (lbm::kQf - 1 + lbm::kQg) * A.n;
     A.k = lbm::step_const(c->d, c->p, o->grav);
+    A.acc = c->result;   // free between statistics; one copy brings it back with the error flag behind it
     A.first_source = o->objective == LBM_OBJ_LIGHT_UZ_MEAN ? o->nsteps - o->window + 1 : o->nsteps;
     A.scale = o->objective == LBM_OBJ_LIGHT_UZ_MEAN ? 1.0 / o->window : 1.0;
 }
@@ -675,16 +675,14 @@ extern "C" int lbm_objective(lbm_ctx *c, const lbm_adjoint_opts *o, double *J)
         }
         if (!rc && k < o->nsteps) rc = A.forward(1);
     }
-    double acc[2] = {0.0, 0.0};
     if (!rc) {
-        e = cudaMemcpyAsync(acc, A.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = lbm::queue_flag(c);
+        e = lbm::queue_report(c);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         rc = e == cudaSuccess ? lbm::flag_status(c) : cuda_fail(e, "lbm_objective: results");
     }
     A.release();
     if (rc) return rc;
-    *J = acc[0];
+    *J = c->result_host[0];
     return LBM_OK;
 }
 
@@ -762,20 +760,18 @@ extern "C" int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoi
                                          A.lam_g[A.cur], lphi0, A.phi, c->stream);
         if (e != cudaSuccess) rc = cuda_fail(e, "lbm_step_adjoint: initial-state adjoint");
     }
-    double acc[2] = {0.0, 0.0};
     if (!rc) {
         if (out->dJ_dphi0) map_result(out->dJ_dphi0, sizeof(float) * n, c->stream);
-        e = cudaMemcpyAsync(acc, A.acc, sizeof(acc), cudaMemcpyDeviceToHost, c->stream);
+        e = lbm::queue_report(c);
         if (e == cudaSuccess && out->dJ_dphi0)
             e = cudaMemcpyAsync(out->dJ_dphi0, lphi0, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = lbm::queue_flag(c);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         rc = e == cudaSuccess ? lbm::flag_status(c) : cuda_fail(e, "lbm_step_adjoint: results");
     }
     A.release();
     if (rc) return rc;
-    out->J = acc[0];
-    out->dJ_dgrav = acc[1];
+    out->J = c->result_host[0];
+    out->dJ_dgrav = c->result_host[1];
     out->slots = (int)nslots;
     out->forward_steps = A.fwd_steps;
     out->adjoint_steps = A.adj_steps;

@@ -270,15 +270,17 @@ namespace lbm {
 // build found a global index outside its field (LBM_ECUDA).
 int device_error(lbm_ctx *c)
 {
-    LBM_CUDA(queue_flag(c), "error flag");
+    // on the context's stream, after the kernels that set it
+    LBM_CUDA(cudaMemcpyAsync(c->result_host + kStatsValues, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream),
+             "error flag");
     LBM_CUDA(cudaStreamSynchronize(c->stream), "error flag");
     return flag_status(c);
 }
 
-cudaError_t queue_flag(lbm_ctx *c)
+cudaError_t queue_report(lbm_ctx *c)
 {
     // on the context's stream, after the kernels that set it
-    return cudaMemcpyAsync(c->result_host + kStatsValues, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    return cudaMemcpyAsync(c->result_host, c->result, kReportBytes, cudaMemcpyDeviceToHost, c->stream);
 }
 
 int flag_status(const lbm_ctx *c)
@@ -538,8 +540,7 @@ extern "C" int lbm_stats(lbm_ctx *c, lbm_stats_out *s, float *phi, float *rho, f
     }
     // the sums (meaningful with s only) and the error flag in one copy, one
     // wait for everything: a 32^3 box's call took two copies and two waits
-    LBM_CUDA(cudaMemcpyAsync(c->result_host, c->result, lbm::kReportBytes, cudaMemcpyDeviceToHost, c->stream),
-             "stats copy");
+    LBM_CUDA(lbm::queue_report(c), "stats copy");
     float *dst[5] = {phi, rho, ux, uy, uz};
     for (int a = 0; a < 5; a++)
         if (dst[a])

@@ -273,10 +273,11 @@ int create_context(lbm_ctx **out, const lbm_params *p, int zghost);
 // moments: the last one writes the phi, rho, u fields.
 int queue_steps(lbm_ctx *c, int nsteps, float grav, bool moments);
 // The kernels' error flag as a status (LBM_ETIMEOUT, LBM_ECUDA) after a sync;
-// its copy to the host alone, for a caller that waits for more than it; and the
-// status of the flag that this or a copy of the report has brought to the host.
+// the report's copy to the host (what c->result holds and the flag behind it),
+// for a caller that waits for more than it; and the status of the flag that
+// either has brought to the host.
 int device_error(lbm_ctx *c);
-cudaError_t queue_flag(lbm_ctx *c);
+cudaError_t queue_report(lbm_ctx *c);
 int flag_status(const lbm_ctx *c);
 // lbm_stats_out from the raw statistics of a box of n nodes.
 int fill_stats_raw(double n, const lbm_params &p, long long steps, const double *raw, lbm_stats_out *s);
