@@ -157,8 +157,8 @@ __device__ __forceinline__ Eq equilibrium_at(const Box &b, const EqConst &c, con
 
 // A block: a 32 x 8 tile (16-bit: 16 words of the pair layout, i.e. 32 nodes, x
 // 8 rows) of EQZ planes.  The stores bound these kernels (104 or 54 bytes a
-// node against 8 read): 256^3 FP32 325 us, 5.8 TB/s; FP16 210 us (5.0 TB/s) and
-// 129 for the maxima.  The equilibrium into an FP32 scratch copy, the maxima of
+// node against 8 read): 256^3 FP32 297 us, 6.3 TB/s; FP16 171 us (6.1 TB/s) and
+// 107 for the maxima (325, 210 and 129 on a grid of three dimensions).  The equilibrium into an FP32 scratch copy, the maxima of
 // that and its conversion took 700, 289 and 498.
 constexpr int EQZ = 4;
 
