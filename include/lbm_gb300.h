@@ -211,14 +211,15 @@ typedef struct lbm_adjoint_out {
  * The work buffers and the checkpoint pool stay allocated in the context for
  * the next call (a pool larger than the next budget is reused, not shrunk)
  * until lbm_adjoint_release or lbm_destroy; checkpoint_bytes <= 0 counts the
- * cached pool as free memory. */
+ * cached pool as free memory.  LBM_ETIMEOUT (or LBM_ECUDA) if a forward step
+ * has set the context's error flag: no result then, as from lbm_sync. */
 int lbm_step_adjoint(lbm_ctx *c, const lbm_adjoint_opts *o, lbm_adjoint_out *out);
 
 /* The objective of lbm_step_adjoint alone (forward run, no gradient), e.g.
  * for finite-difference checks of the gradient: o->checkpoint_bytes is
  * ignored, one state snapshot is held.  No counterpart in the reference.
- * Same preconditions; on return the context holds the initial state again.
- * Synchronises. */
+ * Same preconditions and errors; on return the context holds the initial state
+ * again.  Synchronises. */
 int lbm_objective(lbm_ctx *c, const lbm_adjoint_opts *o, double *J);
 
 /* Free the adjoint work buffers and checkpoint pool that lbm_step_adjoint and
