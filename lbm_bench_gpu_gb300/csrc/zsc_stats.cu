@@ -265,7 +265,7 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
     // a lane holds one value of 16 lanes, then offset 1), 16 additions per thread
     // in place of 50, and FP64 from one value per warp on.  Three floats keep more
     // than FP64's 53 bits (two kept 48).  A warp with a sum of 2^122 or more is
-    // scaled by 2^-5, so that no sum over it leaves FP32's range; what that can
+    // scaled by 2^-6, so that no sum over it leaves FP32's range; what that can
     // shift out is 2^-149.  With FP64 from each thread on, whose additions run at
     // a 60th of the rate, 32^3, 64^3 and 128^3 took 13.6, 22.8 and
     // 37.5 us, so 11.5, 18.7 and 35.2 (as two floats 11.5, 16.7 and 35.2).
@@ -274,7 +274,7 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
 #pragma unroll
     for (int v = 0; v < 10; v++) most = fmaxf(most, fabsf(all[v]->hi));
     const bool wide = __reduce_max_sync(0xffffffffu, __float_as_uint(most)) >= __float_as_uint(0x1p122f);
-    const float scale = wide ? 0x1p-5f : 1.f;
+    const float scale = wide ? 0x1p-6f : 1.f;
     Sum3 t[16];
 #pragma unroll
     for (int v = 0; v < 16; v++)
@@ -299,7 +299,7 @@ stats_kernel(Box b, StatsConst c, const float *__restrict__ phi, const float *__
     const unsigned mx_a = __reduce_max_sync(0xffffffffu, __float_as_uint(umax_all));
     __shared__ double red[kWarps][kStatsValues];
     // lane 2 v (of each pair of lanes) holds sum v: result entries 2..6 and 7..11
-    if ((lane & 1) == 0 && lane < 20) red[warp][2 + (lane >> 1)] = t[0].value() * (wide ? 32.0 : 1.0);
+    if ((lane & 1) == 0 && lane < 20) red[warp][2 + (lane >> 1)] = t[0].value() * (wide ? 64.0 : 1.0);
     if (lane == 31) {
         red[warp][0] = __uint_as_float(mx_c);
         red[warp][1] = cnt_in;

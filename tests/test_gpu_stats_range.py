@@ -34,6 +34,21 @@ def test_sums_beyond_fp32(lib, shape):
     assert got[14] == 0
 
 
+# A warp whose threads' sums all reach the top of FP32's range.
+def test_sums_at_the_end_of_fp32(lib):
+    from lbm_bench_gpu_gb300 import capi
+    shape = (64, 32, 4)
+    p = capi.make_params(*shape, **PHYS)
+    nx, ny, nz = shape
+    n, big = nx * ny * nz, np.float32(2.0**127 * (1 - 2.0**-24))   # two of them: FP32's largest value
+    phi = np.full((nz, ny, nx), -0.45, np.float32)
+    rho = np.full(phi.shape, big)
+    u = [np.full(phi.shape, np.float32(v)) for v in (1.0, -0.5, 0.25)]
+    got = _raw(lib, p, [phi, rho] + u)
+    want = float(big) * n
+    assert abs(got[8] - want) <= n * 2.0**-53 * want and abs(got[9] - want) <= n * 2.0**-53 * want
+
+
 def test_pressure_beside_left_out_nodes(lib):
     from lbm_bench_gpu_gb300 import capi
     shape = (45, 19, 11)
